@@ -245,7 +245,7 @@ int sym_step_timed(sym_handle* h, int nsteps, int use_graph, double ms[4]);
  * subroutine over a (domain, particle, block) table), and one persistent
  * collide launch whose CTAs pull 32x8xX tiles of any domain from a work-tile
  * table (largest first).  Results per domain are identical to sym_step on that
- * domain alone with the same tile x extent.  Member handles stay usable on
+ * domain alone, whatever the tiles' x extents.  Member handles stay usable on
  * their own; the batch rebuilds its graphs when a member was stepped or read
  * back outside it. */
 typedef struct sym_batch sym_batch;
@@ -255,6 +255,8 @@ const char* sym_batch_last_error(const sym_batch* b);
 int sym_batch_step(sym_batch* b, int nsteps);
 /* nsteps graph steps bracketed by CUDA events on the batch stream; *ms = elapsed. */
 int sym_batch_step_timed(sym_batch* b, int nsteps, double* ms);
+/* The most x planes per collide tile of one domain (default 32); shorter tiles
+ * are taken when the batch has too few to fill the GPU.  Never changes a result. */
 int sym_batch_set_xchunk(sym_batch* b, int domain, int xchunk);
 int sym_batch_get_xchunk(sym_batch* b, int domain, int* xchunk);
 /* Resident collide CTAs per SM of the persistent launch (1 .. the most that

@@ -255,6 +255,17 @@ int build(sym_batch* b) {
   std::vector<DomainDesc> desc[2];
   std::vector<long long> off(n + 1, 0);
   std::vector<TileEntry> tiles;
+  // one estimate for the whole batch; each domain's set extent is its cap
+  const int BY = tile_rows(b->storage);
+  std::vector<long long> columns;
+  std::vector<int> extent;
+  for (int i = 0; i < n; i++) {
+    const DevParams& P = b->doms[i]->dp;
+    columns.push_back((long long)((P.nz + BZ - 1) / BZ) * ((P.ny + BY - 1) / BY));
+    extent.push_back(P.nx);
+  }
+  const int most = *std::max_element(b->xchunk.begin(), b->xchunk.end());
+  const int fill = best_extent(columns, extent, most, b->grid);
   for (int i = 0; i < n; i++) {
     sym_handle* h = b->doms[i];
     if (!h->fast.valid) {
@@ -265,9 +276,8 @@ int build(sym_batch* b) {
     b->built_pc[i] = h->fast.pc;
     for (int k = 0; k < 2; k++) desc[k].push_back(make_desc(h, (h->fast.cur + k) & 1, (h->fast.pc + k) & 1));
     off[i + 1] = off[i] + (long long)((h->N + 255) / 256);
-    const int xc = std::max(1, b->xchunk[i]);
     const DevParams& P = h->dp;
-    const int BY = tile_rows(b->storage);
+    const int xc = split_extent(P.nx, std::min(fill, b->xchunk[i]));
     for (int xa = 0; xa < P.nx; xa += xc)
       for (int y0 = 0; y0 < P.ny; y0 += BY)
         for (int z0 = 0; z0 < P.nz; z0 += BZ) {

@@ -110,8 +110,12 @@ int enqueue_step(sym_handle* h, int cur, int pc, cudaEvent_t* ev) {
   // particle coupling and pin fill (cur and pc advance together from 0)
   if (int e = sparse_enqueue(h->fast.sparse, cur, h->st)) return set_error(h, e, "sparse step");
   // (a3-a9) fused derivatives + collision + recolour + stream + bounce-back
-  const int xc = h->fast.xchunk > 0 ? h->fast.xchunk : XCHUNK;
-  dim3 grid((P.nz + BZ - 1) / BZ, (P.ny + kBY<S> - 1) / kBY<S>, (P.nx + xc - 1) / xc);
+  dim3 grid((P.nz + BZ - 1) / BZ, (P.ny + kBY<S> - 1) / kBY<S>);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+  const int xc = split_extent(P.nx, best_extent({(long long)grid.x * grid.y}, {P.nx}, XCHUNK,
+                                                (long long)collide_ctas<S>() * sms));
+  grid.z = (P.nx + xc - 1) / xc;
   const size_t shm = smem_bytes<S>();
   const CUtensorMap& tp = h->fast.tm_phi[pc];
   const CUtensorMap& tr = h->fast.tm_ref[pc];

@@ -3,9 +3,11 @@
 // See fast.cu for the per-step kernel sequence.
 #pragma once
 #include <cuda_fp16.h>
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <utility>
+#include <vector>
 #include "state.cuh"
 #include "tma.cuh"
 
@@ -13,7 +15,7 @@ namespace symb200 {
 namespace fused {
 
 constexpr int BZ = 32;   // tile width along z: one warp per row
-constexpr int XCHUNK = 32;   // x planes marched by one CTA
+constexpr int XCHUNK = 32;   // most x planes marched by one CTA
 
 // ---- halo-padded phase field -----------------------------------------------------
 struct Pad {
@@ -202,15 +204,17 @@ struct Acc<float> {
 template <typename S>
 constexpr bool kAccumulate = sizeof(S) == 8;
 
-// add v to accumulator p (a reduction: nothing is returned); out-of-range
-// values set *status and add nothing
+// v in fixed point; an out-of-range value sets *status and counts as nothing
+template <typename R>
+__device__ __forceinline__ typename Acc<R>::T acc_fix(R v, int* status) {
+  if (Acc<R>::ok(v)) return Acc<R>::fix(v);
+  atomicOr(status, 1);
+  return 0;
+}
+// add v to accumulator p (a reduction: nothing is returned)
 template <typename R>
 __device__ __forceinline__ void acc_add(typename Acc<R>::T* p, R v, int* status) {
-  if (Acc<R>::ok(v)) {
-    atomicAdd(p, Acc<R>::fix(v));
-  } else {
-    atomicOr(status, 1);
-  }
+  atomicAdd(p, acc_fix<R>(v, status));
 }
 
 template <typename F, int... Is>
@@ -541,16 +545,20 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
   // clamped node), so the warp shuffles of the density accumulation below see
   // the whole warp; `act` masks the stores and contributions
   const int yc = min(y, P.ny - 1), zc = min(z, P.nz - 1);
-  // pushes whose destination lies outside this CTA's tile (or across a
-  // periodic wrap) are added to the accumulators directly; the others are
-  // combined inside the CTA first (z through warp shuffles, y through shared
-  // memory, x in registers along the march) and added once per node
+  // Pushes that leave the tile along z (or across the periodic wrap) are added
+  // to the accumulators directly; the others are summed over z through warp
+  // shuffles, then over y through shared memory (a row at the tile's y edge
+  // adds its outgoing sums directly), and the sum a plane sends to each
+  // destination plane is turned into fixed point before the planes are added
+  // in registers along the march: the totals are integer sums of terms that
+  // do not depend on where the march starts or ends, so a domain's result is
+  // the same bit for bit whatever x extent its tiles have.
   const bool ezp = tz == BZ - 1 || z >= P.nz - 1, ezm = tz == 0 || z == 0;
   const bool eyp = ty == BY - 1 || y >= P.ny - 1, eym = ty == 0 || y == 0;
   using AT = typename Acc<R>::T;
   AT* const accR = acc;
   AT* const accB = acc + N;
-  R aPr = R(0), aPb = R(0), aCr = R(0), aCb = R(0), aNr = R(0), aNb = R(0);   // planes x-1, x, x+1
+  AT aPr = 0, aPb = 0, aCr = 0, aCb = 0;   // planes x-1 and x
   for (int x = xa; x < xb; x++) {
     // phi of plane x+3 on its way; normals of plane x+1 from phi planes x..x+2.
     // The slots the load overwrites (phi of plane x-2, reference pairs of plane x-3)
@@ -666,7 +674,6 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
     const bool rzero = sr <= evap, bzero = sb <= evap;
     const R ratio = bzero ? R(1) : (rzero ? R(0) : sr * irho);
     const R coef = (bzero || rzero || !flag) ? R(0) : sr * sb * irho * R(P.beta);
-    const bool exp_ = x == xb - 1, exm = x == xa;
     // rigid-body velocity of particle pp at this node (curve :1009-1014), for
     // the links that bounce back from it
     R uw0 = R(0), uw1 = R(0), uw2 = R(0);
@@ -721,12 +728,7 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
         Codec<S>::template store<i>(pout_, N, T, rd, r, f[i]);
         if constexpr (!ACC) return;
         const R bv = f[i] - r;
-        const bool ext = (CX(i) > 0 && exp_) || (CX(i) < 0 && exm) || (CY(i) > 0 && eyp) || (CY(i) < 0 && eym) ||
-                         (CZ(i) > 0 && ezp) || (CZ(i) < 0 && ezm);
-        if (ext) {
-          acc_add<R>(accR + T, r, status);
-          acc_add<R>(accB + T, bv, status);
-        } else if (CZ(i) == 0) {
+        if (CZ(i) == 0) {
           g[a][b][0] = g[a][b][0] + r;
           g[a][b][1] = g[a][b][1] + bv;
         } else if (CZ(i) > 0) {
@@ -739,15 +741,27 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
       }();
       if constexpr (ACC && CZ(i) < 0) {
         // last of a group with cz = 0, +1, -1: lane l receives the cz = +1 push
-        // of lane l-1 and the cz = -1 push of lane l+1 (lane = tz)
+        // of lane l-1 and the cz = -1 push of lane l+1 (lane = tz); the edge
+        // lanes' outgoing pushes go to the accumulators in one go (a lane that
+        // is both edges, of a one-node tile row, adds its second one after)
 #pragma unroll
         for (int c = 0; c < 2; c++) {
           const R up = __shfl_up_sync(0xffffffffu, zp[c], 1);
           const R dn = __shfl_down_sync(0xffffffffu, zm[c], 1);
           g[a][b][c] = g[a][b][c] + (tz > 0 ? up : R(0)) + (tz < BZ - 1 ? dn : R(0));
-          zp[c] = R(0);
-          zm[c] = R(0);
         }
+        if (act && (ezp || ezm)) {
+          const unsigned T0 = L + (a > 1 ? oxp : (a < 1 ? oxm : 0)) + (b > 1 ? oyp : (b < 1 ? oym : 0));
+          const unsigned T = T0 + (ezp ? ozp : ozm);
+          acc_add<R>(accR + T, ezp ? zp[0] : zm[0], status);
+          acc_add<R>(accB + T, ezp ? zp[1] : zm[1], status);
+          if (ezp && ezm) {
+            acc_add<R>(accR + T0 + ozm, zm[0], status);
+            acc_add<R>(accB + T0 + ozm, zm[1], status);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; c++) zp[c] = zm[c] = R(0);
       }
     });
     }
@@ -761,8 +775,9 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
           sm.xch[a][0][c][ty][tz] = g[a][2][c];
           sm.xch[a][1][c][ty][tz] = g[a][0][c];
         }
+      const int oxp = (x == P.nx - 1) ? -(P.nx - 1) * sx : sx, oxm = (x == 0) ? (P.nx - 1) * sx : -sx;
       __syncthreads();
-      R in[3][2];
+      AT in[3][2];
 #pragma unroll
       for (int a = 0; a < 3; a++)
 #pragma unroll
@@ -770,25 +785,42 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
           R v = g[a][1][c];
           if (ty > 0) v = v + sm.xch[a][0][c][ty - 1][tz];
           if (ty < BY - 1) v = v + sm.xch[a][1][c][ty + 1][tz];
-          in[a][c] = v;
+          if (a == 1) v = v + (c ? sfb : sfr);
+          in[a][c] = inr ? acc_fix<R>(v, status) : 0;
         }
-      aPr = aPr + in[0][0]; aPb = aPb + in[0][1];
-      aCr = aCr + in[1][0] + sfr; aCb = aCb + in[1][1] + sfb;
-      aNr = aNr + in[2][0]; aNb = aNb + in[2][1];
-      // plane x-1 of this column has all its in-tile contributions
-      if (x > xa && inr && (aPr != R(0) || aPb != R(0))) {
-        acc_add<R>(accR + (L - sx), aPr, status);
-        acc_add<R>(accB + (L - sx), aPb, status);
+      if (inr && (eyp || eym)) {
+        // the sums a row at the tile's y edge sends out of it
+        const int oyp = (y == P.ny - 1) ? -(P.ny - 1) * sy : sy, oym = (y == 0) ? (P.ny - 1) * sy : -sy;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+          const unsigned T0 = L + (a > 1 ? oxp : (a < 1 ? oxm : 0));
+          acc_add<R>(accR + T0 + (eyp ? oyp : oym), eyp ? g[a][2][0] : g[a][0][0], status);
+          acc_add<R>(accB + T0 + (eyp ? oyp : oym), eyp ? g[a][2][1] : g[a][0][1], status);
+          if (eyp && eym) {
+            acc_add<R>(accR + T0 + oym, g[a][0][0], status);
+            acc_add<R>(accB + T0 + oym, g[a][0][1], status);
+          }
+        }
+      }
+      // plane x-1 of this column has all its in-tile contributions (plane xa-1
+      // only this plane's)
+      aPr += in[0][0]; aPb += in[0][1];
+      aCr += in[1][0]; aCb += in[1][1];
+      const int om = x > xa ? -sx : oxm;
+      if (inr && (aPr | aPb)) {
+        atomicAdd(accR + (L + om), aPr);
+        atomicAdd(accB + (L + om), aPb);
       }
       aPr = aCr; aPb = aCb;
-      aCr = aNr; aCb = aNb;
-      aNr = R(0); aNb = R(0);
+      aCr = in[2][0]; aCb = in[2][1];
+      if (x == xb - 1 && inr) {
+        // the end of the march: this plane's node and the plane after it
+        atomicAdd(accR + L, aPr);
+        atomicAdd(accB + L, aPb);
+        atomicAdd(accR + (L + oxp), aCr);
+        atomicAdd(accB + (L + oxp), aCb);
+      }
     }
-  }
-  if (ACC && xb > xa && inr && (aPr != R(0) || aPb != R(0))) {
-    const unsigned L = (unsigned)(z + sy * y + sx * (xb - 1));
-    acc_add<R>(accR + L, aPr, status);
-    acc_add<R>(accB + L, aPb, status);
   }
 }
 
@@ -800,6 +832,41 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
 template <typename S>
 constexpr int collide_ctas() {
   return std::is_same<S, __half>::value ? 2 : (sizeof(typename Codec<S>::R) == 4 ? 4 : 2);
+}
+
+// Plane times a tile spends before its first plane (five plane loads and the
+// normals of two planes).
+constexpr double kTileLead = 1.0;
+// x extent of a tile whose column of x planes is nx long, at most `cap`: the
+// column in equal parts
+inline int split_extent(int nx, int cap) {
+  const int parts = (nx + cap - 1) / cap;
+  return (nx + parts - 1) / parts;
+}
+// The tile x extent, at most `cap`, for columns[i] columns (32 x BY
+// footprints) of nx[i] planes each on `slots` resident CTAs: the one with the
+// least estimated time, in planes: the work of all slots evenly shared plus
+// half a tile of tail, or one whole tile when there are fewer tiles than
+// slots.  A CTA needs about 6 us for an FP64 plane (2.8 FP32, 4.9 16-bit)
+// whether the GPU is full or not, so a domain of few columns is bound by the
+// length of one march.  Measured per step, extent 32 against this rule's:
+// 32x32x96 FP64 209 -> 29 us (3 planes), 53x53x374 269 -> 210, 64x64x128
+// 219 -> 111, FP32 113 -> 51, 16-bit 172 -> 57; 256x256x256 keeps 32.
+inline int best_extent(const std::vector<long long>& columns, const std::vector<int>& nx, int cap, long long slots) {
+  int best = 1;
+  double least = 1e300;
+  for (int x = 1; x <= cap; x++) {
+    double sum = 0.0, longest = 0.0;
+    for (size_t i = 0; i < nx.size(); i++) {
+      const int e = split_extent(nx[i], x);
+      const int tiles = (nx[i] + e - 1) / e;
+      sum += (double)columns[i] * (nx[i] + tiles * kTileLead);
+      longest = std::max(longest, e + kTileLead);
+    }
+    const double t = std::max(longest, sum / (double)slots + 0.5 * longest);
+    if (t <= least) { least = t; best = x; }
+  }
+  return best;
 }
 
 template <typename S, bool SOLID>

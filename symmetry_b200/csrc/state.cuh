@@ -19,7 +19,6 @@ struct FastState {
   void* pop[2] = {nullptr, nullptr};
   int cur = 0;             // buffer holding the current post-stream populations
   int pc = 0;              // phase-field buffer written by the next step
-  int xchunk = 0;          // x planes per tile of the fused collide kernel (0 = default)
   double* phi[2] = {nullptr, nullptr};  // FP64 halo-padded phase field (pin-filled)
   float* phif[2] = {nullptr, nullptr};  // FP32 halo-padded phase field for FP32/FP16 storage
   float2* rref[2] = {nullptr, nullptr};  // 16-bit storage: halo-padded reference pairs (rho, red fraction), same parity as phi
