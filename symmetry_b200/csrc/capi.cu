@@ -82,8 +82,23 @@ void fill_devparams(const sym_params& p, DevParams& d) {
   d.inertia = p.inertia > 0 ? p.inertia : 2.0 / 5.0 * d.mass * (p.rad * p.rad);
   d.fg = p.fg; d.alpha = p.alpha;
   d.evap = p.evap_lim > 0 ? p.evap_lim : 1.0e-8;
-  d.inu_r = p.nu_r > 0 ? 1.0 / p.nu_r : 0.0;
-  d.inu_b = p.nu_b > 0 ? 1.0 / p.nu_b : 0.0;
+  // node_rates with phi clamped to [-1, 1] and D = (1+phi)/nu_r + (1-phi)/nu_b:
+  // su = 1/(3 nu + 1/2) = 2D/(12 + D), sq = 8 (2-su)/(8-su) = 32/(16 + D)
+  d.same_nu = p.nu_r == p.nu_b;
+  NodeParams<double>& q = d.nd;
+  q.half_sigma = 0.5 * p.sigma; q.beta = p.beta; q.evap = d.evap;
+  for (int k = 0; k < 3; k++) q.body[k] = p.body[k];
+  q.inu_r = p.nu_r > 0 ? 1.0 / p.nu_r : 0.0;
+  q.inu_b = p.nu_b > 0 ? 1.0 / p.nu_b : 0.0;
+  q.s_e = p.s_e; q.s_eps = p.s_eps; q.s_q = p.s_q; q.s_pi = p.s_pi; q.s_m = p.s_m;
+  q.su = 2.0 * (2.0 * q.inu_r) / (12.0 + 2.0 * q.inu_r);
+  q.sq = 32.0 / (16.0 + 2.0 * q.inu_r);
+  NodeParams<float>& f = d.nf;
+  f.half_sigma = (float)q.half_sigma; f.beta = (float)q.beta; f.evap = (float)q.evap;
+  for (int k = 0; k < 3; k++) f.body[k] = (float)q.body[k];
+  f.inu_r = (float)q.inu_r; f.inu_b = (float)q.inu_b;
+  f.s_e = (float)q.s_e; f.s_eps = (float)q.s_eps; f.s_q = (float)q.s_q; f.s_pi = (float)q.s_pi; f.s_m = (float)q.s_m;
+  f.su = (float)q.su; f.sq = (float)q.sq;
 }
 
 }  // namespace symb200

@@ -8,6 +8,7 @@
 #include <type_traits>
 #include <utility>
 #include <vector>
+#include "nodemath.cuh"
 #include "state.cuh"
 #include "tma.cuh"
 
@@ -367,11 +368,38 @@ __device__ __forceinline__ void wet_rotate(const DevParams& P, const sym_particl
 // (phi x+4 -> slot (x-1)%5, normals x+2 -> (x-2)%4, reference-pair x+4 -> (x-2)%6)
 // are never among them.
 constexpr int kIrrRing = 6;
-// unit normal and |grad phi| of one node, read with one (FP32) or two (FP64)
-// 16-byte shared-memory accesses
-template <typename R>
-struct alignas(4 * sizeof(R)) NormalV {
-  R x, y, z, g;
+// The unit normals and |grad phi| of four planes of a tile, [plane][y][z].  FP32
+// keeps a node's four numbers in one 16-byte access.  FP64 splits them so that
+// a warp's accesses are contiguous (16-byte x, y pairs and 8-byte z: 6 shared
+// memory wavefronts a node's normal for a warp, against 16 of a 32-byte
+// record); only a node's own |grad phi| is read.
+template <typename R, int ROWS>
+struct NormalTile {
+  float4 v[4][ROWS][BZ + 2];
+  __device__ __forceinline__ void set(int s, int y, int z, R nx, R ny, R nz, R g) {
+    v[s][y][z] = make_float4(nx, ny, nz, g);
+  }
+  __device__ __forceinline__ void get(int s, int y, int z, R (&n)[3]) const {
+    const float4 t = v[s][y][z];
+    n[0] = t.x; n[1] = t.y; n[2] = t.z;
+  }
+  __device__ __forceinline__ R grad(int s, int y, int z) const { return v[s][y][z].w; }
+};
+template <int ROWS>
+struct NormalTile<double, ROWS> {
+  double2 xy[4][ROWS][BZ + 2];
+  double z_[4][ROWS][BZ + 2];
+  double g[4][ROWS][BZ + 2];
+  __device__ __forceinline__ void set(int s, int y, int z, double nx, double ny, double nz, double gr) {
+    xy[s][y][z] = make_double2(nx, ny);
+    z_[s][y][z] = nz;
+    g[s][y][z] = gr;
+  }
+  __device__ __forceinline__ void get(int s, int y, int z, double (&n)[3]) const {
+    const double2 t = xy[s][y][z];
+    n[0] = t.x; n[1] = t.y; n[2] = z_[s][y][z];
+  }
+  __device__ __forceinline__ double grad(int s, int y, int z) const { return g[s][y][z]; }
 };
 // Tile height (rows of BZ nodes) of the collide kernels per storage: 16
 // rows for the 16-bit codec, 8 for FP32 and FP64.  Measured on the batched
@@ -399,7 +427,7 @@ struct Smem {
   static constexpr int kRefSlot = (kPlaneTile<S> * 8 + 127) / 128 * 128 / 8;
   alignas(128) R phi[5][kPhiSlot];
   alignas(128) Ref ref[Codec<S>::kRef ? kIrrRing : 1][kRefSlot];   // reference pairs of this step (16-bit storage)
-  NormalV<R> n[4][BY + 2][BZ + 2];   // [plane][y][z]: n and |grad phi|
+  alignas(16) NormalTile<R, BY + 2> n;
   // [cx+1][to row y+1, y-1][colour]: density sums crossing rows (accumulating
   // storages only; a single element otherwise)
   R xch[kAccumulate<S> ? 3 : 1][2][2][kAccumulate<S> ? BY : 1][kAccumulate<S> ? BZ : 1];
@@ -454,7 +482,8 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
   constexpr bool REF = Codec<S>::kRef;
   const int tz = threadIdx.x % BZ, ty = threadIdx.x / BZ;
   const unsigned N = (unsigned)P.N;
-  const R evap = R(P.evap);
+  const NodeParams<R>& np = node_params<R>(P);
+  const R evap = np.evap;
   const int sy = P.nz, sx = P.nz * P.ny;   // element strides of y and x
 
   // phi (and the reference pairs) of plane xp by TMA: one box of (BY+4) x (BZ+4) at the
@@ -512,20 +541,15 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
         });
         g0 = R(3) * g0; g1 = R(3) * g1; g2 = R(3) * g2;
         const R g2s = g0 * g0 + g1 * g1 + g2 * g2;
-        R rf = R(0);
-        if constexpr (sizeof(R) == 4) {
-          // FP32 arithmetic: |grad phi| and its reciprocal from one rsqrt
-          if (g2s > evap * evap) { rf = rsqrtf(g2s); fn = g2s * rf; }
-        } else {
-          fn = sqrt(g2s);
-          if (fn > evap) rf = R(1) / fn; else fn = R(0);
-        }
-        if (fn > R(0)) {
+        // |grad phi| and its reciprocal from one rsqrt
+        if (g2s > evap * evap) {
+          const R rf = rsqrt(g2s);
+          fn = g2s * rf;
           n0 = g0 * rf; n1 = g1 * rf; n2 = g2 * rf;
           if (SOLIDX && pp >= 1) wet_rotate<R>(P, Sp, pp, wrapi(xp, P.nx), wrapi(y, P.ny), wrapi(z, P.nz), n0, n1, n2);
         }
       }
-      sm.n[s][py][pz] = NormalV<R>{n0, n1, n2, fn};
+      sm.n.set(s, py, pz, n0, n1, n2, fn);
     }
   };
 
@@ -606,60 +630,110 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
     if (ACC ? __any_sync(0xffffffffu, act) : act) {
     // calmacros on the own populations
     // (rho_B = rho - rho_R: a pure colour stays exactly pure, as r = f there)
-    R f[19];
-    R sr = R(0), rho = R(0);
+    R f[19], sr, sb, rho, irho;
     const Ref rref = REF ? rr_old[pd.idx(x, yc, zc)] : Ref{};
-    unroll19([&](auto ic) {
-      constexpr int i = decltype(ic)::value;
-      R r;
-      Codec<S>::template load_fr<i>(pin_, N, L, rref, f[i], r);
-      sr = sr + r;
-      rho = rho + f[i];
-    });
-    const R sb = rho - sr;
-    R ux = R(0), uy = R(0), uz = R(0);
-#pragma unroll
-    for (int i = 0; i < 19; i++) {
-      if (CX(i)) ux = ux + f[i] * R(CX(i));
-      if (CY(i)) uy = uy + f[i] * R(CY(i));
-      if (CZ(i)) uz = uz + f[i] * R(CZ(i));
-    }
-    const R irho = qdiv<R>(R(1), rho);
-    ux = ux * irho; uy = uy * irho; uz = uz * irho;
-    const NormalV<R> nown = sm.n[x & 3][ty + 1][tz + 1];
-    const R nx = nown.x, ny = nown.y, nz = nown.z, fn = nown.g;
+    R nown[3];
+    sm.n.get(x & 3, ty + 1, tz + 1, nown);
+    const R nx = nown[0], ny = nown[1], nz = nown[2], fn = sm.n.grad(x & 3, ty + 1, tz + 1);
     const bool flag = fn > evap;
-    const R rhoN = PHI(x, ty + 2, tz + 2);
-    // CSF surface tension from the curvature of the normal field (:624-667)
-    R fx = R(0), fy = R(0), fz = R(0);
-    if (flag && (!SOLIDX || pp <= 0)) {
-      // d_ba = sum_i w_i c_ia n_b(x + c_i) (:635-660), over the nine opposite
-      // pairs: w_i c_ia (n_b(x + c_i) - n_b(x - c_i))
-      R d00 = 0, d01 = 0, d02 = 0, d10 = 0, d11 = 0, d12 = 0, d20 = 0, d21 = 0, d22 = 0;
-      static_for<9>([&](auto kc) {
-        constexpr int i = PREP(decltype(kc)::value);
-        const NormalV<R> p = sm.n[(x + CX(i)) & 3][ty + 1 + CY(i)][tz + 1 + CZ(i)];
-        const NormalV<R> m = sm.n[(x - CX(i)) & 3][ty + 1 - CY(i)][tz + 1 - CZ(i)];
-        const R a = p.x - m.x, b = p.y - m.y, c = p.z - m.z;
-        if (CX(i)) { constexpr double k = W(i) * CX(i); d00 = d00 + R(k) * a; d10 = d10 + R(k) * b; d20 = d20 + R(k) * c; }
-        if (CY(i)) { constexpr double k = W(i) * CY(i); d01 = d01 + R(k) * a; d11 = d11 + R(k) * b; d21 = d21 + R(k) * c; }
-        if (CZ(i)) { constexpr double k = W(i) * CZ(i); d02 = d02 + R(k) * a; d12 = d12 + R(k) * b; d22 = d22 + R(k) * c; }
+    if constexpr (sizeof(R) == 8) {
+      auto ld = [&](auto ic) -> R {   // f[i]; returns the red population
+        constexpr int i = decltype(ic)::value;
+        R r;
+        Codec<S>::template load_fr<i>(pin_, N, L, rref, f[i], r);
+        return r;
+      };
+#define SYM_LD(i) ld(std::integral_constant<int, i>{})
+      // red density, added in the order to_moments adds the totals: a pure red
+      // node (r = f) gets sr = rho exactly
+      const R rest = SYM_LD(0);
+      const R rx = SYM_LD(1) + SYM_LD(2), ry = SYM_LD(3) + SYM_LD(4), rz = SYM_LD(5) + SYM_LD(6);
+      const R rxp = SYM_LD(7) + SYM_LD(10), rxm = SYM_LD(8) + SYM_LD(9);
+      const R rzp = SYM_LD(11) + SYM_LD(14), rzm = SYM_LD(12) + SYM_LD(13);
+      const R ryp = SYM_LD(15) + SYM_LD(18), rym = SYM_LD(16) + SYM_LD(17);
+#undef SYM_LD
+      sr = rest + (rx + ry + rz) + ((rxp + rxm) + (rzp + rzm) + (ryp + rym));
+      Moments<R> m;
+      to_moments<R, R>(f, m);
+      rho = m.rho;
+      sb = rho - sr;
+      R su, sq;
+      node_rates_fused<R>(P, np, PHI(x, ty + 2, tz + 2), rho, irho, su, sq);
+      // CSF surface tension from the curvature of the normal field (:624-667)
+      R fx = R(0), fy = R(0), fz = R(0);
+      if (flag && (!SOLIDX || pp <= 0)) {
+        const R kurv = curvature<R, R>(
+            [&](auto ic, R (&d)[3]) {
+              constexpr int i = decltype(ic)::value;
+              R p[3], q[3];
+              sm.n.get((x + CX(i)) & 3, ty + 1 + CY(i), tz + 1 + CZ(i), p);
+              sm.n.get((x - CX(i)) & 3, ty + 1 - CY(i), tz + 1 - CZ(i), q);
+              d[0] = p[0] - q[0]; d[1] = p[1] - q[1]; d[2] = p[2] - q[2];
+            },
+            nx, ny, nz);
+        const R val = np.half_sigma * kurv * fn;
+        fx = val * nx; fy = val * ny; fz = val * nz;
+      }
+      fx = fx + rho * np.body[0];
+      fy = fy + rho * np.body[1];
+      fz = fz + rho * np.body[2];
+      const R ux = (m.jx + R(0.5) * fx) * irho, uy = (m.jy + R(0.5) * fy) * irho, uz = (m.jz + R(0.5) * fz) * irho;
+      relax<R, R>(m, ux, uy, uz, fx, fy, fz, su, np.s_e > R(0) ? np.s_e : su, np.s_eps > R(0) ? np.s_eps : su,
+                  np.s_q > R(0) ? np.s_q : sq, np.s_pi > R(0) ? np.s_pi : su, np.s_m > R(0) ? np.s_m : sq);
+      from_moments<R, R>(m, f);
+    } else {
+      sr = R(0);
+      rho = R(0);
+      unroll19([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        R r;
+        Codec<S>::template load_fr<i>(pin_, N, L, rref, f[i], r);
+        sr = sr + r;
+        rho = rho + f[i];
       });
-      d00 *= R(3); d01 *= R(3); d02 *= R(3); d10 *= R(3); d11 *= R(3); d12 *= R(3);
-      d20 *= R(3); d21 *= R(3); d22 *= R(3);
-      const R kurv = nx * ny * (d10 + d01) + nx * nz * (d20 + d02) + ny * nz * (d12 + d21) -
-                     (ny * ny + nz * nz) * d00 - (nx * nx + nz * nz) * d11 - (nx * nx + ny * ny) * d22;
-      const R val = R(0.5) * R(P.sigma) * kurv;
-      fx = val * (fn * nx); fy = val * (fn * ny); fz = val * (fn * nz);
+      sb = rho - sr;
+      R ux = R(0), uy = R(0), uz = R(0);
+#pragma unroll
+      for (int i = 0; i < 19; i++) {
+        if (CX(i)) ux = ux + f[i] * R(CX(i));
+        if (CY(i)) uy = uy + f[i] * R(CY(i));
+        if (CZ(i)) uz = uz + f[i] * R(CZ(i));
+      }
+      irho = qdiv<R>(R(1), rho);
+      ux = ux * irho; uy = uy * irho; uz = uz * irho;
+      const R rhoN = PHI(x, ty + 2, tz + 2);
+      // CSF surface tension from the curvature of the normal field (:624-667)
+      R fx = R(0), fy = R(0), fz = R(0);
+      if (flag && (!SOLIDX || pp <= 0)) {
+        // d_ba = sum_i w_i c_ia n_b(x + c_i) (:635-660), over the nine opposite
+        // pairs: w_i c_ia (n_b(x + c_i) - n_b(x - c_i))
+        R d00 = 0, d01 = 0, d02 = 0, d10 = 0, d11 = 0, d12 = 0, d20 = 0, d21 = 0, d22 = 0;
+        static_for<9>([&](auto kc) {
+          constexpr int i = PREP(decltype(kc)::value);
+          R p[3], q[3];
+          sm.n.get((x + CX(i)) & 3, ty + 1 + CY(i), tz + 1 + CZ(i), p);
+          sm.n.get((x - CX(i)) & 3, ty + 1 - CY(i), tz + 1 - CZ(i), q);
+          const R a = p[0] - q[0], b = p[1] - q[1], c = p[2] - q[2];
+          if (CX(i)) { constexpr double k = W(i) * CX(i); d00 = d00 + R(k) * a; d10 = d10 + R(k) * b; d20 = d20 + R(k) * c; }
+          if (CY(i)) { constexpr double k = W(i) * CY(i); d01 = d01 + R(k) * a; d11 = d11 + R(k) * b; d21 = d21 + R(k) * c; }
+          if (CZ(i)) { constexpr double k = W(i) * CZ(i); d02 = d02 + R(k) * a; d12 = d12 + R(k) * b; d22 = d22 + R(k) * c; }
+        });
+        d00 *= R(3); d01 *= R(3); d02 *= R(3); d10 *= R(3); d11 *= R(3); d12 *= R(3);
+        d20 *= R(3); d21 *= R(3); d22 *= R(3);
+        const R kurv = nx * ny * (d10 + d01) + nx * nz * (d20 + d02) + ny * nz * (d12 + d21) -
+                       (ny * ny + nz * nz) * d00 - (nx * nx + nz * nz) * d11 - (nx * nx + ny * ny) * d22;
+        const R val = R(0.5) * R(P.sigma) * kurv;
+        fx = val * (fn * nx); fy = val * (fn * ny); fz = val * (fn * nz);
+      }
+      fx = fx + rho * R(P.body[0]);
+      fy = fy + rho * R(P.body[1]);
+      fz = fz + rho * R(P.body[2]);
+      const R hirho = R(0.5) * irho;
+      ux = ux + fx * hirho;
+      uy = uy + fy * hirho;
+      uz = uz + fz * hirho;
+      mrt_collide_pairs<R>(P, f, rho, ux, uy, uz, fx, fy, fz, rhoN);
     }
-    fx = fx + rho * R(P.body[0]);
-    fy = fy + rho * R(P.body[1]);
-    fz = fz + rho * R(P.body[2]);
-    const R hirho = R(0.5) * irho;
-    ux = ux + fx * hirho;
-    uy = uy + fy * hirho;
-    uz = uz + fz * hirho;
-    mrt_collide_pairs<R>(P, f, rho, ux, uy, uz, fx, fy, fz, rhoN);
     // post-collision populations for the momentum exchange (:1241-1243), read
     // only next to particles (pout = particle id); wall planes (ids > par)
     // need none, and a handle without particles holds no ffi array
@@ -673,7 +747,9 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
     // two coefficients express once per node
     const bool rzero = sr <= evap, bzero = sb <= evap;
     const R ratio = bzero ? R(1) : (rzero ? R(0) : sr * irho);
-    const R coef = (bzero || rzero || !flag) ? R(0) : sr * sb * irho * R(P.beta);
+    const R coef = (bzero || rzero || !flag) ? R(0) : sr * sb * irho * np.beta;
+    // beta rhoR rhoB / rho times a diagonal link's weight, along each axis
+    [[maybe_unused]] const R cd = coef * R(1.0 / 36.0), cnx = cd * nx, cny = cd * ny, cnz = cd * nz;
     // rigid-body velocity of particle pp at this node (curve :1009-1014), for
     // the links that bounce back from it
     R uw0 = R(0), uw1 = R(0), uw2 = R(0);
@@ -698,8 +774,20 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
       constexpr int i = PUSH_ORDER(k);
       constexpr int a = CX(i) + 1, b = CY(i) + 1;
       [&] {
-        R r = ratio * f[i];
-        if (i > 0) r = r + coef * R(W(i)) * (nx * R(CX(i)) + ny * R(CY(i)) + nz * R(CZ(i)));
+        R r;
+        if constexpr (sizeof(R) == 4) {
+          r = ratio * f[i];
+          if (i > 0) r = r + coef * R(W(i)) * (nx * R(CX(i)) + ny * R(CY(i)) + nz * R(CZ(i)));
+        } else if constexpr (i == 0) {
+          r = ratio * f[i];
+        } else if constexpr (i < 7) {
+          constexpr double c = 2 * (CX(i) + CY(i) + CZ(i));   // twice the diagonal weight
+          r = vfma(ratio, f[i], R(c) * (CX(i) ? cnx : (CY(i) ? cny : cnz)));
+        } else {
+          constexpr int s1 = CX(i) ? CX(i) : CY(i), s2 = CZ(i) ? CZ(i) : CY(i);   // the two axes of the link
+          const R c1 = CX(i) ? cnx : cny, c2 = CZ(i) ? cnz : cny;
+          r = vfma(ratio, f[i], s1 > 0 ? (s2 > 0 ? c1 + c2 : c1 - c2) : (s2 > 0 ? c2 - c1 : -(c1 + c2)));
+        }
         const unsigned T = L + (CX(i) > 0 ? oxp : (CX(i) < 0 ? oxm : 0)) +
                            (CY(i) > 0 ? oyp : (CY(i) < 0 ? oym : 0)) + (CZ(i) > 0 ? ozp : (CZ(i) < 0 ? ozm : 0));
         if (!act) return;

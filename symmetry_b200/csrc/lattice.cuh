@@ -80,6 +80,14 @@ __host__ __device__ __forceinline__ constexpr double MNORM(int r) {
 __host__ __device__ __forceinline__ constexpr double MINV(int i, int j) { return MROW(j, i) / MNORM(j); }
 
 // ---------------------------------------------------------------------------
+// What the fused path's node arithmetic reads, in the type it computes in (a
+// conversion from FP64 per node and parameter costs more than the arithmetic
+// it feeds).  su, sq: the rates of a node when both colours have the same
+// viscosity (same_nu), else taken from the node's phase field.
+template <typename R>
+struct NodeParams {
+  R half_sigma, beta, evap, body[3], inu_r, inu_b, s_e, s_eps, s_q, s_pi, s_m, su, sq;
+};
 // Device view of the parameters (filled on the host from sym_params).
 struct DevParams {
   int nx, ny, nz;
@@ -96,8 +104,15 @@ struct DevParams {
   double body[3];
   double rad, mass, inertia, fg, alpha, evap;
   double sin_cita, cos_cita;   // of the contact angle (fused path)
-  double inu_r, inu_b;     // 1/nu_r, 1/nu_b (fused path)
+  int same_nu;             // both colours have the same viscosity
+  NodeParams<double> nd;   // fused path
+  NodeParams<float> nf;
 };
+template <typename R>
+__device__ __forceinline__ const NodeParams<R>& node_params(const DevParams& P) {
+  if constexpr (sizeof(R) == 8) return P.nd;
+  else return P.nf;
+}
 
 template <typename T>
 __device__ __forceinline__ T wrapi(T v, T n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
@@ -205,7 +220,7 @@ template <typename R>
 __device__ __forceinline__ void node_rates_fast(const DevParams& P, R rhoN, R& su, R& se, R& seps, R& sq, R& spi,
                                                 R& sm) {
   const R ph = fmin(fmax(rhoN, R(-1)), R(1));
-  const R D = (R(1) + ph) * R(P.inu_r) + (R(1) - ph) * R(P.inu_b);
+  const R D = (R(1) + ph) * R(P.nd.inu_r) + (R(1) - ph) * R(P.nd.inu_b);
   su = qdiv<R>(R(2) * D, R(12) + D);
   const R sq_ = qdiv<R>(R(8) * (R(2) - su), R(8) - su);
   se = P.s_e > 0 ? R(P.s_e) : su;
@@ -253,7 +268,7 @@ __device__ __forceinline__ void mrt_collide(const DevParams& P, R f[19], R rho, 
   }
 }
 
-// The same collision in the opposite-pair basis (fused path).  Row r of M is
+// The same collision in the opposite-pair basis (fused path, FP32 arithmetic).  Row r of M is
 // even (M(r,opc(c)) = M(r,c)) or odd (= -M(r,c)) under velocity reversal, so
 // with p_k = f_i + f_opc(i) and q_k = f_i - f_opc(i) over the 9 pairs the even
 // moments need only p (and f_0) and the odd ones only q; back-transformed,

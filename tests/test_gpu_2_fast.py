@@ -61,6 +61,19 @@ def test_fast_fp64_ragged_periodic_domain():
     assert max(e.values()) <= 1e-10, e
 
 
+@pytest.mark.parametrize("ratio,rates", [(5.0, {}), (0.2, dict(s_e=1.1, s_q=1.3)), (1.0, dict(s_eps=0.9, s_m=1.6))])
+def test_fast_fp64_two_viscosities_and_rates(ratio, rates):
+    """Node-local rates from the phase field (nu_r != nu_b) and from the
+    runtime inputs, against the oracle: the FP64 parity bound, 1e-10."""
+    w = configs.c1_thread(nx=21, ny=18, nz=40, radius=5.0)
+    w.params.nu_b = w.params.nu_r / ratio
+    for k in ("s_e", "s_eps", "s_q", "s_pi", "s_m"):
+        setattr(w.params, k, rates.get(k, 0.0))
+    o, L = fast_run(w, 200)
+    e = errors(o, L)
+    assert max(e.values()) <= 1e-10, e
+
+
 def test_fast_fp64_walls_only():
     w = driven_channel()
     o, L = fast_run(w, 300)
