@@ -21,7 +21,7 @@
 #include <string>
 #include <vector>
 #include "state.cuh"
-#include "fused.cuh"
+#include "paired.cuh"
 
 using namespace symb200;
 using namespace symb200::fused;
@@ -43,8 +43,8 @@ struct DomainDesc {
   Ref* rr_new;
   void* acc;            // accumulated colour densities of the next step (see fused.cuh)
   int* status;
-  const CUtensorMap* tm_phi;    // TMA descriptors (device copies) of this step's phase field
-  const CUtensorMap* tm_ref;   // and reference-pair arrays
+  const CUtensorMap* tm_phi;   // TMA descriptors (device copies) of this step's phase field
+  const CUtensorMap* tm_ref;   // and reference pairs
   int solid;
   int pad_;
 };
@@ -82,15 +82,50 @@ __global__ void __launch_bounds__(256) k_finalize_batch(const DomainDesc* __rest
     finalize_nodes<S, false, 1>(D.P, D.pd, (AT*)D.acc, (R*)D.phic, D.walls_all, D.rr_new, D.status, L);
 }
 
+// What the collide kernel reads of one domain.
 template <typename S>
-__global__ void __launch_bounds__(kTPB<S>, collide_ctas<S>()) k_collide_batch(const DomainDesc* __restrict__ descs,
-                                                           const TileEntry* __restrict__ tiles, int ntiles,
-                                                           int* __restrict__ counter) {
-  using R = typename Codec<S>::R;
+struct TileDesc {
+  TileParams<typename Codec<S>::R> P;
+  Pad pd;
+  const S* pin;
+  S* pnext;
+  const int32_t *walls, *walls_all, *pout;
+  const sym_particles* Sp;
+  double* ffi;
+  const Ref* rr_old;
+  typename Acc<typename Codec<S>::R>::T* acc;
+  int* status;
+  const CUtensorMap *tm_phi, *tm_ref;
+  int solid;
+};
+// The descriptors of a batch of up to kParamDomains domains are kernel
+// parameters: read from the constant bank they cost no registers and nothing
+// stored can alias them.  (Staged in shared memory, their pointers and
+// parameters took registers that the node arithmetic then spilled: one 16-bit
+// domain of 128x128x256 took 328 us in a batch and 163 alone.)  Larger batches
+// read a tile's descriptor from global memory into shared memory.
+template <typename S>
+constexpr int kParamDomains = 32 * 1000 / (int)sizeof(TileDesc<S>) < 128 ? 32 * 1000 / (int)sizeof(TileDesc<S>) : 128;
+constexpr int kFewDomains = 16;   // a smaller table, copied with each launch
+template <typename S, int N>
+struct DescTable {
+  TileDesc<S> d[N];
+};
+template <typename S>
+__device__ __forceinline__ void run_tile(const TileDesc<S>& D, const TileEntry& e, TileSmem<S>& sm, unsigned& nload) {
+  collide_any<S, true>(D.P, D.pd, as_global(D.pin), as_global(D.pnext), as_global(D.walls), as_global(D.walls_all),
+                       as_global(D.pout), as_global(D.Sp), as_global(D.ffi), as_global(D.rr_old), as_global(D.acc),
+                       as_global(D.status), D.tm_phi, D.tm_ref, e.z0, e.y0, e.xa, e.xb, sm, nload, D.solid != 0);
+}
+// N = 0: descriptors in global memory
+template <typename S, int N>
+__global__ void __launch_bounds__(kTPB, collide_ctas<S>())
+    k_collide_batch(const __grid_constant__ DescTable<S, N ? N : 1> table, const TileDesc<S>* __restrict__ descs,
+                    const TileEntry* __restrict__ tiles, int ntiles, int* __restrict__ counter) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  Smem<S>& sm = smem_view<S>(smem_raw);
+  TileSmem<S>& sm = smem_view<S>(smem_raw);
   __shared__ int s_tile;
-  __shared__ __align__(16) DomainDesc s_desc;
+  [[maybe_unused]] __shared__ __align__(16) TileDesc<S> s_desc;
   collide_init_barriers<S>(sm);
   unsigned nload = 0;
   for (;;) {
@@ -99,20 +134,15 @@ __global__ void __launch_bounds__(kTPB<S>, collide_ctas<S>()) k_collide_batch(co
     const int t = s_tile;
     if (t >= ntiles) break;
     const TileEntry e = tiles[t];
-    {  // stage the tile's domain descriptor in shared memory
+    if constexpr (N > 0) {
+      run_tile<S>(table.d[e.dom], e, sm, nload);
+    } else {
       const int* src = reinterpret_cast<const int*>(&descs[e.dom]);
       int* dst = reinterpret_cast<int*>(&s_desc);
-      for (int k = threadIdx.x; k < (int)(sizeof(DomainDesc) / sizeof(int)); k += kTPB<S>) dst[k] = src[k];
+      for (int k = threadIdx.x; k < (int)(sizeof(TileDesc<S>) / sizeof(int)); k += kTPB) dst[k] = src[k];
+      __syncthreads();
+      run_tile<S>(s_desc, e, sm, nload);
     }
-    __syncthreads();
-    const DomainDesc& D = s_desc;
-    using AT = typename Acc<R>::T;
-    // one compiled variant for every tile (solid handling switched per
-    // domain): the instruction working set of the persistent kernel stays
-    // that of one variant
-    collide_tile<S, true>(D.P, D.pd, (const S*)D.pin, (S*)D.pnext, (const R*)D.phic, D.walls, D.walls_all, D.pout,
-                          D.Sp, D.ffi, D.rr_old, D.rr_new, (AT*)D.acc, D.status, D.tm_phi, D.tm_ref, e.z0, e.y0,
-                          e.xa, e.xb, sm, nload, D.solid != 0);
     __syncthreads();
   }
 }
@@ -122,9 +152,18 @@ __global__ void __launch_bounds__(kTPB<S>, collide_ctas<S>()) k_collide_batch(co
 template <typename S>
 int set_batch_smem(int device, int* per_sm, int* sms) {
   const int shm = (int)smem_bytes<S>();
-  if (cudaFuncSetAttribute(k_collide_batch<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm) != cudaSuccess)
+  auto set = [&](auto kern) {
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, shm) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kTPB, shm) != cudaSuccess)
+      return false;
+    *per_sm = std::min(*per_sm, n);
+    return true;
+  };
+  *per_sm = 32;
+  if (!set(k_collide_batch<S, kFewDomains>) || !set(k_collide_batch<S, kParamDomains<S>>) ||
+      !set(k_collide_batch<S, 0>))
     return SYM_ERR_CUDA;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_collide_batch<S>, kTPB<S>, shm);
   cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device);
   *per_sm = std::max(1, *per_sm);
   *sms = std::max(1, *sms);
@@ -142,6 +181,8 @@ struct sym_batch {
   std::vector<int> built_cur, built_pc;   // domain parities graph 0 was built for
   int steps_since_build = 0;
   DomainDesc* d_desc[2] = {nullptr, nullptr};
+  std::vector<DomainDesc> hdesc[2];
+  void* d_tdesc[2] = {nullptr, nullptr};   // collide descriptors (TileDesc) of a batch too large for parameters
   CUtensorMap* d_tmaps = nullptr;   // [parity][domain][phase field, reference pairs]
   int2* d_blk = nullptr;          // phase block -> (domain, block in domain)
   TileEntry* d_tiles = nullptr;
@@ -185,6 +226,8 @@ void free_tables(sym_batch* b) {
   b->sparse = nullptr;
   for (int k = 0; k < 2; k++)
     if (b->d_desc[k]) { cudaFree(b->d_desc[k]); b->d_desc[k] = nullptr; }
+  for (int k = 0; k < 2; k++)
+    if (b->d_tdesc[k]) { cudaFree(b->d_tdesc[k]); b->d_tdesc[k] = nullptr; }
   if (b->d_blk) { cudaFree(b->d_blk); b->d_blk = nullptr; }
   if (b->d_tiles) { cudaFree(b->d_tiles); b->d_tiles = nullptr; }
   if (b->d_tmaps) { cudaFree(b->d_tmaps); b->d_tmaps = nullptr; }
@@ -216,6 +259,37 @@ DomainDesc make_desc(sym_handle* h, int cur, int pc) {
   return d;
 }
 
+template <typename S>
+TileDesc<S> tile_desc(const DomainDesc& d) {
+  using R = typename Codec<S>::R;
+  TileDesc<S> t;
+  t.P = tile_params<R>(d.P);
+  t.pd = d.pd;
+  t.pin = (const S*)d.pin; t.pnext = (S*)d.pnext;
+  t.walls = d.walls; t.walls_all = d.walls_all; t.pout = d.pout;
+  t.Sp = d.Sp; t.ffi = d.ffi; t.rr_old = d.rr_old;
+  t.acc = (typename Acc<R>::T*)d.acc;
+  t.status = d.status; t.tm_phi = d.tm_phi; t.tm_ref = d.tm_ref; t.solid = d.solid;
+  return t;
+}
+template <typename S, int N>
+void launch_collide_params(sym_batch* b, int k) {
+  DescTable<S, N> t;
+  std::memset(&t, 0, sizeof t);
+  for (size_t i = 0; i < b->hdesc[k].size(); i++) t.d[i] = tile_desc<S>(b->hdesc[k][i]);
+  k_collide_batch<S, N><<<b->grid, kTPB, smem_bytes<S>(), b->st>>>(t, nullptr, b->d_tiles, b->ntiles,
+                                                                   b->d_counter + k);
+}
+template <typename S>
+void launch_collide(sym_batch* b, int k) {
+  const int n = (int)b->doms.size();
+  if (n <= kFewDomains) return launch_collide_params<S, kFewDomains>(b, k);
+  if (n <= kParamDomains<S>) return launch_collide_params<S, kParamDomains<S>>(b, k);
+  static const DescTable<S, 1> none = {};
+  k_collide_batch<S, 0><<<b->grid, kTPB, smem_bytes<S>(), b->st>>>(none, (const TileDesc<S>*)b->d_tdesc[k], b->d_tiles,
+                                                                   b->ntiles, b->d_counter + k);
+}
+
 // One batch step on b->st (captured into a graph, or eager when timing):
 // descriptor table k, domain i at buffer parity (built_cur[i] + k) & 1.
 // ev (optional, eager only): 4 events recorded before the phase launch, after
@@ -231,9 +305,7 @@ int enqueue_batch_step(sym_batch* b, int k, cudaEvent_t* ev) {
   if (int e = sparse_enqueue(b->sparse, k, b->st)) return berr(b, e, "sparse step");
   if (ev) cudaEventRecord(ev[2], b->st);
   cudaMemsetAsync(b->d_counter + k, 0, sizeof(int), b->st);
-  using R = typename Codec<S>::R;
-  k_collide_batch<S><<<b->grid, kTPB<S>, smem_bytes<S>(), b->st>>>(b->d_desc[k], b->d_tiles, b->ntiles,
-                                                                  b->d_counter + k);
+  launch_collide<S>(b, k);
   if (int e = sparse_enqueue_post(b->sparse, k, b->st)) return berr(b, e, "interpolated bounce-back");
   if (ev) cudaEventRecord(ev[3], b->st);
   return bcuda(b, cudaGetLastError(), "batch step");
@@ -243,6 +315,17 @@ int enqueue_any(sym_batch* b, int k, cudaEvent_t* ev) {
   return b->storage == SYM_STORE_FP64 ? enqueue_batch_step<double>(b, k, ev)
        : b->storage == SYM_STORE_FP32 ? enqueue_batch_step<float>(b, k, ev)
                                       : enqueue_batch_step<__half>(b, k, ev);
+}
+
+// the collide descriptors of a batch too large for kernel parameters
+template <typename S>
+int upload_tdesc(sym_batch* b, int k) {
+  if ((int)b->doms.size() <= kParamDomains<S>) return SYM_OK;
+  std::vector<TileDesc<S>> t;
+  for (const DomainDesc& d : b->hdesc[k]) t.push_back(tile_desc<S>(d));
+  if (int e = bcuda(b, cudaMalloc(&b->d_tdesc[k], sizeof(TileDesc<S>) * t.size()), "collide descriptors")) return e;
+  return bcuda(b, cudaMemcpy(b->d_tdesc[k], t.data(), sizeof(TileDesc<S>) * t.size(), cudaMemcpyHostToDevice),
+               "collide descriptors");
 }
 
 // (re)build the descriptor and tile tables and both step graphs
@@ -307,6 +390,10 @@ int build(sym_batch* b) {
   for (int k = 0; k < 2; k++) {
     if (int e = bcuda(b, cudaMalloc(&b->d_desc[k], sizeof(DomainDesc) * n), "descriptors")) return e;
     cudaMemcpyAsync(b->d_desc[k], desc[k].data(), sizeof(DomainDesc) * n, cudaMemcpyHostToDevice, b->st);
+    b->hdesc[k] = desc[k];
+    const int e = b->storage == SYM_STORE_FP64 ? upload_tdesc<double>(b, k)
+                : b->storage == SYM_STORE_FP32 ? upload_tdesc<float>(b, k) : upload_tdesc<__half>(b, k);
+    if (e) return e;
   }
   std::vector<int2> blk((size_t)off[n]);
   for (int i = 0; i < n; i++)

@@ -486,6 +486,9 @@ int sym_set_particles(sym_handle* h, const sym_particles* s) {
   if (int e = guard(h)) return e;
   if (!s) return set_error(h, SYM_ERR_PARAM, "null particles");
   cudaMemcpyAsync(h->dpart, s, sizeof(sym_particles), cudaMemcpyHostToDevice, h->st);
+  // a particle moved away by hand leaves its masks behind until set_walls
+  if (h->fast.valid)
+    if (int e = fast_solid_tiles(h)) return e;
   return check_cuda(h, cudaStreamSynchronize(h->st), "set_particles");
 }
 

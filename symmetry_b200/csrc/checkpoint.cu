@@ -183,8 +183,9 @@ int sym_checkpoint_load(sym_handle* h, const char* path) {
     void* dst = s.dev ? s.dev : (void*)h->dpart;
     if (int e = check_cuda(h, cudaMemcpy(dst, buf.data(), n, cudaMemcpyHostToDevice), "checkpoint write")) return e;
   }
-  if (fused) {   // the momentum link lists follow from the restored masks
+  if (fused) {   // the momentum link lists and solid tiles follow from the restored masks
     if (int e = sparse_links_build(h, h->st)) return set_error(h, e, "checkpoint: momentum link lists");
+    if (int e = fast_solid_tiles(h)) return e;
     if (int e = check_cuda(h, cudaStreamSynchronize(h->st), "checkpoint links")) return e;
   }
   h->fast.valid = fused;

@@ -31,7 +31,7 @@
 #include <utility>
 #include <vector>
 #include "state.cuh"
-#include "fused.cuh"
+#include "paired.cuh"
 #include "particles.cuh"
 
 namespace symb200 {
@@ -121,13 +121,11 @@ int enqueue_step(sym_handle* h, int cur, int pc, cudaEvent_t* ev) {
   const CUtensorMap& tr = h->fast.tm_ref[pc];
   if (ev) cudaEventRecord(ev[2], h->st);
   if (solid)
-    k_collide<S, true><<<grid, kTPB<S>, shm, h->st>>>(P, pd, pin_, pnext, phic, h->walls, h->walls_all, h->pout,
-                                                  h->dpart, h->ffi, rr_old(h, pc), rr_new(h, pc), accbuf<S>(h),
-                                                  h->fast.status, tp, tr, xc);
+    k_collide<S, true><<<grid, kTPB, shm, h->st>>>(tile_params<R>(P), pd, pin_, pnext, h->walls, h->walls_all, h->pout, h->dpart,
+                                                   h->ffi, rr_old(h, pc), accbuf<S>(h), h->fast.status, tp, tr, xc);
   else
-    k_collide<S, false><<<grid, kTPB<S>, shm, h->st>>>(P, pd, pin_, pnext, phic, h->walls, h->walls_all, h->pout,
-                                                   h->dpart, h->ffi, rr_old(h, pc), rr_new(h, pc), accbuf<S>(h),
-                                                   h->fast.status, tp, tr, xc);
+    k_collide<S, false><<<grid, kTPB, shm, h->st>>>(tile_params<R>(P), pd, pin_, pnext, h->walls, h->walls_all, h->pout, h->dpart,
+                                                    h->ffi, rr_old(h, pc), accbuf<S>(h), h->fast.status, tp, tr, xc);
   if (int e = sparse_enqueue_post(h->fast.sparse, cur, h->st)) return set_error(h, e, "interpolated bounce-back");
   if (ev) cudaEventRecord(ev[3], h->st);
   return check_cuda(h, cudaGetLastError(), "fast step");
@@ -208,6 +206,12 @@ int fast_alloc(sym_handle* h) {
     if (int e = dev_carve(h, (void**)&F.links, segs * 256 * sizeof(uint2))) return e;
     if (int e = dev_carve(h, (void**)&F.nlinks, segs * sizeof(int))) return e;
   }
+  if (has_solids(h)) {
+    h->dp.tiles_y = (h->dp.ny + tile_rows(F.storage) - 1) / tile_rows(F.storage);
+    h->dp.tiles_z = (h->dp.nz + BZ - 1) / BZ;
+    if (int e = dev_carve(h, (void**)&F.solid_tiles, (size_t)h->dp.nx * h->dp.tiles_y * h->dp.tiles_z)) return e;
+    h->dp.solid_tiles = F.solid_tiles;
+  }
   if (int e = dev_carve(h, (void**)&F.status, sizeof(int))) return e;
   if (h->planning) return SYM_OK;
   F.bytes = h->bytes - before;
@@ -244,6 +248,8 @@ void fast_free(sym_handle* h) {
       dev_release(h, (void*)F.status);
       dev_release(h, (void*)F.links);
       dev_release(h, (void*)F.nlinks);
+      dev_release(h, (void*)F.solid_tiles);
+      F.solid_tiles = nullptr;
       F.acc = nullptr;
       F.status = nullptr;
       F.links = nullptr;
@@ -283,7 +289,37 @@ int fast_import(sym_handle* h) {
       k_import_phi<float><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, h->rhoN, F.phif[1]);
   }
   if (int e = sparse_links_build(h, h->st)) return set_error(h, e, "momentum link lists");
+  if (int e = fast_solid_tiles(h)) return e;
   return check_cuda(h, cudaStreamSynchronize(h->st), "fast import");
+}
+
+namespace {
+// one block per tile plane
+__global__ void __launch_bounds__(128) k_solid_tiles(DevParams P, int rows, const int32_t* __restrict__ walls_all,
+                                                     const int32_t* __restrict__ pout, unsigned char* out) {
+  const int tz = blockIdx.x, ty = blockIdx.y, x = blockIdx.z;
+  bool any = false;
+  for (int t = threadIdx.x; t < (rows + 2) * (BZ + 2); t += 128) {
+    const int y = ty * rows - 1 + t / (BZ + 2), z = tz * BZ - 1 + t % (BZ + 2);
+    if (y > P.ny || z > P.nz) continue;
+    const long long L = lin(P, x, wrapi(y, P.ny), wrapi(z, P.nz));
+    any |= walls_all[L] > 0 || pout[L] != 0;
+  }
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) out[((size_t)x * P.tiles_y + ty) * P.tiles_z + tz] = any ? 1 : 0;
+}
+}  // namespace
+int fast_solid_tiles(sym_handle* h) {
+  if (!h->fast.solid_tiles) return SYM_OK;
+  const DevParams& P = h->dp;
+  for (int x0 = 0; x0 < P.nx; x0 += 65535) {   // grid.z is at most 65535
+    DevParams Q = P;
+    const size_t off = (size_t)x0 * P.ny * P.nz;
+    k_solid_tiles<<<dim3(P.tiles_z, P.tiles_y, std::min(65535, P.nx - x0)), 128, 0, h->st>>>(
+        Q, tile_rows(h->fast.storage), h->walls_all + off, h->pout + off,
+        h->fast.solid_tiles + (size_t)x0 * P.tiles_y * P.tiles_z);
+  }
+  return check_cuda(h, cudaGetLastError(), "solid tiles");
 }
 
 // fused -> canonical: populations, the last pin-filled phi as rho_N, and the

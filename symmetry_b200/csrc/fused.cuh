@@ -18,6 +18,15 @@ namespace fused {
 constexpr int BZ = 32;   // tile width along z: one warp per row
 constexpr int XCHUNK = 32;   // most x planes marched by one CTA
 
+// A pointer read from a descriptor, marked as one to global memory: its accesses
+// are then global loads and stores (through a pointer of unknown space they are
+// generic ones, which also wait for the shared-memory writes around them:
+// 16-bit collide of a one-domain batch 328 us against 163 alone).
+template <typename T>
+__device__ __forceinline__ T* as_global(T* p) {
+  return static_cast<T*>(__cvta_global_to_generic(__cvta_generic_to_global(p)));
+}
+
 // ---- halo-padded phase field -----------------------------------------------------
 struct Pad {
   int nxp, nyp, nzp;
@@ -346,8 +355,8 @@ __global__ void __launch_bounds__(256) k_finalize(DevParams P, Pad pd, typename 
 }
 
 // ---- wetting rotation of a node normal (derivatives :535-587) ---------------------
-template <typename R>
-__device__ __forceinline__ void wet_rotate(const DevParams& P, const sym_particles* S, int pp, int x, int y, int z,
+template <typename R, typename PT>
+__device__ __forceinline__ void wet_rotate(const PT& P, const sym_particles* S, int pp, int x, int y, int z,
                                            R& n0, R& n1, R& n2) {
   double nwd[3];
   wall_normal_dev(P, S, pp, x, y, z, nwd);
@@ -368,25 +377,12 @@ __device__ __forceinline__ void wet_rotate(const DevParams& P, const sym_particl
 // (phi x+4 -> slot (x-1)%5, normals x+2 -> (x-2)%4, reference-pair x+4 -> (x-2)%6)
 // are never among them.
 constexpr int kIrrRing = 6;
-// The unit normals and |grad phi| of four planes of a tile, [plane][y][z].  FP32
-// keeps a node's four numbers in one 16-byte access.  FP64 splits them so that
-// a warp's accesses are contiguous (16-byte x, y pairs and 8-byte z: 6 shared
-// memory wavefronts a node's normal for a warp, against 16 of a 32-byte
+// The unit normals and |grad phi| of four planes of a tile, [plane][y][z], split
+// so that a warp's accesses are contiguous (16-byte x, y pairs and 8-byte z: 6
+// shared-memory wavefronts for a warp's normals, against 16 of a 32-byte
 // record); only a node's own |grad phi| is read.
-template <typename R, int ROWS>
-struct NormalTile {
-  float4 v[4][ROWS][BZ + 2];
-  __device__ __forceinline__ void set(int s, int y, int z, R nx, R ny, R nz, R g) {
-    v[s][y][z] = make_float4(nx, ny, nz, g);
-  }
-  __device__ __forceinline__ void get(int s, int y, int z, R (&n)[3]) const {
-    const float4 t = v[s][y][z];
-    n[0] = t.x; n[1] = t.y; n[2] = t.z;
-  }
-  __device__ __forceinline__ R grad(int s, int y, int z) const { return v[s][y][z].w; }
-};
 template <int ROWS>
-struct NormalTile<double, ROWS> {
+struct NormalTile {
   double2 xy[4][ROWS][BZ + 2];
   double z_[4][ROWS][BZ + 2];
   double g[4][ROWS][BZ + 2];
@@ -401,247 +397,242 @@ struct NormalTile<double, ROWS> {
   }
   __device__ __forceinline__ double grad(int s, int y, int z) const { return g[s][y][z]; }
 };
-// Tile height (rows of BZ nodes) of the collide kernels per storage: 16
-// rows for the 16-bit codec, 8 for FP32 and FP64.  Measured on the batched
-// mix: 16 rows (2 CTAs of 512 threads per SM) took the 16-bit collide from
-// 4.79 to 4.28 ms against 8 rows (4 CTAs of 256) -- fewer halo normals, halo
-// bytes and barriers per node -- and changed nothing in FP32; FP64 at 16 rows
-// fits one CTA per SM and was slower (C3: 4.70 against 4.52 ms).
+// Tile height (rows of BZ nodes) of the collide kernels per storage, on 256
+// threads: 8 rows for FP64 (16 would fit one CTA per SM and was slower,
+// 256x256x512: 4.70 against 4.52 ms), 16 for FP32 arithmetic (two nodes a thread,
+// paired.cuh).
 template <typename S>
-constexpr int kBY = std::is_same<S, __half>::value ? 16 : 8;
-template <typename S>
-constexpr int kTPB = BZ * kBY<S>;
+constexpr int kBY = sizeof(S) == 8 ? 8 : 16;
+constexpr int kTPB = 256;
 // the same for a storage mode chosen at run time (SYM_STORE_*)
 inline int tile_rows(int storage) {
   return storage == SYM_STORE_FP16 ? kBY<__half> : (storage == SYM_STORE_FP32 ? kBY<float> : kBY<double>);
 }
-// phi and reference-pair plane tiles ((BY+4) x (BZ+4), z fastest) arrive by TMA:
-// each slot starts on a 128-byte boundary
-template <typename S>
-constexpr int kPlaneTile = (kBY<S> + 4) * (BZ + 4);
-template <typename S>
+// most x planes of a tile
+constexpr int kMaxExtent = 64;
+// phi plane tiles ((BY+4) x (BZ+4), z fastest) arrive by TMA: each slot starts on
+// a 128-byte boundary
 struct Smem {
-  using R = typename Codec<S>::R;
-  static constexpr int BY = kBY<S>;
-  static constexpr int kPhiSlot = (kPlaneTile<S> * (int)sizeof(R) + 127) / 128 * 128 / (int)sizeof(R);
-  static constexpr int kRefSlot = (kPlaneTile<S> * 8 + 127) / 128 * 128 / 8;
-  alignas(128) R phi[5][kPhiSlot];
-  alignas(128) Ref ref[Codec<S>::kRef ? kIrrRing : 1][kRefSlot];   // reference pairs of this step (16-bit storage)
-  alignas(16) NormalTile<R, BY + 2> n;
-  // [cx+1][to row y+1, y-1][colour]: density sums crossing rows (accumulating
-  // storages only; a single element otherwise)
-  R xch[kAccumulate<S> ? 3 : 1][2][2][kAccumulate<S> ? BY : 1][kAccumulate<S> ? BZ : 1];
+  static constexpr int BY = kBY<double>;
+  static constexpr int kTile = (BY + 4) * (BZ + 4);
+  static constexpr int kPhiSlot = (kTile * 8 + 127) / 128 * 128 / 8;
+  alignas(128) double phi[5][kPhiSlot];
+  alignas(16) NormalTile<BY + 2> n;
+  double xch[3][2][2][BY][BZ];   // [cx+1][to row y+1, y-1][colour]: density sums crossing rows
+  // [beside lane 0, beside the last lane][cx+1][cy = 0, +1, -1][colour][row]:
+  // pushes crossing the tile's z edges (cy = +-1 for cx = 0 only)
+  double zx[2][3][3][2][BY];
   uint64_t bar[kIrrRing];   // one mbarrier per plane load, used round robin
+  unsigned char near_solid[kMaxExtent + 2];   // planes xa-1 .. xb
 };
-// dynamic shared memory of the collide kernels: the Smem block on a 128-byte
-// boundary inside the allocation
-template <typename S>
-constexpr size_t smem_bytes() { return sizeof(Smem<S>) + 128; }
-template <typename S>
-__device__ __forceinline__ Smem<S>& smem_view(unsigned char* raw) {
-  const uintptr_t a = (reinterpret_cast<uintptr_t>(raw) + 127) & ~uintptr_t(127);
-  return *reinterpret_cast<Smem<S>*>(a);
+// Whether plane xp of the tile at (z0, y0) may hold a solid or a node next to
+// one: where the masks had any when the fused state was built, and around the
+// particles where they are now (a solid reaches rad from its centre, the nodes
+// next to it one more).  Planes without take no masks: two dependent reads a
+// node and plane made the solid variant 1.2 to 2 times slower than the plain one.
+template <typename R>
+__device__ __forceinline__ bool solid_near(const TileParams<R>& P, const sym_particles* __restrict__ S, int rows, int xp,
+                                           int y0, int z0) {
+  if (P.solid_tiles[((size_t)wrapi(xp, P.nx) * P.tiles_y + y0 / rows) * P.tiles_z + z0 / BZ]) return true;
+  const double reach = P.rad + 2.0;
+  const double yc = y0 + 0.5 * (rows - 1), yh = 0.5 * (rows - 1) + 1.0;
+  const double zc = z0 + 0.5 * (BZ - 1), zh = 0.5 * (BZ - 1) + 1.0;
+  for (int k = 0; k < P.par; k++)
+    if (fabs(disp(P, (double)xp, S->center[k], 0)) <= reach &&
+        fabs(disp(P, yc, S->center[P.par + k], 1)) <= reach + yh &&
+        fabs(disp(P, zc, S->center[2 * P.par + k], 2)) <= reach + zh)
+      return true;
+  return false;
 }
-// the CTA's mbarriers: initialised once per kernel by thread 0
-template <typename S>
-__device__ __forceinline__ void collide_init_barriers(Smem<S>& sm) {
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < kIrrRing; k++) tma::mbar_init(&sm.bar[k], 1);
-    tma::mbar_fence_init();
+// node t of the one-node ring around a tile of `rows` rows, in normal-ring
+// coordinates (the tile's own nodes are y 1 .. rows, z 1 .. BZ): rows 0 and
+// rows + 1, then the two z columns
+__device__ __forceinline__ void ring_node(int t, int rows, int& y, int& z) {
+  if (t < 2 * (BZ + 2)) {
+    y = t < BZ + 2 ? 0 : rows + 1;
+    z = t < BZ + 2 ? t : t - (BZ + 2);
+  } else {
+    t -= 2 * (BZ + 2);
+    y = 1 + t % rows;
+    z = t < rows ? 0 : BZ + 1;
   }
-  __syncthreads();
 }
-// push order of the collide kernel: groups of equal (cx, cy), cz = 0, +1, -1
-// last (velocity numbering of Source1.f90:132-134)
-__host__ __device__ __forceinline__ constexpr int PUSH_ORDER(int k) {
-  constexpr int a[19] = {0, 5, 6, 1, 11, 13, 2, 12, 14, 3, 15, 17, 4, 16, 18, 7, 8, 9, 10};
-  return a[k];
-}
-
-// One tile: the 32(z) x BY(y) footprint at (z0, y0), planes xa..xb-1.  Called
+// One FP64 tile: the 32(z) x 8(y) footprint at (z0, y0), planes xa..xb-1.  Called
 // by the single-domain kernel (tile from blockIdx) and by the batched
-// persistent kernel (tile from the work-tile table).
-template <typename S, bool SOLID>
-__device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, const S* __restrict__ pin_,
-                                             S* __restrict__ pout_, const typename Codec<S>::R* __restrict__ phi,
-                                             const int32_t* __restrict__ walls,
+// persistent kernel (tile from the work-tile table).  solid_rt: solid handling
+// wanted by this domain (the batched kernel compiles one variant and decides
+// per tile).
+//
+// Besides the pushed populations the tile adds up the next step's colour
+// densities.  Per plane the pushes are summed over z by warp shuffles and over
+// y through shared memory; what leaves the tile along z is handed over as ten
+// numbers per row in shared memory, and what leaves along y is a row of the
+// exchange.  The sum a plane sends to each destination node is turned into
+// fixed point and added to the sums of the planes before and after it in
+// registers -- the tile's own nodes by their threads, the one-node ring around
+// it by 168 threads beside that work -- so each node gets one addition per
+// tile and plane.  The totals are integer sums of terms that do not depend on
+// where the march starts or ends: a domain's result is the same bit for bit
+// whatever x extent its tiles have.
+template <bool SOLID>
+__device__ __forceinline__ void collide_tile(const TileParams<double>& P, const double* __restrict__ pin_,
+                                             double* __restrict__ pout_, const int32_t* __restrict__ walls,
                                              const int32_t* __restrict__ walls_all,
                                              const int32_t* __restrict__ pout,
                                              const sym_particles* __restrict__ Sp, double* __restrict__ ffi,
-                                             const Ref* __restrict__ rr_old, const Ref* __restrict__ rr_new,
-                                             typename Acc<typename Codec<S>::R>::T* acc, int* status,
-                                             const CUtensorMap* tm_phi, const CUtensorMap* tm_ref,
-                                             int z0, int y0, int xa, int xb, Smem<S>& sm, unsigned& nload,
+                                             Acc<double>::T* acc, int* status, const CUtensorMap* tm_phi,
+                                             int z0, int y0, int xa, int xb, Smem& sm, unsigned& nload,
                                              bool solid_rt = true) {
-  using R = typename Codec<S>::R;
-  constexpr int BY = kBY<S>, TPB = kTPB<S>, kTile = kPlaneTile<S>;
-  // solid handling: compiled in (SOLID) and wanted by this domain (solid_rt);
-  // the batched kernel compiles one variant and decides per tile
+  using R = double;
+  using A = Acc<double>;
+  using AT = A::T;
+  constexpr int BY = kBY<double>, kRow = BZ + 4;
   const bool SOLIDX = SOLID && solid_rt;
-  constexpr bool ACC = kAccumulate<S>;
-  constexpr bool REF = Codec<S>::kRef;
   const int tz = threadIdx.x % BZ, ty = threadIdx.x / BZ;
-  const unsigned N = (unsigned)P.N;
-  const NodeParams<R>& np = node_params<R>(P);
-  const R evap = np.evap;
   const int sy = P.nz, sx = P.nz * P.ny;   // element strides of y and x
+  const int Ni = sx * P.nx;                // 19 N < 2^31 on the fused path
+  const NodeParams<R>& np = P.np;
+  const R evap = np.evap;
 
-  // phi (and the reference pairs) of plane xp by TMA: one box of (BY+4) x (BZ+4) at the
-  // padded origin (z0, y0, xp+2) -- z0 is a multiple of 32 elements, so the
-  // innermost coordinate is 128-byte aligned; rows past the padded extent read
-  // as zeros.  Plane xp is load number nl0 + xp - (xa - 2) of this CTA, on
-  // mbarrier (number mod 6) with phase parity (number / 6) mod 2.
+  // phi of plane xp by TMA: one box of (BY+4) x (BZ+4) at the padded origin
+  // (z0, y0, xp+2) -- z0 is a multiple of 32 elements, so the innermost
+  // coordinate is 128-byte aligned; rows past the padded extent read as zeros.
+  // Plane xp is load number nl0 + xp - (xa - 2) of this CTA, on mbarrier
+  // (number mod 6) with phase parity (number / 6) mod 2.
   const unsigned nl0 = nload;
   auto load_no = [&](int xp) { return nl0 + (unsigned)(xp - (xa - 2)); };
-  constexpr uint32_t kTx = kTile * (sizeof(R) + (REF ? sizeof(Ref) : 0));
   auto load_phi = [&](int xp) {   // thread 0 only
-    const unsigned q = load_no(xp);
-    uint64_t* bar = &sm.bar[q % kIrrRing];
-    tma::mbar_expect_tx(bar, kTx);
-    tma::load_3d(sm.phi[((xp % 5) + 5) % 5], tm_phi, z0, y0, xp + 2, bar);
-    if (REF) tma::load_3d(sm.ref[(unsigned)(xp + kIrrRing) % kIrrRing], tm_ref, z0, y0, xp + 2, bar);
+    uint64_t* bar = &sm.bar[load_no(xp) % kIrrRing];
+    tma::mbar_expect_tx(bar, Smem::kTile * sizeof(R));
+    tma::load_3d(sm.phi[(unsigned)(xp + 5) % 5u], tm_phi, z0, y0, xp + 2, bar);
   };
   auto wait_phi = [&](int xp) {   // every thread
     const unsigned q = load_no(xp);
     if (!tma::mbar_wait(&sm.bar[q % kIrrRing], (q / kIrrRing) & 1u)) atomicOr(status, 2);
   };
-  auto PHI = [&](int xp, int py, int pz) -> R { return sm.phi[((xp % 5) + 5) % 5][py * (BZ + 4) + pz]; };
-  // unit normal (rotated at wetting nodes) and |grad phi| of plane xp, halo 1
-  auto compute_n = [&](int xp) {
+  int ring_y, ring_z;
+  ring_node(threadIdx.x, BY, ring_y, ring_z);
+  constexpr int kRing = 2 * (BZ + 2) + 2 * BY;
+  // unit normals (rotated at wetting nodes) and |grad phi| of plane xp, halo 1
+  auto compute_n_as = [&](auto solidc, int xp) __attribute__((always_inline)) {
+    constexpr bool solid = decltype(solidc)::value;
     const int s = xp & 3;   // xp >= -1: the slot in the 4-plane normal ring
     // phi planes xp-1, xp, xp+1 in the 5-plane ring (xp >= -1)
     const R* const pm = sm.phi[(unsigned)(xp + 4) % 5u];
     const R* const p0 = sm.phi[(unsigned)(xp + 5) % 5u];
     const R* const pp1 = sm.phi[(unsigned)(xp + 6) % 5u];
-    for (int t = threadIdx.x; t < (BY + 2) * (BZ + 2); t += TPB) {
-      const int py = t / (BZ + 2), pz = t % (BZ + 2);
-      const int y = y0 - 1 + py, z = z0 - 1 + pz;
-      R n0 = R(0), n1 = R(0), n2 = R(0), fn = R(0);
-      bool ok = y <= P.ny && z <= P.nz;
-      int pp = 0;
-      if (SOLIDX && ok) {
-        const unsigned Lw = (unsigned)(wrapi(z, P.nz) + sy * wrapi(y, P.ny) + sx * wrapi(xp, P.nx));
-        if (walls_all[Lw] > 0) ok = false;
-        else pp = pout[Lw];
+    auto one = [&](int py, int pz) __attribute__((always_inline)) {
+      R n0 = 0, n1 = 0, n2 = 0, fn = 0;
+      bool ok = true;
+      int id = 0, y = 0, z = 0;
+      if (solid) {   // nodes beyond the halo, read by nobody, take the last one's masks
+        y = wrapi(min(y0 - 1 + py, P.ny), P.ny);
+        z = wrapi(min(z0 - 1 + pz, P.nz), P.nz);
+        const unsigned Lw = (unsigned)(z + sy * y + sx * wrapi(xp, P.nx));
+        const int wall = walls_all[Lw];
+        id = pout[Lw];
+        ok = wall <= 0;
       }
       if (ok) {
-        // grad phi = 3 sum_i w_i c_i phi(x + c_i) (:510-521), summed over the
-        // nine opposite pairs: w_i c_i (phi(x + c_i) - phi(x - c_i))
-        R g0 = R(0), g1 = R(0), g2 = R(0);
-        static_for<9>([&](auto kc) {
-          constexpr int i = PREP(decltype(kc)::value);
-          constexpr int o = CY(i) * (BZ + 4) + CZ(i);
-          const int b = (py + 1) * (BZ + 4) + pz + 1;
-          const R* const pa = CX(i) > 0 ? pp1 : (CX(i) < 0 ? pm : p0);
-          const R* const pb = CX(i) > 0 ? pm : (CX(i) < 0 ? pp1 : p0);
-          const R d = pa[b + o] - pb[b - o];
-          if (CX(i)) g0 = g0 + R(W(i) * CX(i)) * d;
-          if (CY(i)) g1 = g1 + R(W(i) * CY(i)) * d;
-          if (CZ(i)) g2 = g2 + R(W(i) * CZ(i)) * d;
-        });
-        g0 = R(3) * g0; g1 = R(3) * g1; g2 = R(3) * g2;
+        // grad phi = 3 sum_i w_i c_i phi(x + c_i) (:510-521) from the
+        // differences over opposite neighbours: an axis pair weighs twice a
+        // diagonal one
+        const int b = (py + 1) * kRow + pz + 1;
+        const R xyp = pp1[b + kRow] - pm[b - kRow], xym = pp1[b - kRow] - pm[b + kRow];
+        const R xzp = pp1[b + 1] - pm[b - 1], xzm = pp1[b - 1] - pm[b + 1];
+        const R yzp = p0[b + kRow + 1] - p0[b - kRow - 1], yzm = p0[b + kRow - 1] - p0[b - kRow + 1];
+        const R g0 = (1.0 / 12.0) * fma(2.0, pp1[b] - pm[b], (xyp + xym) + (xzp + xzm));
+        const R g1 = (1.0 / 12.0) * fma(2.0, p0[b + kRow] - p0[b - kRow], (xyp - xym) + (yzp + yzm));
+        const R g2 = (1.0 / 12.0) * fma(2.0, p0[b + 1] - p0[b - 1], (xzp - xzm) + (yzp - yzm));
         const R g2s = g0 * g0 + g1 * g1 + g2 * g2;
         // |grad phi| and its reciprocal from one rsqrt
         if (g2s > evap * evap) {
           const R rf = rsqrt(g2s);
           fn = g2s * rf;
           n0 = g0 * rf; n1 = g1 * rf; n2 = g2 * rf;
-          if (SOLIDX && pp >= 1) wet_rotate<R>(P, Sp, pp, wrapi(xp, P.nx), wrapi(y, P.ny), wrapi(z, P.nz), n0, n1, n2);
+          if (solid && id >= 1) wet_rotate<R>(P, Sp, id, wrapi(xp, P.nx), y, z, n0, n1, n2);
         }
       }
       sm.n.set(s, py, pz, n0, n1, n2, fn);
-    }
+    };
+    one(ty + 1, tz + 1);   // the thread's own node, then the ring around the tile
+    if (threadIdx.x < kRing) one(ring_y, ring_z);
   };
+  // every plane is compiled twice, with and without solids; a plane's flag is
+  // the whole CTA's, and the code of the planes without stays that of a domain
+  // without
+  auto near_solid = [&](int xp) { return SOLIDX && sm.near_solid[xp - xa + 1]; };
+  auto compute_n = [&](int xp) {
+    if constexpr (SOLID) {
+      if (near_solid(xp)) {
+        compute_n_as(std::true_type{}, xp);
+        return;
+      }
+    }
+    compute_n_as(std::false_type{}, xp);
+  };
+  if (SOLIDX) {
+    for (int t = threadIdx.x; t < xb - xa + 2; t += kTPB)
+      sm.near_solid[t] = solid_near(P, Sp, BY, xa - 1 + t, y0, z0);
+    __syncthreads();
+  }
 
   if (threadIdx.x == 0)
     for (int xp = xa - 2; xp <= xa + 2; xp++) load_phi(xp);
-  for (int xp = xa - 2; xp <= xa + 2; xp++) wait_phi(xp);
-  compute_n(xa - 1);
-  compute_n(xa);
-  // the first iteration's phi load reuses the slot of plane xa-2, which
-  // compute_n(xa-1) above reads
-  __syncthreads();
+  wait_phi(xa - 2);
+  wait_phi(xa - 1);
   nload = nl0 + (unsigned)(xb - xa + 4);   // loads of this tile: planes xa-2 .. xb+1
 
-  const int y = y0 + ty, z = z0 + tz;
-  const bool inr = y < P.ny && z < P.nz;
-  // every lane runs the node arithmetic (lanes outside the domain on a
-  // clamped node), so the warp shuffles of the density accumulation below see
-  // the whole warp; `act` masks the stores and contributions
-  const int yc = min(y, P.ny - 1), zc = min(z, P.nz - 1);
-  // Pushes that leave the tile along z (or across the periodic wrap) are added
-  // to the accumulators directly; the others are summed over z through warp
-  // shuffles, then over y through shared memory (a row at the tile's y edge
-  // adds its outgoing sums directly), and the sum a plane sends to each
-  // destination plane is turned into fixed point before the planes are added
-  // in registers along the march: the totals are integer sums of terms that
-  // do not depend on where the march starts or ends, so a domain's result is
-  // the same bit for bit whatever x extent its tiles have.
-  const bool ezp = tz == BZ - 1 || z >= P.nz - 1, ezm = tz == 0 || z == 0;
-  const bool eyp = ty == BY - 1 || y >= P.ny - 1, eym = ty == 0 || y == 0;
-  using AT = typename Acc<R>::T;
-  AT* const accR = acc;
-  AT* const accB = acc + N;
-  AT aPr = 0, aPb = 0, aCr = 0, aCb = 0;   // planes x-1 and x
-  for (int x = xa; x < xb; x++) {
-    // phi of plane x+3 on its way; normals of plane x+1 from phi planes x..x+2.
-    // The slots the load overwrites (phi of plane x-2, reference pairs of plane x-3)
-    // were last read before the previous plane's barriers.
-    if (threadIdx.x == 0 && x + 3 <= xb + 1) load_phi(x + 3);
+  // last row and lane of the tile inside the domain; rows past the last one
+  // have no work, lanes past the last one run the node arithmetic on a clamped
+  // node for the shuffles' sake (nothing of theirs is stored or added)
+  const int ylast = min(BY - 1, P.ny - 1 - y0), zlast = min(BZ - 1, P.nz - 1 - z0);
+  const int y = y0 + ty, z = z0 + min(tz, zlast);
+  const bool inr = ty <= ylast && tz <= zlast;
+  const bool ezp = tz == zlast, ezm = tz == 0;
+  const int oyp = (y == P.ny - 1) ? -(P.ny - 1) * sy : sy, oym = (y == 0) ? (P.ny - 1) * sy : -sy;
+  const int ozp = (z == P.nz - 1) ? -(P.nz - 1) : 1, ozm = (z == 0) ? (P.nz - 1) : -1;
+  // ring nodes: threads 0..127 the rows before and after the tile (two
+  // colours, 32 lanes), threads 128..167 the columns beside it, their rows -1
+  // to ylast + 1 (the corners included)
+  constexpr int kRowItems = 4 * BZ, kColItems = 4 * (BY + 2);
+  const bool row_item = threadIdx.x < kRowItems;
+  const int u = (int)threadIdx.x - kRowItems;
+  const int o_side = row_item ? (int)threadIdx.x / (2 * BZ) : u / (2 * (BY + 2));
+  const int o_col = row_item ? ((int)threadIdx.x / BZ) & 1 : (u / (BY + 2)) & 1;
+  const int o_row = row_item ? (o_side ? ylast + 1 : -1) : u % (BY + 2) - 1;
+  const bool o_valid =
+      row_item ? tz <= zlast : ((int)threadIdx.x < kRowItems + kColItems && o_row <= ylast + 1);
+  const int o_z = row_item ? z0 + min(tz, zlast) : wrapi(o_side ? z0 + zlast + 1 : z0 - 1, P.nz);
+  AT* const o_acc = acc + (o_col ? Ni : 0) + (o_z + sy * wrapi(y0 + o_row, P.ny));
+  AT* const n_acc = acc + (z + sy * min(y, P.ny - 1));
+  AT aPr = 0, aPb = 0, aCr = 0, aCb = 0, oP = 0, oC = 0;   // planes x-1 and x
+  bool fine = true;   // every density finite and in the fixed-point range
+  // the node arithmetic, pushes and density sums of plane x
+  auto plane = [&](auto solidc, int x) __attribute__((always_inline)) {
+    constexpr bool solid = decltype(solidc)::value;
     wait_phi(x + 2);
     compute_n(x + 1);
     __syncthreads();
-    const unsigned L = (unsigned)(zc + sy * yc + sx * x);
-    int pp = 0;
-    bool act = inr;
-    if (SOLIDX) {
-      if (walls_all[L] > 0) act = false;
-      else pp = pout[L];
-    }
-    // g[cx+1][cy+1][colour]: in-tile pushes summed per destination column and
-    // plane (cz = +-1 pushes arrive from the neighbouring lanes); sf: links
-    // bounced back into this node
-    R g[3][3][2];
-#pragma unroll
-    for (int a = 0; a < 3; a++)
-#pragma unroll
-      for (int b = 0; b < 3; b++)
-#pragma unroll
-        for (int c = 0; c < 2; c++) g[a][b][c] = R(0);
-    R sfr = R(0), sfb = R(0);
-    // accumulating kernels run every lane of a warp with an active node (the
-    // shuffles need the whole warp); the others skip inactive nodes
-    if (sizeof(R) == 8 && x + 1 < xb && threadIdx.x < 19 * BY) {
-      // FP64: the next plane's populations toward L2 while this plane
-      // computes, one bulk prefetch per (velocity, row) of the tile, by
-      // 19 x BY threads; the range is widened to 16-byte boundaries inside
-      // the array.  (Measured: FP64 collide 4.71 ms with it, 4.87 with one
-      // prefetch per population and thread, 4.89 without on the C3 thread;
-      // the FP32-math kernels are faster without any.)
-      constexpr size_t PB = 2 * sizeof(S);   // bytes per slot pair
-      const int i = threadIdx.x / BY, yy = y0 + (int)threadIdx.x % BY;
-      if (yy < P.ny) {
-        const size_t a = ((size_t)i * N + (size_t)(z0 + sy * yy + sx * (x + 1))) * PB;
-        const size_t e = min(a + (size_t)min(BZ, P.nz - z0) * PB + 15, (size_t)19 * N * PB) & ~size_t(15);
-        const size_t b = a & ~size_t(15);
-        if (e > b) tma::prefetch_l2(reinterpret_cast<const char*>(pin_) + b, (uint32_t)(e - b));
+    const int oxp = (x == P.nx - 1) ? -(P.nx - 1) * sx : sx, oxm = (x == 0) ? (P.nx - 1) * sx : -sx;
+    R cen[3][2];   // sums this row sends to its own row in planes x-1, x, x+1
+    if (ty <= ylast) {
+      const int L = z + sy * y + sx * x;
+      int pp = 0;
+      bool act = inr;
+      if (solid) {
+        const int wall = walls_all[L], id = pout[L];
+        if (wall > 0) act = false;
+        else pp = id;
       }
-    }
-    if (ACC ? __any_sync(0xffffffffu, act) : act) {
-    // calmacros on the own populations
-    // (rho_B = rho - rho_R: a pure colour stays exactly pure, as r = f there)
-    R f[19], sr, sb, rho, irho;
-    const Ref rref = REF ? rr_old[pd.idx(x, yc, zc)] : Ref{};
-    R nown[3];
-    sm.n.get(x & 3, ty + 1, tz + 1, nown);
-    const R nx = nown[0], ny = nown[1], nz = nown[2], fn = sm.n.grad(x & 3, ty + 1, tz + 1);
-    const bool flag = fn > evap;
-    if constexpr (sizeof(R) == 8) {
-      auto ld = [&](auto ic) -> R {   // f[i]; returns the red population
+      // calmacros on the own populations
+      R f[19];
+      const double2* const in = reinterpret_cast<const double2*>(pin_) + L;
+      auto ld = [&](auto ic) __attribute__((always_inline)) -> R {   // f[i]; returns the red population
         constexpr int i = decltype(ic)::value;
-        R r;
-        Codec<S>::template load_fr<i>(pin_, N, L, rref, f[i], r);
-        return r;
+        const double2 v = in[i * Ni];
+        f[i] = v.x + v.y;
+        return v.x;
       };
 #define SYM_LD(i) ld(std::integral_constant<int, i>{})
       // red density, added in the order to_moments adds the totals: a pure red
@@ -652,16 +643,19 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
       const R rzp = SYM_LD(11) + SYM_LD(14), rzm = SYM_LD(12) + SYM_LD(13);
       const R ryp = SYM_LD(15) + SYM_LD(18), rym = SYM_LD(16) + SYM_LD(17);
 #undef SYM_LD
-      sr = rest + (rx + ry + rz) + ((rxp + rxm) + (rzp + rzm) + (ryp + rym));
+      const R sr = rest + (rx + ry + rz) + ((rxp + rxm) + (rzp + rzm) + (ryp + rym));
       Moments<R> m;
       to_moments<R, R>(f, m);
-      rho = m.rho;
-      sb = rho - sr;
-      R su, sq;
-      node_rates_fused<R>(P, np, PHI(x, ty + 2, tz + 2), rho, irho, su, sq);
-      // CSF surface tension from the curvature of the normal field (:624-667)
-      R fx = R(0), fy = R(0), fz = R(0);
-      if (flag && (!SOLIDX || pp <= 0)) {
+      const R rho = m.rho, sb = rho - sr;
+      R nown[3];
+      sm.n.get(x & 3, ty + 1, tz + 1, nown);
+      const R nx = nown[0], ny = nown[1], nz = nown[2], fn = sm.n.grad(x & 3, ty + 1, tz + 1);
+      R irho, su, sq;
+      node_rates_fused<R>(P, sm.phi[(unsigned)(x + 5) % 5u][(ty + 2) * kRow + tz + 2], rho, irho, su, sq);
+      // CSF surface tension from the curvature of the normal field (:624-667);
+      // a node without a normal has n = 0 and |grad phi| = 0
+      R val = 0;
+      if (!solid || pp <= 0) {
         const R kurv = curvature<R, R>(
             [&](auto ic, R (&d)[3]) {
               constexpr int i = decltype(ic)::value;
@@ -671,255 +665,216 @@ __device__ __forceinline__ void collide_tile(const DevParams& P, const Pad& pd, 
               d[0] = p[0] - q[0]; d[1] = p[1] - q[1]; d[2] = p[2] - q[2];
             },
             nx, ny, nz);
-        const R val = np.half_sigma * kurv * fn;
-        fx = val * nx; fy = val * ny; fz = val * nz;
+        val = np.half_sigma * kurv * fn;
       }
-      fx = fx + rho * np.body[0];
-      fy = fy + rho * np.body[1];
-      fz = fz + rho * np.body[2];
-      const R ux = (m.jx + R(0.5) * fx) * irho, uy = (m.jy + R(0.5) * fy) * irho, uz = (m.jz + R(0.5) * fz) * irho;
-      relax<R, R>(m, ux, uy, uz, fx, fy, fz, su, np.s_e > R(0) ? np.s_e : su, np.s_eps > R(0) ? np.s_eps : su,
-                  np.s_q > R(0) ? np.s_q : sq, np.s_pi > R(0) ? np.s_pi : su, np.s_m > R(0) ? np.s_m : sq);
+      const R fx = fma(val, nx, rho * np.body[0]), fy = fma(val, ny, rho * np.body[1]),
+              fz = fma(val, nz, rho * np.body[2]);
+      relax<R, R>(m, rho, (m.jx + 0.5 * fx) * irho, (m.jy + 0.5 * fy) * irho, (m.jz + 0.5 * fz) * irho, fx, fy, fz, su,
+                  np.s_e > 0 ? np.s_e : su, np.s_eps > 0 ? np.s_eps : su, np.s_q > 0 ? np.s_q : sq,
+                  np.s_pi > 0 ? np.s_pi : su, np.s_m > 0 ? np.s_m : sq);
       from_moments<R, R>(m, f);
-    } else {
-      sr = R(0);
-      rho = R(0);
-      unroll19([&](auto ic) {
+      // Latva-Kokko recolouring (:712-726): r_i = (rhoR/rho) f_i + beta rhoR rhoB /
+      // rho w_i (n.c_i); a colour at or below EVAP_LIM empties (r_i = 0 when
+      // rhoR is, r_i = f_i when rhoB is, the latter taking precedence), which the
+      // two coefficients express once per node
+      const bool rzero = sr <= evap, bzero = sb <= evap;
+      R ratio = bzero ? 1.0 : (rzero ? 0.0 : sr * irho);
+      // beta rhoR rhoB / rho times a diagonal link's weight, along each axis
+      R cd = (bzero || rzero) ? 0.0 : sr * sb * irho * np.beta * (1.0 / 36.0);
+      // links that come back (bit i: the push along c_i enters a solid, curve
+      // :1001-1019), from a wall without velocity (flat) or from particle pp
+      unsigned back = 0, flat = 0;
+      R uw0 = 0, uw1 = 0, uw2 = 0;
+      if (solid) {
+        if (!act) {   // a solid node (or a lane outside the domain) sends nothing
+          ratio = 0;
+          cd = 0;
+#pragma unroll
+          for (int i = 0; i < 19; i++) f[i] = 0;
+        }
+        if (pp >= 1) {
+          const int par = P.par;
+          static_for<18>([&](auto kc) {   // the neighbours' masks are read together, not one per push
+            constexpr int i = decltype(kc)::value + 1;
+            const int wb = walls[L + (CX(i) > 0 ? oxp : (CX(i) < 0 ? oxm : 0)) +
+                                 (CY(i) > 0 ? oyp : (CY(i) < 0 ? oym : 0)) + (CZ(i) > 0 ? ozp : (CZ(i) < 0 ? ozm : 0))];
+            if (wb > par) flat |= 1u << i;
+            else if (wb == pp) back |= 1u << i;
+          });
+          back |= flat;
+          if (pp <= par && act) {
+            // rigid-body velocity of particle pp at this node (curve :1009-1014)
+            const R xr = disp(P, (double)(x + P.origin), Sp->center[0 * par + pp - 1], 0);
+            const R yr = disp(P, (double)(y + P.origin), Sp->center[1 * par + pp - 1], 1);
+            const R zr = disp(P, (double)(z + P.origin), Sp->center[2 * par + pp - 1], 2);
+            uw0 = Sp->up[0 * par + pp - 1] + zr * Sp->rp[1 * par + pp - 1] - yr * Sp->rp[2 * par + pp - 1];
+            uw1 = Sp->up[1 * par + pp - 1] + xr * Sp->rp[2 * par + pp - 1] - zr * Sp->rp[0 * par + pp - 1];
+            uw2 = Sp->up[2 * par + pp - 1] + yr * Sp->rp[0 * par + pp - 1] - xr * Sp->rp[1 * par + pp - 1];
+            // post-collision populations for the momentum exchange (:1241-1243),
+            // read only next to particles
+#pragma unroll
+            for (int i = 0; i < 19; i++) ffi[(size_t)i * Ni + L] = f[i];
+          }
+        }
+      }
+      const R cnx = cd * nx, cny = cd * ny, cnz = cd * nz;
+      double2* const out = reinterpret_cast<double2*>(pout_) + L;
+      R sfr = 0, sfb = 0;   // links bounced back into this node
+      // push along c_i: red r and blue b, as stored (0 if the link came back)
+      auto push = [&](auto ic, R& r, R& b) __attribute__((always_inline)) {
         constexpr int i = decltype(ic)::value;
-        R r;
-        Codec<S>::template load_fr<i>(pin_, N, L, rref, f[i], r);
-        sr = sr + r;
-        rho = rho + f[i];
-      });
-      sb = rho - sr;
-      R ux = R(0), uy = R(0), uz = R(0);
-#pragma unroll
-      for (int i = 0; i < 19; i++) {
-        if (CX(i)) ux = ux + f[i] * R(CX(i));
-        if (CY(i)) uy = uy + f[i] * R(CY(i));
-        if (CZ(i)) uz = uz + f[i] * R(CZ(i));
-      }
-      irho = qdiv<R>(R(1), rho);
-      ux = ux * irho; uy = uy * irho; uz = uz * irho;
-      const R rhoN = PHI(x, ty + 2, tz + 2);
-      // CSF surface tension from the curvature of the normal field (:624-667)
-      R fx = R(0), fy = R(0), fz = R(0);
-      if (flag && (!SOLIDX || pp <= 0)) {
-        // d_ba = sum_i w_i c_ia n_b(x + c_i) (:635-660), over the nine opposite
-        // pairs: w_i c_ia (n_b(x + c_i) - n_b(x - c_i))
-        R d00 = 0, d01 = 0, d02 = 0, d10 = 0, d11 = 0, d12 = 0, d20 = 0, d21 = 0, d22 = 0;
-        static_for<9>([&](auto kc) {
-          constexpr int i = PREP(decltype(kc)::value);
-          R p[3], q[3];
-          sm.n.get((x + CX(i)) & 3, ty + 1 + CY(i), tz + 1 + CZ(i), p);
-          sm.n.get((x - CX(i)) & 3, ty + 1 - CY(i), tz + 1 - CZ(i), q);
-          const R a = p[0] - q[0], b = p[1] - q[1], c = p[2] - q[2];
-          if (CX(i)) { constexpr double k = W(i) * CX(i); d00 = d00 + R(k) * a; d10 = d10 + R(k) * b; d20 = d20 + R(k) * c; }
-          if (CY(i)) { constexpr double k = W(i) * CY(i); d01 = d01 + R(k) * a; d11 = d11 + R(k) * b; d21 = d21 + R(k) * c; }
-          if (CZ(i)) { constexpr double k = W(i) * CZ(i); d02 = d02 + R(k) * a; d12 = d12 + R(k) * b; d22 = d22 + R(k) * c; }
-        });
-        d00 *= R(3); d01 *= R(3); d02 *= R(3); d10 *= R(3); d11 *= R(3); d12 *= R(3);
-        d20 *= R(3); d21 *= R(3); d22 *= R(3);
-        const R kurv = nx * ny * (d10 + d01) + nx * nz * (d20 + d02) + ny * nz * (d12 + d21) -
-                       (ny * ny + nz * nz) * d00 - (nx * nx + nz * nz) * d11 - (nx * nx + ny * ny) * d22;
-        const R val = R(0.5) * R(P.sigma) * kurv;
-        fx = val * (fn * nx); fy = val * (fn * ny); fz = val * (fn * nz);
-      }
-      fx = fx + rho * R(P.body[0]);
-      fy = fy + rho * R(P.body[1]);
-      fz = fz + rho * R(P.body[2]);
-      const R hirho = R(0.5) * irho;
-      ux = ux + fx * hirho;
-      uy = uy + fy * hirho;
-      uz = uz + fz * hirho;
-      mrt_collide_pairs<R>(P, f, rho, ux, uy, uz, fx, fy, fz, rhoN);
-    }
-    // post-collision populations for the momentum exchange (:1241-1243), read
-    // only next to particles (pout = particle id); wall planes (ids > par)
-    // need none, and a handle without particles holds no ffi array
-    if (SOLIDX && act && pp >= 1 && pp <= P.par) {
-#pragma unroll
-      for (int i = 0; i < 19; i++) ffi[(size_t)i * N + L] = (double)f[i];
-    }
-    // Latva-Kokko recolouring (:712-726): r_i = (rhoR/rho) f_i + beta rhoR rhoB /
-    // rho w_i (n.c_i); a colour at or below EVAP_LIM empties (r_i = 0 when
-    // rhoR is, r_i = f_i when rhoB is, the latter taking precedence), which the
-    // two coefficients express once per node
-    const bool rzero = sr <= evap, bzero = sb <= evap;
-    const R ratio = bzero ? R(1) : (rzero ? R(0) : sr * irho);
-    const R coef = (bzero || rzero || !flag) ? R(0) : sr * sb * irho * np.beta;
-    // beta rhoR rhoB / rho times a diagonal link's weight, along each axis
-    [[maybe_unused]] const R cd = coef * R(1.0 / 36.0), cnx = cd * nx, cny = cd * ny, cnz = cd * nz;
-    // rigid-body velocity of particle pp at this node (curve :1009-1014), for
-    // the links that bounce back from it
-    R uw0 = R(0), uw1 = R(0), uw2 = R(0);
-    if (SOLIDX && pp >= 1 && pp <= P.par) {
-      const int par = P.par;
-      const R xr = R(disp(P, (double)(x + P.origin), Sp->center[0 * par + pp - 1], 0));
-      const R yr = R(disp(P, (double)(y + P.origin), Sp->center[1 * par + pp - 1], 1));
-      const R zr = R(disp(P, (double)(z + P.origin), Sp->center[2 * par + pp - 1], 2));
-      uw0 = R(Sp->up[0 * par + pp - 1]) + zr * R(Sp->rp[1 * par + pp - 1]) - yr * R(Sp->rp[2 * par + pp - 1]);
-      uw1 = R(Sp->up[1 * par + pp - 1]) + xr * R(Sp->rp[2 * par + pp - 1]) - zr * R(Sp->rp[0 * par + pp - 1]);
-      uw2 = R(Sp->up[2 * par + pp - 1]) + yr * R(Sp->rp[0 * par + pp - 1]) - xr * R(Sp->rp[1 * par + pp - 1]);
-    }
-    // neighbour offsets with the periodic wrap folded in (one select per face)
-    const int oxp = (x == P.nx - 1) ? -(P.nx - 1) * sx : sx, oxm = (x == 0) ? (P.nx - 1) * sx : -sx;
-    const int oyp = (yc == P.ny - 1) ? -(P.ny - 1) * sy : sy, oym = (yc == 0) ? (P.ny - 1) * sy : -sy;
-    const int ozp = (zc == P.nz - 1) ? -(P.nz - 1) : 1, ozm = (zc == 0) ? (P.nz - 1) : -1;
-    R zp[2] = {R(0), R(0)}, zm[2] = {R(0), R(0)};
-    // directions in groups of equal (cx, cy): within a group only cz differs,
-    // and the cz = +-1 pushes of the group move one lane up / down right after it
-    static_for<19>([&](auto kc) {
-      constexpr int k = decltype(kc)::value;
-      constexpr int i = PUSH_ORDER(k);
-      constexpr int a = CX(i) + 1, b = CY(i) + 1;
-      [&] {
-        R r;
-        if constexpr (sizeof(R) == 4) {
-          r = ratio * f[i];
-          if (i > 0) r = r + coef * R(W(i)) * (nx * R(CX(i)) + ny * R(CY(i)) + nz * R(CZ(i)));
-        } else if constexpr (i == 0) {
+        if constexpr (i == 0) {
           r = ratio * f[i];
         } else if constexpr (i < 7) {
           constexpr double c = 2 * (CX(i) + CY(i) + CZ(i));   // twice the diagonal weight
-          r = vfma(ratio, f[i], R(c) * (CX(i) ? cnx : (CY(i) ? cny : cnz)));
+          r = fma(ratio, f[i], c * (CX(i) ? cnx : (CY(i) ? cny : cnz)));
         } else {
           constexpr int s1 = CX(i) ? CX(i) : CY(i), s2 = CZ(i) ? CZ(i) : CY(i);   // the two axes of the link
           const R c1 = CX(i) ? cnx : cny, c2 = CZ(i) ? cnz : cny;
-          r = vfma(ratio, f[i], s1 > 0 ? (s2 > 0 ? c1 + c2 : c1 - c2) : (s2 > 0 ? c2 - c1 : -(c1 + c2)));
+          r = fma(ratio, f[i], s1 > 0 ? (s2 > 0 ? c1 + c2 : c1 - c2) : (s2 > 0 ? c2 - c1 : -(c1 + c2)));
         }
-        const unsigned T = L + (CX(i) > 0 ? oxp : (CX(i) < 0 ? oxm : 0)) +
-                           (CY(i) > 0 ? oyp : (CY(i) < 0 ? oym : 0)) + (CZ(i) > 0 ? ozp : (CZ(i) < 0 ? ozm : 0));
-        if (!act) return;
-        // interpolated bounce-back: the red post-collision populations of the
-        // nodes next to particles, for the link update after this kernel
-        if (SOLIDX && P.bounce && pp >= 1 && pp <= P.par) ffi[(size_t)(19 + i) * N + L] = (double)r;
-        if (SOLIDX && i > 0 && pp >= 1) {
-          const int wb = walls[T];
-          const bool flat = wb > P.par;
-          if (wb == pp || flat) {
-            // curve (:1001-1019): link OPC(i) of this node comes back reversed
+        b = f[i] - r;
+        int o = i * Ni + (CX(i) > 0 ? oxp : (CX(i) < 0 ? oxm : 0)) + (CY(i) > 0 ? oyp : (CY(i) < 0 ? oym : 0)) +
+                (CZ(i) > 0 ? ozp : (CZ(i) < 0 ? ozm : 0));
+        if (solid) {
+          // interpolated bounce-back: the red post-collision populations of the
+          // nodes next to particles, for the link update after this kernel
+          if (P.bounce && pp >= 1 && pp <= P.par && act) ffi[(size_t)(19 + i) * Ni + L] = r;
+          if (i > 0 && (back >> i & 1u)) {
             constexpr int j = OPC(i);
-            const R star = flat ? R(0) : uw0 * R(CX(j)) + uw1 * R(CY(j)) + uw2 * R(CZ(j));
-            const R rr = r + R(6.0 * W(j)) * sr * star;
-            const R bb = (f[i] - r) + R(6.0 * W(j)) * sb * star;
-            const Ref rd = REF ? sm.ref[(unsigned)x % kIrrRing][(ty + 2) * (BZ + 4) + tz + 2] : Ref{};
-            Codec<S>::template store<j>(pout_, N, L, rd, rr, rr + bb);
+            const R star = (flat >> i & 1u) ? 0.0 : 6.0 * W(j) * (uw0 * CX(j) + uw1 * CY(j) + uw2 * CZ(j));
+            const R rr = fma(sr, star, r), bb = fma(sb, star, b);
+            if (act) out[j * Ni] = make_double2(rr, bb);
             sfr = sfr + rr;
             sfb = sfb + bb;
+            r = b = 0;
             return;
           }
         }
-        const Ref rd = REF ? sm.ref[(unsigned)(x + CX(i) + kIrrRing) % kIrrRing]
-                                   [(ty + 2 + CY(i)) * (BZ + 4) + tz + 2 + CZ(i)]
-                           : Ref{};
-        Codec<S>::template store<i>(pout_, N, T, rd, r, f[i]);
-        if constexpr (!ACC) return;
-        const R bv = f[i] - r;
-        if (CZ(i) == 0) {
-          g[a][b][0] = g[a][b][0] + r;
-          g[a][b][1] = g[a][b][1] + bv;
-        } else if (CZ(i) > 0) {
-          zp[0] = r;
-          zp[1] = bv;
-        } else {
-          zm[0] = r;
-          zm[1] = bv;
-        }
-      }();
-      if constexpr (ACC && CZ(i) < 0) {
-        // last of a group with cz = 0, +1, -1: lane l receives the cz = +1 push
-        // of lane l-1 and the cz = -1 push of lane l+1 (lane = tz); the edge
-        // lanes' outgoing pushes go to the accumulators in one go (a lane that
-        // is both edges, of a one-node tile row, adds its second one after)
+        if (act) out[o] = make_double2(r, b);
+      };
+      // the pushes along equal (cx, cy): lane l receives the cz = +1 push of
+      // lane l-1 and the cz = -1 push of lane l+1; the edge lanes' outgoing ones
+      // go to the columns' exchange
+      auto group = [&](auto ac, auto bc, auto i0, auto ip, auto im, R& r, R& b) __attribute__((always_inline)) {
+        constexpr int a = decltype(ac)::value, g = decltype(bc)::value;
+        R up[2], dn[2];
+        push(i0, r, b);
+        push(ip, up[0], up[1]);
+        push(im, dn[0], dn[1]);
+        if (ezp) { sm.zx[1][a][g][0][ty] = up[0]; sm.zx[1][a][g][1][ty] = up[1]; }
+        if (ezm) { sm.zx[0][a][g][0][ty] = dn[0]; sm.zx[0][a][g][1][ty] = dn[1]; }
 #pragma unroll
         for (int c = 0; c < 2; c++) {
-          const R up = __shfl_up_sync(0xffffffffu, zp[c], 1);
-          const R dn = __shfl_down_sync(0xffffffffu, zm[c], 1);
-          g[a][b][c] = g[a][b][c] + (tz > 0 ? up : R(0)) + (tz < BZ - 1 ? dn : R(0));
+          up[c] = __shfl_up_sync(0xffffffffu, up[c], 1);
+          dn[c] = __shfl_down_sync(0xffffffffu, dn[c], 1);
         }
-        if (act && (ezp || ezm)) {
-          const unsigned T0 = L + (a > 1 ? oxp : (a < 1 ? oxm : 0)) + (b > 1 ? oyp : (b < 1 ? oym : 0));
-          const unsigned T = T0 + (ezp ? ozp : ozm);
-          acc_add<R>(accR + T, ezp ? zp[0] : zm[0], status);
-          acc_add<R>(accB + T, ezp ? zp[1] : zm[1], status);
-          if (ezp && ezm) {
-            acc_add<R>(accR + T0 + ozm, zm[0], status);
-            acc_add<R>(accB + T0 + ozm, zm[1], status);
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < 2; c++) zp[c] = zm[c] = R(0);
+        if (!ezm) { r = r + up[0]; b = b + up[1]; }
+        if (!ezp) { r = r + dn[0]; b = b + dn[1]; }
+      };
+#define SYM_I(v) std::integral_constant<int, v>{}
+      R r, b;
+      auto row = [&](int a, int dir) __attribute__((always_inline)) {   // to row y+1 (0) or y-1 (1) of plane x + a - 1
+        sm.xch[a][dir][0][ty][tz] = r;
+        sm.xch[a][dir][1][ty][tz] = b;
+      };
+      group(SYM_I(1), SYM_I(1), SYM_I(3), SYM_I(15), SYM_I(17), r, b); row(1, 0);
+      group(SYM_I(1), SYM_I(2), SYM_I(4), SYM_I(16), SYM_I(18), r, b); row(1, 1);
+      push(SYM_I(7), r, b); row(2, 0);
+      push(SYM_I(9), r, b); row(2, 1);
+      push(SYM_I(8), r, b); row(0, 0);
+      push(SYM_I(10), r, b); row(0, 1);
+      group(SYM_I(2), SYM_I(0), SYM_I(1), SYM_I(11), SYM_I(13), cen[2][0], cen[2][1]);
+      group(SYM_I(0), SYM_I(0), SYM_I(2), SYM_I(12), SYM_I(14), cen[0][0], cen[0][1]);
+      group(SYM_I(1), SYM_I(0), SYM_I(0), SYM_I(5), SYM_I(6), cen[1][0], cen[1][1]);
+#undef SYM_I
+      if (solid) {
+        cen[1][0] = cen[1][0] + sfr;
+        cen[1][1] = cen[1][1] + sfb;
       }
-    });
     }
-    if constexpr (ACC) {
-      // along y through shared memory: row ty+1 receives the cy = +1 sums of row
-      // ty and row ty-1 the cy = -1 sums, for each destination plane
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-          sm.xch[a][0][c][ty][tz] = g[a][2][c];
-          sm.xch[a][1][c][ty][tz] = g[a][0][c];
-        }
-      const int oxp = (x == P.nx - 1) ? -(P.nx - 1) * sx : sx, oxm = (x == 0) ? (P.nx - 1) * sx : -sx;
-      __syncthreads();
+    __syncthreads();
+    const int om = x > xa ? -sx : oxm;
+    auto fix = [&](R v) __attribute__((always_inline)) -> AT {
+      fine = fine && A::ok(v);
+      return A::fix(v);
+    };
+    if (inr) {
       AT in[3][2];
 #pragma unroll
       for (int a = 0; a < 3; a++)
 #pragma unroll
         for (int c = 0; c < 2; c++) {
-          R v = g[a][1][c];
+          R v = cen[a][c];
           if (ty > 0) v = v + sm.xch[a][0][c][ty - 1][tz];
-          if (ty < BY - 1) v = v + sm.xch[a][1][c][ty + 1][tz];
-          if (a == 1) v = v + (c ? sfb : sfr);
-          in[a][c] = inr ? acc_fix<R>(v, status) : 0;
+          if (ty < ylast) v = v + sm.xch[a][1][c][ty + 1][tz];
+          in[a][c] = fix(v);
         }
-      if (inr && (eyp || eym)) {
-        // the sums a row at the tile's y edge sends out of it
-        const int oyp = (y == P.ny - 1) ? -(P.ny - 1) * sy : sy, oym = (y == 0) ? (P.ny - 1) * sy : -sy;
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-          const unsigned T0 = L + (a > 1 ? oxp : (a < 1 ? oxm : 0));
-          acc_add<R>(accR + T0 + (eyp ? oyp : oym), eyp ? g[a][2][0] : g[a][0][0], status);
-          acc_add<R>(accB + T0 + (eyp ? oyp : oym), eyp ? g[a][2][1] : g[a][0][1], status);
-          if (eyp && eym) {
-            acc_add<R>(accR + T0 + oym, g[a][0][0], status);
-            acc_add<R>(accB + T0 + oym, g[a][0][1], status);
-          }
-        }
-      }
       // plane x-1 of this column has all its in-tile contributions (plane xa-1
       // only this plane's)
-      aPr += in[0][0]; aPb += in[0][1];
-      aCr += in[1][0]; aCb += in[1][1];
-      const int om = x > xa ? -sx : oxm;
-      if (inr && (aPr | aPb)) {
-        atomicAdd(accR + (L + om), aPr);
-        atomicAdd(accB + (L + om), aPb);
-      }
-      aPr = aCr; aPb = aCb;
+      AT* const at = n_acc + sx * x;
+      atomicAdd(at + om, aPr + in[0][0]);
+      atomicAdd(at + om + Ni, aPb + in[0][1]);
+      aPr = aCr + in[1][0]; aPb = aCb + in[1][1];
       aCr = in[2][0]; aCb = in[2][1];
-      if (x == xb - 1 && inr) {
-        // the end of the march: this plane's node and the plane after it
-        atomicAdd(accR + L, aPr);
-        atomicAdd(accB + L, aPb);
-        atomicAdd(accR + (L + oxp), aCr);
-        atomicAdd(accB + (L + oxp), aCb);
+      if (x == xb - 1) {   // the end of the march: this plane's node and the one after it
+        atomicAdd(at, aPr);
+        atomicAdd(at + Ni, aPb);
+        atomicAdd(at + oxp, aCr);
+        atomicAdd(at + oxp + Ni, aCb);
       }
     }
+    if (o_valid) {
+      AT in[3];
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        R v;
+        if (row_item) {
+          v = sm.xch[a][o_side ? 0 : 1][o_col][o_side ? ylast : 0][tz];
+        } else {
+          // rows o_row (same row), o_row - 1 (its cy = +1) and o_row + 1 (cy = -1);
+          // only the planes' own x has diagonal links that leave along y and z
+          v = 0;
+          if (o_row >= 0 && o_row <= ylast) v = sm.zx[o_side][a][0][o_col][o_row];
+          if (a == 1) {
+            if (o_row >= 1) v = v + sm.zx[o_side][1][1][o_col][o_row - 1];
+            if (o_row < ylast) v = v + sm.zx[o_side][1][2][o_col][o_row + 1];
+          }
+        }
+        in[a] = fix(v);
+      }
+      AT* const at = o_acc + sx * x;
+      atomicAdd(at + om, oP + in[0]);
+      oP = oC + in[1];
+      oC = in[2];
+      if (x == xb - 1) {
+        atomicAdd(at, oP);
+        atomicAdd(at + oxp, oC);
+      }
+    }
+  };
+#pragma unroll 1
+  for (int x = xa - 2; x < xa; x++) {
+    wait_phi(x + 2);
+    compute_n(x + 1);
   }
-}
-
-// Resident CTAs per SM the collide kernels are compiled for: the FP32-math
-// codecs fit 64 registers (32 warps per SM: 4 CTAs of 256 threads for FP32,
-// 2 of 512 for the 16-bit codec; measured faster than 3 CTAs of 256 at 80
-// registers, the latency-bound kernel gains from the extra warps), FP64 needs
-// the 128 of 2 CTAs of 256.
-template <typename S>
-constexpr int collide_ctas() {
-  return std::is_same<S, __half>::value ? 2 : (sizeof(typename Codec<S>::R) == 4 ? 4 : 2);
+  // the first phi load below reuses the slot of plane xa-2, read by the first turn
+  __syncthreads();
+#pragma unroll 1
+  for (int x = xa; x < xb; x++) {
+    // phi of plane x+3 on its way; normals of plane x+1 from phi planes x..x+2.
+    // The slots the load overwrites (phi of plane x-2) were last read before the
+    // previous plane's barriers.
+    if (threadIdx.x == 0 && x + 3 <= xb + 1) load_phi(x + 3);
+    if constexpr (SOLID) {
+      if (near_solid(x)) {
+        plane(std::true_type{}, x);
+        continue;
+      }
+    }
+    plane(std::false_type{}, x);
+  }
+  if (!fine) atomicOr(status, 1);
 }
 
 // Plane times a tile spends before its first plane (five plane loads and the
@@ -928,6 +883,7 @@ constexpr double kTileLead = 1.0;
 // x extent of a tile whose column of x planes is nx long, at most `cap`: the
 // column in equal parts
 inline int split_extent(int nx, int cap) {
+  cap = std::min(cap, kMaxExtent);
   const int parts = (nx + cap - 1) / cap;
   return (nx + parts - 1) / parts;
 }
@@ -955,28 +911,6 @@ inline int best_extent(const std::vector<long long>& columns, const std::vector<
     if (t <= least) { least = t; best = x; }
   }
   return best;
-}
-
-template <typename S, bool SOLID>
-__global__ void __launch_bounds__(kTPB<S>, collide_ctas<S>()) k_collide(DevParams P, Pad pd, const S* __restrict__ pin_,
-                                                   S* __restrict__ pout_,
-                                                   const typename Codec<S>::R* __restrict__ phi,
-                                                   const int32_t* __restrict__ walls,
-                                                   const int32_t* __restrict__ walls_all,
-                                                   const int32_t* __restrict__ pout,
-                                                   const sym_particles* __restrict__ Sp, double* __restrict__ ffi,
-                                                   const Ref* __restrict__ rr_old, const Ref* __restrict__ rr_new,
-                                                   typename Acc<typename Codec<S>::R>::T* acc, int* status,
-                                                   const __grid_constant__ CUtensorMap tm_phi,
-                                                   const __grid_constant__ CUtensorMap tm_ref, int xchunk) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  Smem<S>& sm = smem_view<S>(smem_raw);
-  collide_init_barriers<S>(sm);
-  unsigned nload = 0;
-  const int xa = blockIdx.z * xchunk;
-  collide_tile<S, SOLID>(P, pd, pin_, pout_, phi, walls, walls_all, pout, Sp, ffi, rr_old, rr_new, acc, status,
-                         &tm_phi, &tm_ref, blockIdx.x * BZ, blockIdx.y * kBY<S>, xa, min(xa + xchunk, P.nx), sm,
-                         nload);
 }
 
 // ---- the fused state's side of the particle and wall work ---------------------------

@@ -104,14 +104,39 @@ struct DevParams {
   double body[3];
   double rad, mass, inertia, fg, alpha, evap;
   double sin_cita, cos_cita;   // of the contact angle (fused path)
+  const unsigned char* solid_tiles;   // see TileParams
+  int tiles_y, tiles_z;
   int same_nu;             // both colours have the same viscosity
   NodeParams<double> nd;   // fused path
   NodeParams<float> nf;
 };
+// What the fused collide kernels read of a (CONFIG) domain, small enough that a
+// batch's descriptors are kernel parameters.
 template <typename R>
-__device__ __forceinline__ const NodeParams<R>& node_params(const DevParams& P) {
-  if constexpr (sizeof(R) == 8) return P.nd;
-  else return P.nf;
+struct TileParams {
+  static constexpr int ref = 0, origin = 0;
+  int nx, ny, nz;
+  int wall_x, par, bounce, same_nu;
+  // domains with solids: 1 where a tile's plane (its nodes and their one-node
+  // ring) held a solid or a node next to one when the fused state was built,
+  // [x][y tile][z tile]; particles' own surroundings are added in the kernel
+  int tiles_y, tiles_z;
+  const unsigned char* solid_tiles;
+  double rad, sin_cita, cos_cita;
+  R rho0;
+  NodeParams<R> np;
+};
+template <typename R>
+inline TileParams<R> tile_params(const DevParams& P) {
+  TileParams<R> t;
+  t.nx = P.nx; t.ny = P.ny; t.nz = P.nz;
+  t.wall_x = P.wall_x; t.par = P.par; t.bounce = P.bounce; t.same_nu = P.same_nu;
+  t.tiles_y = P.tiles_y; t.tiles_z = P.tiles_z; t.solid_tiles = P.solid_tiles;
+  t.rad = P.rad; t.sin_cita = P.sin_cita; t.cos_cita = P.cos_cita;
+  t.rho0 = R(P.rho0);
+  if constexpr (sizeof(R) == 8) t.np = P.nd;
+  else t.np = P.nf;
+  return t;
 }
 
 template <typename T>
@@ -131,7 +156,8 @@ __device__ __forceinline__ long long lin(const DevParams& P, int x, int y, int z
 
 // Displacement of node coordinate c from centre `cen` along axis k (minimum
 // image in periodic CONFIG axes).
-__device__ __forceinline__ double disp(const DevParams& P, double c, double cen, int k) {
+template <typename PT>
+__device__ __forceinline__ double disp(const PT& P, double c, double cen, int k) {
   double d = c - cen;
   if (!P.ref) {
     const int n = k == 0 ? P.nx : (k == 1 ? P.ny : P.nz);
@@ -142,20 +168,18 @@ __device__ __forceinline__ double disp(const DevParams& P, double c, double cen,
 }
 
 // equilf (Source1.f90:397-450): equilibrium moments and Guo forcing moments.
-// EXACT keeps the reference's divisions by 1.5; the fused path multiplies by
-// 2/3 instead (same value up to one rounding).
-template <typename R, bool EXACT = true>
+template <typename R>
 __device__ __forceinline__ void equilf(R meq[19], R fk[19], R rho, R ux, R uy, R uz, R fx, R fy, R fz) {
   const R usqr = ux * ux + uy * uy + uz * uz;
   meq[0] = R(1);
   meq[1] = R(19) * usqr - R(11);
   meq[2] = R(3) - R(5.5) * usqr;
   meq[3] = ux;
-  meq[4] = EXACT ? -ux / R(1.5) : ux * R(-2.0 / 3.0);
+  meq[4] = -ux / R(1.5);
   meq[5] = uy;
-  meq[6] = EXACT ? -uy / R(1.5) : uy * R(-2.0 / 3.0);
+  meq[6] = -uy / R(1.5);
   meq[7] = uz;
-  meq[8] = EXACT ? -uz / R(1.5) : uz * R(-2.0 / 3.0);
+  meq[8] = -uz / R(1.5);
   meq[9] = R(3) * ux * ux - usqr;
   meq[10] = R(-0.5) * (R(3) * ux * ux - usqr);
   meq[11] = uy * uy - uz * uz;
@@ -173,11 +197,11 @@ __device__ __forceinline__ void equilf(R meq[19], R fk[19], R rho, R ux, R uy, R
   fk[1] = R(38) * uf;
   fk[2] = R(-11) * uf;
   fk[3] = fx;
-  fk[4] = EXACT ? -fx / R(1.5) : fx * R(-2.0 / 3.0);
+  fk[4] = -fx / R(1.5);
   fk[5] = fy;
-  fk[6] = EXACT ? -fy / R(1.5) : fy * R(-2.0 / 3.0);
+  fk[6] = -fy / R(1.5);
   fk[7] = fz;
-  fk[8] = EXACT ? -fz / R(1.5) : fz * R(-2.0 / 3.0);
+  fk[8] = -fz / R(1.5);
   fk[9] = R(6) * ux * fx - R(2) * uf;
   fk[10] = -(R(3) * ux * fx - uf);
   fk[11] = R(2) * (uy * fy - uz * fz);
@@ -206,23 +230,6 @@ __device__ __forceinline__ void node_rates(const DevParams& P, R rhoN, R& su, R&
   else nu = R(2) / ((R(1) + rhoN) / R(P.nu_r) + (R(1) - rhoN) / R(P.nu_b));
   su = R(1) / (R(3) * nu + R(0.5));
   const R sq_ = R(8) * (R(2) - su) / (R(8) - su);
-  se = P.s_e > 0 ? R(P.s_e) : su;
-  seps = P.s_eps > 0 ? R(P.s_eps) : su;
-  sq = P.s_q > 0 ? R(P.s_q) : sq_;
-  spi = P.s_pi > 0 ? R(P.s_pi) : su;
-  sm = P.s_m > 0 ? R(P.s_m) : sq_;
-}
-
-// The same rates with two divisions (fused path): with phi clamped to
-// [-1, 1] and D = (1+phi)/nu_r + (1-phi)/nu_b, nu = 2/D gives the branches
-// of the reference at the ends, so su = 1/(3 nu + 1/2) = 2D/(12 + D).
-template <typename R>
-__device__ __forceinline__ void node_rates_fast(const DevParams& P, R rhoN, R& su, R& se, R& seps, R& sq, R& spi,
-                                                R& sm) {
-  const R ph = fmin(fmax(rhoN, R(-1)), R(1));
-  const R D = (R(1) + ph) * R(P.nd.inu_r) + (R(1) - ph) * R(P.nd.inu_b);
-  su = qdiv<R>(R(2) * D, R(12) + D);
-  const R sq_ = qdiv<R>(R(8) * (R(2) - su), R(8) - su);
   se = P.s_e > 0 ? R(P.s_e) : su;
   seps = P.s_eps > 0 ? R(P.s_eps) : su;
   sq = P.s_q > 0 ? R(P.s_q) : sq_;
@@ -268,26 +275,6 @@ __device__ __forceinline__ void mrt_collide(const DevParams& P, R f[19], R rho, 
   }
 }
 
-// The same collision in the opposite-pair basis (fused path, FP32 arithmetic).  Row r of M is
-// even (M(r,opc(c)) = M(r,c)) or odd (= -M(r,c)) under velocity reversal, so
-// with p_k = f_i + f_opc(i) and q_k = f_i - f_opc(i) over the 9 pairs the even
-// moments need only p (and f_0) and the odd ones only q; back-transformed,
-// f_i = E_i + O_i and f_opc(i) = E_i - O_i with E (O) the sum over even (odd)
-// rows.  Half the multiply-adds of the dense form; the result differs from it
-// only by rounding order.
-__host__ __device__ __forceinline__ constexpr int PREP(int k) {   // pair representatives, k = 0..8
-  constexpr int a[9] = {1, 3, 5, 7, 8, 11, 12, 15, 16};
-  return a[k];
-}
-__host__ __device__ __forceinline__ constexpr bool MEVEN(int r) {
-  for (int c = 0; c < 19; c++)
-    if (MROW(r, OPC(c)) != MROW(r, c)) return false;
-  return true;
-}
-
-// rows relaxed with the fixed rate 1 (density, momentum)
-__host__ __device__ __forceinline__ constexpr bool MCONS(int r) { return r == 0 || r == 3 || r == 5 || r == 7; }
-
 template <int... Is, typename F>
 __device__ __forceinline__ void static_for_impl(F&& f, std::integer_sequence<int, Is...>) {
   (f(std::integral_constant<int, Is>{}), ...);
@@ -297,76 +284,6 @@ __device__ __forceinline__ void static_for_impl(F&& f, std::integer_sequence<int
 template <int N, typename F>
 __device__ __forceinline__ void static_for(F&& f) {
   static_for_impl(f, std::make_integer_sequence<int, N>{});
-}
-
-template <typename R>
-__device__ __forceinline__ void mrt_collide_pairs(const DevParams& P, R f[19], R rho, R ux, R uy, R uz, R fx, R fy,
-                                                  R fz, R rhoN) {
-  R su, se, seps, sq, spi, sm;
-  node_rates_fast<R>(P, rhoN, su, se, seps, sq, spi, sm);
-  R pp[9], qq[9];
-  static_for<9>([&](auto kc) {
-    constexpr int k = decltype(kc)::value;
-    pp[k] = f[PREP(k)] + f[OPC(PREP(k))];
-    qq[k] = f[PREP(k)] - f[OPC(PREP(k))];
-  });
-  R m[19];
-  static_for<19>([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    constexpr bool even = MEVEN(r);
-    R acc = R(0);
-    if constexpr (MCONS(r)) return;   // relaxed with rate 1: not needed (below)
-    if constexpr (even && MROW(r, 0) != 0.0) acc = R(MROW(r, 0)) * f[0];
-    static_for<9>([&](auto kc) {
-      constexpr int k = decltype(kc)::value;
-      constexpr double c = MROW(r, PREP(k));
-      const R v = even ? pp[k] : qq[k];
-      if constexpr (c == 1.0) acc = acc + v;
-      else if constexpr (c == -1.0) acc = acc - v;
-      else if constexpr (c != 0.0) acc = acc + R(c) * v;
-    });
-    m[r] = acc;
-  });
-  R meq[19], fk[19];
-  equilf<R, false>(meq, fk, rho, ux, uy, uz, fx, fy, fz);
-  const R s[19] = {R(1), se, seps, R(1), sq, R(1), sq, R(1), sq, su, spi, su, spi, su, su, su, sm, sm, sm};
-  // density and momentum relax with rate 1 (:684): m - (m - meq) + fk/2 = meq + fk/2
-  static_for<19>([&](auto kc) {
-    constexpr int k = decltype(kc)::value;
-    if constexpr (MCONS(k)) m[k] = meq[k] + R(0.5) * fk[k];
-    else m[k] = m[k] - s[k] * (m[k] - meq[k]) + (R(1) - R(0.5) * s[k]) * fk[k];
-  });
-  static_for<9>([&](auto kc) {
-    constexpr int i = PREP(decltype(kc)::value);
-    R e = R(0), o = R(0);
-    static_for<19>([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      if constexpr (MINV(i, r) != 0.0) {
-        if constexpr (MEVEN(r)) e = e + R(MINV(i, r)) * m[r];
-        else o = o + R(MINV(i, r)) * m[r];
-      }
-    });
-    f[i] = e + o;
-    f[OPC(i)] = e - o;
-  });
-  if constexpr (sizeof(R) == 4) {
-    // FP32 arithmetic: the rest population closes the mass balance, so the
-    // post-collision populations sum to rho up to the rounding of these
-    // additions.  The rounded inverse-transform coefficients would otherwise
-    // bias every node's mass the same way, step after step (a drift of about
-    // 1e-9 per step).
-    R s = R(0);
-#pragma unroll
-    for (int i = 1; i < 19; i++) s = s + f[i];
-    f[0] = rho - s;
-  } else {
-    R e = R(0);
-    static_for<19>([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      if constexpr (MEVEN(r) && MINV(0, r) != 0.0) e = e + R(MINV(0, r)) * m[r];
-    });
-    f[0] = e;
-  }
 }
 
 // Link fraction of curve2 (Source1.f90:1055-1070): node at displacement
@@ -450,7 +367,8 @@ __device__ __forceinline__ void akai_rotate_sc(R sc, R cc, const R nw[3], const 
 }
 
 // wall normal for solid object `id` seen from node (x,y,z) (0-based indices)
-__device__ __forceinline__ void wall_normal_dev(const DevParams& P, const sym_particles* S, int id, int x, int y,
+template <typename PT>
+__device__ __forceinline__ void wall_normal_dev(const PT& P, const sym_particles* S, int id, int x, int y,
                                                 int z, double nw[3]) {
   if (id <= P.par) {
     const int par = P.par;

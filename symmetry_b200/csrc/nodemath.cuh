@@ -1,5 +1,7 @@
 // nodemath.cuh -- the fused path's per-node arithmetic (collision + Recolor,
-// Source1.f90:599-732) over a value type V: double, or float.
+// Source1.f90:599-732) over a value type V: double, or F2, two nodes' FP32
+// values in one register pair (one instruction does both: FP32 arithmetic is
+// bound by instruction issue, not by the FP32 units).
 //
 // The 19x19 moment transform of the reference is factored through the sums
 // and differences of opposite populations: an even row of M sees only
@@ -17,6 +19,19 @@ namespace fused {
 
 __device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
+
+struct F2 {
+  float2 v;
+  __device__ __forceinline__ F2() {}
+  __device__ __forceinline__ explicit F2(float a) : v(make_float2(a, a)) {}
+  __device__ __forceinline__ F2(float a, float b) : v(make_float2(a, b)) {}
+  __device__ __forceinline__ explicit F2(float2 a) : v(a) {}
+  __device__ __forceinline__ float operator[](int k) const { return k ? v.y : v.x; }
+};
+__device__ __forceinline__ F2 vfma(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v, b.v, c.v)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return F2(__fadd2_rn(a.v, b.v)); }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return F2(__fmul2_rn(a.v, b.v)); }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return vfma(b, F2(-1.0f), a); }
 
 // Moments of one node in the order of the reference's M (density and momentum
 // first): what a node holds between its loads and its pushes.
@@ -63,8 +78,8 @@ __device__ __forceinline__ void to_moments(const V (&f)[19], Moments<V>& m) {
 // Reciprocal density and relaxation rates of a node (:674-684).  FP64 takes
 // one division for all three quotients.
 template <typename R>
-__device__ __forceinline__ void node_rates_fused(const DevParams& P, const NodeParams<R>& q, R phi, R rho, R& irho,
-                                                 R& su, R& sq) {
+__device__ __forceinline__ void node_rates_fused(const TileParams<R>& P, R phi, R rho, R& irho, R& su, R& sq) {
+  const NodeParams<R>& q = P.np;
   if (P.same_nu) {
     irho = qdiv<R>(R(1), rho);
     su = q.su;
@@ -89,38 +104,40 @@ __device__ __forceinline__ void node_rates_fused(const DevParams& P, const NodeP
 // Relaxation with Guo forcing (:686): m - s (m - meq) + (1 - s/2) fk per row, the
 // equilibrium and forcing moments of equilf (:397-450).  Density and momentum
 // relax with rate 1: meq + fk/2.  u already carries half the force.
+// m may hold the moments of f - w rho_ref for any rho_ref (w rho_ref is the rest
+// equilibrium, its own fixed point); rho is the node's whole density.
 template <typename V, typename R>
-__device__ __forceinline__ void relax(Moments<V>& m, V ux, V uy, V uz, V fx, V fy, V fz, V su, V se, V seps, V sq,
-                                      V spi, V sm) {
+__device__ __forceinline__ void relax(Moments<V>& m, V rho, V ux, V uy, V uz, V fx, V fy, V fz, V su, V se, V seps,
+                                      V sq, V spi, V sm) {
   auto k = [](double v) { return V(R(v)); };
-  const V rho = m.rho;
   const V rx = rho * ux, ry = rho * uy, rz = rho * uz;
   const V xx = rx * ux, yy = ry * uy, zz = rz * uz;
-  const V us = xx + yy + zz;                                  // rho u^2
+  const V yz = yy + zz, us = xx + yz;                         // rho u^2
   const V gx = ux * fx, gy = uy * fy, gz = uz * fz;
-  const V uf = gx + gy + gz;
+  const V gyz = gy + gz, uf = gx + gyz;
   const V one = k(1), half = k(-0.5);
   const V hu = vfma(half, su, one), he = vfma(half, se, one), hp = vfma(half, seps, one), hq = vfma(half, sq, one),
           hi = vfma(half, spi, one);
   // row = row + s (eq - row) + h fk
   auto row = [](V& v, V s, V eq, V h, V fk) { v = vfma(s, eq - v, vfma(h, fk, v)); };
-  row(m.e, se, vfma(k(19), us, k(-11) * rho), he, k(38) * uf);
-  row(m.eps, seps, vfma(k(-5.5), us, k(3) * rho), hp, k(-11) * uf);
-  const V exx = vfma(k(3), xx, -us), fxx = vfma(k(3), gx, -uf);
-  row(m.pxx, su, exx, hu, fxx + fxx);
-  row(m.pixx, spi, half * exx, hi, -fxx);
-  const V eww = yy - zz, fww = gy - gz;
-  row(m.pww, su, eww, hu, fww + fww);
-  row(m.piww, spi, half * eww, hi, -fww);
+  row(m.e, se, vfma(k(19), us, k(-11) * m.rho), he, k(38) * uf);
+  row(m.eps, seps, vfma(k(-5.5), us, k(3) * m.rho), hp, k(-11) * uf);
+  const V exx = vfma(k(2), xx, k(-1) * yz), fxx = vfma(k(4), gx, k(-2) * gyz);
+  row(m.pxx, su, exx, hu, fxx);
+  row(m.pixx, spi, half * exx, half * hi, fxx);
+  const V eww = yy - zz, fww = k(2) * (gy - gz);
+  row(m.pww, su, eww, hu, fww);
+  row(m.piww, spi, half * eww, half * hi, fww);
   row(m.pxy, su, rx * uy, hu, vfma(ux, fy, uy * fx));
   row(m.pyz, su, ry * uz, hu, vfma(uy, fz, uz * fy));
   row(m.pxz, su, rx * uz, hu, vfma(ux, fz, uz * fx));
-  const V t = k(-2.0 / 3.0), hqt = hq * t, sqt = sq * t;
-  // q: eq = t rho u, fk = t f
-  m.qx = vfma(sqt, rx, vfma(-sq, m.qx, vfma(hqt, fx, m.qx)));
-  m.qy = vfma(sqt, ry, vfma(-sq, m.qy, vfma(hqt, fy, m.qy)));
-  m.qz = vfma(sqt, rz, vfma(-sq, m.qz, vfma(hqt, fz, m.qz)));
-  m.mx = vfma(-sm, m.mx, m.mx); m.my = vfma(-sm, m.my, m.my); m.mz = vfma(-sm, m.mz, m.mz);
+  // q: eq = -2/3 rho u, fk = -2/3 f
+  const V hqt = hq * k(-2.0 / 3.0), nq = k(-1) * sq, c = k(2.0 / 3.0);
+  m.qx = vfma(nq, vfma(c, rx, m.qx), vfma(hqt, fx, m.qx));
+  m.qy = vfma(nq, vfma(c, ry, m.qy), vfma(hqt, fy, m.qy));
+  m.qz = vfma(nq, vfma(c, rz, m.qz), vfma(hqt, fz, m.qz));
+  const V om = one - sm;
+  m.mx = om * m.mx; m.my = om * m.my; m.mz = om * m.mz;
   m.jx = vfma(k(0.5), fx, rx); m.jy = vfma(k(0.5), fy, ry); m.jz = vfma(k(0.5), fz, rz);
 }
 

@@ -26,6 +26,7 @@ struct FastState {
   uint2* links = nullptr;  // particles: momentum link lists [particle][box block][256] (see particles.cuh)
   int* nlinks = nullptr;   // entries of each [particle][box block]
   long long link_blocks = 0;   // blocks of one particle's momentum box
+  unsigned char* solid_tiles = nullptr;   // domains with solids: see DevParams
   int* status = nullptr;   // sticky: bit 0 an accumulated density was not finite or out of
                            // range, bit 1 a shared-memory tile load did not complete in time
   // TMA descriptors of the halo-padded phase field and reference-pair arrays, per parity
@@ -120,6 +121,7 @@ int fast_import(sym_handle* h);   // canonical -> fast
 int fast_export(sym_handle* h);   // fast -> canonical
 int fast_macros(sym_handle* h);   // calmacros of the fused populations into rho, u, rho_N (fused state kept)
 int current_macros(sym_handle* h);   // calmacros of whichever state is current (capi.cu)
+int fast_solid_tiles(sym_handle* h);   // which tile planes have solids near, from the current masks
 int fast_step(sym_handle* h, int nsteps);
 int fast_step_timed(sym_handle* h, int nsteps, double ms[4]);
 int fast_neck_planes(sym_handle* h, double* out, cudaStream_t st);   // per-z red area, nz doubles

@@ -169,6 +169,24 @@ def test_reduced_storage_early_thread(storage, bound):
     assert e["u"] <= bound, e
 
 
+@pytest.mark.parametrize("storage,bound", [("fp32", 3e-3), ("fp16", 5e-3)])
+@pytest.mark.parametrize("bounce", [0, 1])
+@pytest.mark.parametrize("centre", [(16.0, 16.0, 20.0), (4.6, 31.2, 0.4)])
+def test_reduced_storage_walls_and_particle(storage, bound, bounce, centre):
+    """Wetting walls and a moving sphere in FP32 arithmetic against the oracle,
+    the sphere inside the box and close to a wall across the periodic edges of
+    y and z (rows of both halves of a tile, first and last tiles), with either
+    bounce-back, 50 steps.  Bounds: those of the early thread, whose velocities
+    are smaller."""
+    w = configs.c2_wall_particle(nx=32, ny=35, nz=61, rad=3.4, centre=centre, z0=20.0, z1=44.0)
+    w.params.bounce = bounce
+    o, L = fast_run(w, 50, storage)
+    fluid = o.arr("walls_all") == 0
+    e = errors(o, L, ["ux", "uy", "uz", "rho", "rho_N"], mask=fluid)
+    assert e["u"] <= bound and e["rho"] <= 1e-4 and e["rho_N"] <= bound, e
+    compare_masks(o, L, ["walls", "walls_all", "pin", "pout"])
+
+
 def test_reduced_storage_breakup_time():
     """Breakup time of the reduced storages within 1 % of FP64's on two
     unstable threads of the batched mix that break within 12,000 steps

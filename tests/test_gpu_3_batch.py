@@ -114,3 +114,21 @@ def test_tile_extent_does_not_change_results(storage, xchunk):
         rm, bm, cm = state(m)
         assert np.array_equal(ra, rm) and np.array_equal(ba, bm), w.name
     B.close()
+
+
+@pytest.mark.parametrize("storage", ["fp64", "fp16"])
+@pytest.mark.parametrize("n", [16, 17, 130])
+def test_batch_sizes_of_the_descriptor_tables(storage, n):
+    """A batch's descriptors are kernel parameters in a small or a large table,
+    or in global memory beyond it: at the tables' edges each domain's result
+    equals the one it gets alone, bit for bit."""
+    ws = [configs.c1_thread(nx=6 + k % 5, ny=7 + k % 3, nz=9 + k % 7, radius=2.0, storage=storage) for k in range(n)]
+    members = [setup_workload(w) for w in ws]
+    B = Batch(members)
+    B.step(4)
+    for k in sorted({0, 1, n // 2, n - 2, n - 1}):
+        a = setup_workload(ws[k])
+        a.step(4)
+        assert np.array_equal(a.get("ri"), members[k].get("ri")), k
+        assert np.array_equal(a.get("bi"), members[k].get("bi")), k
+    B.close()
