@@ -228,8 +228,11 @@ int sym_movement(sym_handle* h);          /* movement         Source1.f90:1263-1
 int sym_refilling(sym_handle* h);         /* refilling        Source1.f90:1351-1418 */
 
 /* One loop body of main (Source1.f90:216-251, output gate excluded), nsteps
- * times.  REFERENCE mode runs the subroutine kernels above in the reference
- * order; CONFIG mode runs the fused fast path in the handle's storage mode. */
+ * times.  REFERENCE mode runs the reference's order with passes over the
+ * populations merged (halfway bounce-back; the first call allocates a second
+ * streaming target of 152 bytes per node, and where there is no room for it the
+ * subroutine kernels above run one by one); CONFIG mode runs the fused fast path
+ * in the handle's storage mode. */
 int sym_step(sym_handle* h, int nsteps);
 /* sym_step with CUDA events recorded on the handle's stream (CONFIG mode).
  * use_graph=0: eager launches, ms[0]=whole region, ms[1]=phase-field kernel,

@@ -213,20 +213,80 @@ int canonical_step_once(sym_handle* h) {
   return ref_curve(h);
 }
 
-int canonical_steps(sym_handle* h, int nsteps) {
-  if (!h->gexec) {
+// Pieces a run of steps is made of, each a captured graph.  STEP is one loop
+// body by itself.  In the reference's geometry with the halfway bounce-back a
+// run is HEAD, MID ..., TAIL (or ONLY), cut between calmacros' streaming and
+// calmacros (see k_step_macros in ref_kernels.cu).
+enum { STEP, HEAD, MID, TAIL, ONLY };
+
+int canonical_piece(sym_handle* h, int piece) {
+  if (piece == STEP) return canonical_step_once(h);
+  const bool last = piece == TAIL || piece == ONLY;
+  int e;
+  if ((e = ref_step_macros(h, piece == MID || piece == TAIL, last))) return e;
+  if (h->p.par > 0) {
+    if ((e = part_lagrange_points(h))) return e;
+    if ((e = part_capillary_force2(h))) return e;
+    if ((e = part_momentum(h))) return e;
+    if ((e = part_repulsive(h))) return e;
+    if ((e = part_movement(h))) return e;
+  }
+  if ((e = part_set_walls(h))) return e;
+  if (h->p.par > 0)
+    if ((e = part_refilling(h, !last))) return e;
+  if ((e = ref_derivatives(h))) return e;
+  if ((e = ref_collide_recolor(h, last))) return e;
+  if ((e = ref_boundary(h))) return e;
+  if (!last) return SYM_OK;
+  if ((e = ref_stream_both(h))) return e;
+  return ref_curve(h);
+}
+
+// launches a piece, captured on its first use from the present arrangement of
+// the arrays (streaming leaves them permuted)
+int run_piece(sym_handle* h, int piece) {
+  double** const cur[4] = {&h->ri, &h->bi, &h->ft, &h->ft2};
+  StepGraph* g = nullptr;
+  for (StepGraph& q : h->graphs)
+    if (q.piece == piece && q.from[0] == h->ri && q.from[1] == h->bi && q.from[2] == h->ft && q.from[3] == h->ft2)
+      g = &q;
+  if (!g) {
+    StepGraph q;
+    q.piece = piece;
+    for (int k = 0; k < 4; k++) q.from[k] = *cur[k];
     if (int e = check_cuda(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal), "begin capture"))
       return e;
-    const int e1 = canonical_step_once(h);
-    cudaGraph_t g = nullptr;
-    const cudaError_t e2 = cudaStreamEndCapture(h->st, &g);
-    if (e1) { if (g) cudaGraphDestroy(g); return e1; }
-    if (int e = check_cuda(h, e2, "end capture")) return e;
-    h->graph = g;
-    if (int e = check_cuda(h, cudaGraphInstantiate(&h->gexec, g, 0), "graph instantiate")) return e;
+    const int e1 = canonical_piece(h, piece);
+    const cudaError_t e2 = cudaStreamEndCapture(h->st, &q.graph);
+    for (int k = 0; k < 4; k++) {
+      q.to[k] = *cur[k];
+      *cur[k] = q.from[k];   // captured, not run
+    }
+    int e = e1 ? e1 : check_cuda(h, e2, "end capture");
+    if (!e) e = check_cuda(h, cudaGraphInstantiate(&q.exec, q.graph, 0), "graph instantiate");
+    if (e) {
+      if (q.graph) cudaGraphDestroy(q.graph);
+      return e;
+    }
+    h->graphs.push_back(q);
+    g = &h->graphs.back();
   }
-  for (int t = 0; t < nsteps; t++)
-    if (int e = check_cuda(h, cudaGraphLaunch(h->gexec, h->st), "graph launch")) return e;
+  if (int e = check_cuda(h, cudaGraphLaunch(g->exec, h->st), "graph launch")) return e;
+  for (int k = 0; k < 4; k++) *cur[k] = g->to[k];
+  return SYM_OK;
+}
+
+int canonical_steps(sym_handle* h, int nsteps) {
+  // the second streaming target: without room for it the steps run one by one
+  bool runs = h->dp.ref && !h->p.bounce;
+  if (runs && !h->ft2 && dalloc(h, &h->ft2, 19 * h->N)) {
+    h->ft2 = nullptr;
+    runs = false;
+  }
+  for (int t = 0; t < nsteps; t++) {
+    const int piece = !runs ? STEP : (nsteps == 1 ? ONLY : (t == 0 ? HEAD : (t + 1 < nsteps ? MID : TAIL)));
+    if (int e = run_piece(h, piece)) return e;
+  }
   return check_cuda(h, cudaStreamSynchronize(h->st), "step");
 }
 
@@ -388,10 +448,12 @@ int sym_destroy(sym_handle* h) {
   if (!h) return SYM_OK;
   cudaSetDevice(h->device);
   if (h->st) cudaStreamSynchronize(h->st);
-  if (h->gexec) cudaGraphExecDestroy(h->gexec);
-  if (h->graph) cudaGraphDestroy(h->graph);
+  for (StepGraph& g : h->graphs) {
+    cudaGraphExecDestroy(g.exec);
+    cudaGraphDestroy(g.graph);
+  }
   fast_free(h);
-  void* ptrs[] = {h->ri, h->bi, h->fi, h->ffi, h->ft, h->rho, h->ux, h->uy, h->uz, h->rhoN, h->rhoR, h->rhoB,
+  void* ptrs[] = {h->ri, h->bi, h->fi, h->ffi, h->ft, h->ft2, h->rho, h->ux, h->uy, h->uz, h->rhoN, h->rhoR, h->rhoB,
                   h->nx, h->ny, h->nz, h->gx, h->gy, h->gz, h->flag, h->walls, h->walls_old, h->walls_all,
                   h->pin, h->pout, h->dpart, h->lax, h->lay, h->laz, h->larhon, h->lanx, h->lany, h->lanz,
                   h->lads, h->laflag, h->red};

@@ -7,8 +7,9 @@
 
 namespace symb200 {
 
-void mirror_int_all(sym_handle* h, int32_t* a, int axis);
+void mirror_masks(sym_handle* h);
 void mirror_macros_all(sym_handle* h);
+void mirror_phi(sym_handle* h);
 
 namespace {
 
@@ -34,18 +35,21 @@ __global__ void k_walls_flat(DevParams P, int32_t* walls, int32_t* walls_all) {
   walls[a] = P.par + 1; walls_all[a] = 10;
   walls[b] = P.par + 2; walls_all[b] = 10;
 }
-__global__ void k_walls_mark(DevParams P, Box b, const sym_particles* __restrict__ S, int pp, double r2,
-                             int32_t* walls, int32_t* walls_all) {
+// blockIdx.y: the particle (every particle of a handle in one launch: a driver's
+// set_walls of 12 particles was 24 launches)
+__global__ void k_walls_mark(DevParams P, Box b, const sym_particles* __restrict__ S, double r2, int32_t* walls,
+                             int32_t* walls_all) {
   int x, y, z;
+  const int pp = blockIdx.y + 1;
   if (!box_node(P, b, S->center, pp, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
-  walls_mark_node(P, S, pp, r2, x, y, z, walls, walls_all);
+  walls_mark_last(P, S, pp, r2, x, y, z, walls, walls_all);
 }
-__global__ void k_walls_pinpout_box(DevParams P, Box b, const sym_particles* __restrict__ S, int id,
+__global__ void k_walls_pinpout_box(DevParams P, Box b, const sym_particles* __restrict__ S,
                                     const int32_t* __restrict__ walls, const int32_t* __restrict__ walls_all,
                                     int32_t* pin, int32_t* pout) {
   int x, y, z;
-  if (!box_node(P, b, S->center, id, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
-  pinpout_node(P, x, y, z, id, walls, walls_all, pin, pout);
+  if (!box_node(P, b, S->center, blockIdx.y + 1, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
+  pinpout_particles(P, x, y, z, walls, walls_all, pin, pout);
 }
 __global__ void k_walls_pinpout_plane(DevParams P, int xplane, int id, const int32_t* __restrict__ walls,
                                       const int32_t* __restrict__ walls_all, int32_t* pin, int32_t* pout) {
@@ -82,12 +86,12 @@ __global__ void k_capillary_final(DevParams P, sym_particles* S, const double* _
 }
 
 // ---- momentum (Source1.f90:1178-1261) ------------------------------------------
-__global__ void k_momentum(DevParams P, Box b, int pp, const sym_particles* __restrict__ S,
+__global__ void k_momentum(DevParams P, Box b, const sym_particles* __restrict__ S,
                            const int32_t* __restrict__ walls, const int32_t* __restrict__ pout,
                            const double* __restrict__ fi, const double* __restrict__ ffi, double* part,
                            long long nblk) {
   __shared__ double sh[256];
-  momentum_partial(P, b, pp, S, walls, pout, fi, ffi, part, nblk, blockIdx.x, sh);
+  momentum_partial(P, b, blockIdx.y + 1, S, walls, pout, fi, ffi, part, nblk, blockIdx.x, sh);
 }
 __global__ void k_momentum_final(DevParams P, sym_particles* S, const double* part, long long nblk) {
   __shared__ double sh[256];
@@ -95,21 +99,22 @@ __global__ void k_momentum_final(DevParams P, sym_particles* S, const double* pa
 }
 
 // ---- repulsive (Source1.f90:1594-1671) and movement (:1263-1349) -----------------
-__global__ void k_repulsive(DevParams P, sym_particles* S) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  repulsive_body(P, S);
+__global__ void k_repulsive(DevParams P, sym_particles* S) {   // one thread per particle
+  if ((int)threadIdx.x < P.par) repulsive_one(P, S, threadIdx.x + 1);
 }
 __global__ void k_movement(DevParams P, sym_particles* S) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  movement_body(P, S);
+  if ((int)threadIdx.x < P.par) movement_one(P, S, threadIdx.x + 1);
 }
 
 // ---- refilling (Source1.f90:1351-1418) --------------------------------------------
-__global__ void k_refill(DevParams P, Box b, int pp, const sym_particles* __restrict__ S,
+// every particle in one launch: a refilled node belongs to one particle (pout)
+// and reads fluid neighbours of the previous masks only, which no refill writes
+__global__ void k_refill(DevParams P, Box b, const sym_particles* __restrict__ S,
                          const int32_t* __restrict__ pout, const int32_t* __restrict__ walls_old, double* rho,
                          double* rhoN, double* rhoR, double* rhoB, double* ux, double* uy, double* uz, double* ri,
                          double* bi, double* fi) {
   int x, y, z;
+  const int pp = blockIdx.y + 1;
   if (!box_node(P, b, S->center_old, pp, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
   refill_node(P, pp, S, pout, walls_old, rho, rhoN, rhoR, rhoB, ux, uy, uz, ri, bi, fi, x, y, z);
 }
@@ -152,21 +157,17 @@ int part_set_walls(sym_handle* h) {
     k_walls_flat<<<blocks_for((long long)P.ny * P.nz), TPB, 0, h->st>>>(P, h->walls, h->walls_all);
   const double r2 = P.rad * P.rad;
   const Box bm = sphere_box(h, 1.0), bp = sphere_box(h, 3.0);
-  for (int pp = 1; pp <= P.par; pp++)
-    k_walls_mark<<<blocks_for(bm.count()), TPB, 0, h->st>>>(P, bm, h->dpart, pp, r2, h->walls, h->walls_all);
+  if (P.par)
+    k_walls_mark<<<dim3(blocks_for(bm.count()), P.par), TPB, 0, h->st>>>(P, bm, h->dpart, r2, h->walls, h->walls_all);
   if (!P.ref && P.wall_x) {
     const unsigned g = blocks_for((long long)P.ny * P.nz);
     k_walls_pinpout_plane<<<g, TPB, 0, h->st>>>(P, 1, P.par + 1, h->walls, h->walls_all, h->pin, h->pout);
     k_walls_pinpout_plane<<<g, TPB, 0, h->st>>>(P, P.nx - 2, P.par + 2, h->walls, h->walls_all, h->pin, h->pout);
   }
-  for (int pp = 1; pp <= P.par; pp++)
-    k_walls_pinpout_box<<<blocks_for(bp.count()), TPB, 0, h->st>>>(P, bp, h->dpart, pp, h->walls, h->walls_all,
-                                                                    h->pin, h->pout);
-  if (P.ref) {
-    int32_t* arrs[4] = {h->walls, h->walls_all, h->pin, h->pout};
-    for (int ax = 0; ax < 3; ax++)
-      for (auto* a : arrs) mirror_int_all(h, a, ax);
-  }
+  if (P.par)
+    k_walls_pinpout_box<<<dim3(blocks_for(bp.count()), P.par), TPB, 0, h->st>>>(P, bp, h->dpart, h->walls,
+                                                                                h->walls_all, h->pin, h->pout);
+  if (P.ref) mirror_masks(h);
   return check_cuda(h, cudaGetLastError(), "set_walls");
 }
 
@@ -199,33 +200,34 @@ int part_momentum(sym_handle* h) {
   const Box b = sphere_box(h, 3.0);
   const long long nblk = (b.count() + 255) / 256;
   if ((size_t)(nblk * 6 * P.par) > h->red_len) return set_error(h, SYM_ERR_STATE, "momentum scratch too small");
-  for (int pp = 1; pp <= P.par; pp++)
-    k_momentum<<<(unsigned)nblk, 256, 0, h->st>>>(P, b, pp, h->dpart, h->walls, h->pout, h->fi, h->ffi, h->red,
-                                                  nblk);
+  k_momentum<<<dim3((unsigned)nblk, P.par), 256, 0, h->st>>>(P, b, h->dpart, h->walls, h->pout, h->fi, h->ffi, h->red,
+                                                             nblk);
   k_momentum_final<<<P.par, 256, 0, h->st>>>(P, h->dpart, h->red, nblk);
   return check_cuda(h, cudaGetLastError(), "momentum");
 }
 
 int part_repulsive(sym_handle* h) {
   if (h->dp.par == 0) return SYM_OK;
-  k_repulsive<<<1, 1, 0, h->st>>>(h->dp, h->dpart);
+  k_repulsive<<<1, SYM_MAX_PAR, 0, h->st>>>(h->dp, h->dpart);
   return check_cuda(h, cudaGetLastError(), "repulsive");
 }
 
 int part_movement(sym_handle* h) {
   if (h->dp.par == 0) return SYM_OK;
-  k_movement<<<1, 1, 0, h->st>>>(h->dp, h->dpart);
+  k_movement<<<1, SYM_MAX_PAR, 0, h->st>>>(h->dp, h->dpart);
   return check_cuda(h, cudaGetLastError(), "movement");
 }
 
-int part_refilling(sym_handle* h) {
+// phi_only: only rho_N goes onto the mirror planes (inside a run of steps)
+int part_refilling(sym_handle* h, bool phi_only) {
   const DevParams& P = h->dp;
   if (P.par == 0) return SYM_OK;
   const Box b = sphere_box(h, 4.0);
-  for (int pp = 1; pp <= P.par; pp++)
-    k_refill<<<blocks_for(b.count()), TPB, 0, h->st>>>(P, b, pp, h->dpart, h->pout, h->walls_old, h->rho, h->rhoN,
-                                                        h->rhoR, h->rhoB, h->ux, h->uy, h->uz, h->ri, h->bi, h->fi);
-  if (P.ref) mirror_macros_all(h);
+  k_refill<<<dim3(blocks_for(b.count()), P.par), TPB, 0, h->st>>>(P, b, h->dpart, h->pout, h->walls_old, h->rho,
+                                                                  h->rhoN, h->rhoR, h->rhoB, h->ux, h->uy, h->uz,
+                                                                  h->ri, h->bi, h->fi);
+  if (P.ref && phi_only) mirror_phi(h);
+  else if (P.ref) mirror_macros_all(h);
   return check_cuda(h, cudaGetLastError(), "refilling");
 }
 

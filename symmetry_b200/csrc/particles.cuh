@@ -78,19 +78,35 @@ __device__ __forceinline__ void walls_reset_node(long long L, int32_t* walls, in
   walls_old[L] = walls_all[L];
   walls_all[L] = 0; walls[L] = 0; pin[L] = 0; pout[L] = 0;
 }
-// distance test with separately rounded products and sums (bit-exact masks)
-__device__ __forceinline__ void walls_mark_node(const DevParams& P, const sym_particles* S, int pp, double r2, int x,
-                                                int y, int z, int32_t* walls, int32_t* walls_all) {
+// node inside particle pp: distance test with separately rounded products and
+// sums (bit-exact masks)
+__device__ __forceinline__ bool inside(const DevParams& P, const sym_particles* S, int pp, double r2, int x, int y,
+                                       int z) {
   const int par = P.par;
   const double dx = disp(P, (double)(x + P.origin), PC(S->center, par, pp, 0), 0);
   const double dy = disp(P, (double)(y + P.origin), PC(S->center, par, pp, 1), 1);
   const double dz = disp(P, (double)(z + P.origin), PC(S->center, par, pp, 2), 2);
   const double d = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-  if (d <= r2) {
+  return d <= r2;
+}
+__device__ __forceinline__ void walls_mark_node(const DevParams& P, const sym_particles* S, int pp, double r2, int x,
+                                                int y, int z, int32_t* walls, int32_t* walls_all) {
+  if (inside(P, S, pp, r2, x, y, z)) {
     const long long L = lin(P, x, y, z);
     walls[L] = pp;
     walls_all[L] = 10;
   }
+}
+// the same where all particles are marked at once: a node inside several keeps
+// the last one's mark
+__device__ __forceinline__ void walls_mark_last(const DevParams& P, const sym_particles* S, int pp, double r2, int x,
+                                                int y, int z, int32_t* walls, int32_t* walls_all) {
+  if (!inside(P, S, pp, r2, x, y, z)) return;
+  for (int q = pp + 1; q <= P.par; q++)
+    if (inside(P, S, q, r2, x, y, z)) return;
+  const long long L = lin(P, x, y, z);
+  walls[L] = pp;
+  walls_all[L] = 10;
 }
 __device__ __forceinline__ void pinpout_node(const DevParams& P, int x, int y, int z, int id,
                                              const int32_t* __restrict__ walls, const int32_t* __restrict__ walls_all,
@@ -102,6 +118,26 @@ __device__ __forceinline__ void pinpout_node(const DevParams& P, int x, int y, i
     const long long nb = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
     if (walls[nb] == id) { pout[L] = id; pin[nb] = id; }
   }
+}
+
+// pin and pout of node (x,y,z) next to any particles: pout names the last of them
+// (the threads of several particles' boxes write the same values)
+__device__ __forceinline__ void pinpout_particles(const DevParams& P, int x, int y, int z,
+                                                  const int32_t* __restrict__ walls,
+                                                  const int32_t* __restrict__ walls_all, int32_t* pin, int32_t* pout) {
+  if (!in_range(P, x, y, z)) return;
+  const long long L = lin(P, x, y, z);
+  if (walls_all[L] != 0) return;
+  int last = 0;
+  for (int i = 1; i < 19; i++) {
+    const long long nb = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
+    const int w = walls[nb];
+    if (w >= 1 && w <= P.par) {
+      pin[nb] = w;
+      last = w > last ? w : last;
+    }
+  }
+  if (last) pout[L] = last;
 }
 
 // ---- Lagrange_points (Source1.f90:1799-1978) ----------------------------------
@@ -473,13 +509,14 @@ __device__ __forceinline__ void momentum_links_partial(const DevParams& P, int p
   }
 }
 
-// ---- repulsive (Source1.f90:1594-1671), one thread ---------------------------------
-__device__ __forceinline__ void repulsive_body(const DevParams& P, sym_particles* S) {
+// ---- repulsive (Source1.f90:1594-1671) of particle pp ------------------------------
+// (each particle's sum runs over the others in the reference's order, so one
+// thread per particle gives the reference's result)
+__device__ __forceinline__ void repulsive_one(const DevParams& P, sym_particles* S, int pp) {
   const int par = P.par;
   const double range = 3.0, order = 0.01, Fg = P.fg, rad = P.rad;
-  for (int c = 0; c < 3 * par; c++) S->fre[c] = 0.0;
   auto sqd = [](double a) { return a * a; };
-  for (int pp = 1; pp <= par; pp++) {
+  {
     const double cx = PC(S->center, par, pp, 0), cy = PC(S->center, par, pp, 1), cz = PC(S->center, par, pp, 2);
     double fx = 0.0, fy = 0.0, fz = 0.0;
     if (P.ref) {
@@ -499,8 +536,8 @@ __device__ __forceinline__ void repulsive_body(const DevParams& P, sym_particles
     }
     S->fre[0 * par + pp - 1] = fx; S->fre[1 * par + pp - 1] = fy; S->fre[2 * par + pp - 1] = fz;
   }
-  for (int i = 1; i <= par; i++)
-    for (int j = 1; j <= par; j++) {
+  const int i = pp;
+  for (int j = 1; j <= par; j++) {
       if (i == j) continue;
       double d[3];
       for (int c = 0; c < 3; c++) d[c] = PC(S->center, par, i, c) - PC(S->center, par, j, c);
@@ -516,12 +553,13 @@ __device__ __forceinline__ void repulsive_body(const DevParams& P, sym_particles
     }
 }
 
-// ---- movement (Source1.f90:1263-1349), one thread ------------------------------------
-__device__ __forceinline__ void movement_body(const DevParams& P, sym_particles* S) {
+// ---- movement (Source1.f90:1263-1349) of particle pp, after every particle's
+// repulsive_one -------------------------------------------------------------------
+__device__ __forceinline__ void movement_one(const DevParams& P, sym_particles* S, int pp) {
   const int par = P.par;
   auto A = [&](double* a, int pp, int k) -> double& { return a[k * par + pp - 1]; };
   if (P.ref) {
-    for (int pp = 1; pp <= par; pp++) {
+    {
       if (fabs(A(S->center0, pp, 0) - ((double)P.nx - 0.5)) < 0.1) {
         A(S->fp, pp, 0) = 0.0; A(S->fp, pp, 1) = 2.0 * A(S->fp, pp, 1); A(S->fp, pp, 2) = 2.0 * A(S->fp, pp, 2);
         A(S->tp, pp, 0) = 2.0 * A(S->tp, pp, 0); A(S->tp, pp, 1) = 0.0; A(S->tp, pp, 2) = 0.0;
@@ -550,7 +588,7 @@ __device__ __forceinline__ void movement_body(const DevParams& P, sym_particles*
         A(S->tension_t, pp, 2) = 2.0 * A(S->tension_t, pp, 2);
       }
     }
-    for (int pp = 1; pp <= par; pp++) {
+    {
       if (pp == par / 3 + 1) {
         double t = (A(S->tension, pp, 0) + A(S->tension, pp, 2)) / 2.0;
         A(S->tension, pp, 0) = t; A(S->tension, pp, 2) = t;
@@ -564,19 +602,14 @@ __device__ __forceinline__ void movement_body(const DevParams& P, sym_particles*
     }
   }
   const double m = P.mass, I = P.inertia;
-  double F[3 * SYM_MAX_PAR];
-  for (int pp = 1; pp <= par; pp++)
-    for (int c = 0; c < 3; c++) {
-      double f = A(S->fp, pp, c) + A(S->fre, pp, c) + A(S->tension, pp, c);
-      if (!P.ref) f = f + m * P.body[c];
-      F[c * par + pp - 1] = f;
-      A(S->up, pp, c) = A(S->up, pp, c) + f / m;
-      A(S->rp, pp, c) = A(S->rp, pp, c) + (A(S->tp, pp, c) + A(S->tension_t, pp, c)) / I;
-    }
-  for (int c = 0; c < 3 * par; c++) S->center_old[c] = S->center[c];
-  for (int pp = 1; pp <= par; pp++)
-    for (int c = 0; c < 3; c++)
-      A(S->center, pp, c) = A(S->center, pp, c) + A(S->up, pp, c) + 0.5 * F[c * par + pp - 1] / m;
+  for (int c = 0; c < 3; c++) {
+    double f = A(S->fp, pp, c) + A(S->fre, pp, c) + A(S->tension, pp, c);
+    if (!P.ref) f = f + m * P.body[c];
+    A(S->up, pp, c) = A(S->up, pp, c) + f / m;
+    A(S->rp, pp, c) = A(S->rp, pp, c) + (A(S->tp, pp, c) + A(S->tension_t, pp, c)) / I;
+    A(S->center_old, pp, c) = A(S->center, pp, c);
+    A(S->center, pp, c) = A(S->center, pp, c) + A(S->up, pp, c) + 0.5 * f / m;
+  }
 }
 
 // ---- refilling (Source1.f90:1351-1418) --------------------------------------------

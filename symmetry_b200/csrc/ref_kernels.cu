@@ -6,7 +6,9 @@
 // kernel cites the loop it replaces.  Indices are 0-based: a reference node
 // (x,y,z) (1-based) is (x-1,y-1,z-1) here.
 #include <cstdio>
+#include <utility>
 #include <vector>
+#include "nodemath.cuh"
 #include "state.cuh"
 
 namespace symb200 {
@@ -35,71 +37,99 @@ __device__ __forceinline__ long long nbr(const DevParams& P, int x, int y, int z
   return lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
 }
 
-// ---- mirror-plane copies (symmetry_X/Y/Z_phi/_u/_fi, Source1.f90:1443-1542) ----
-// Copy plane `src` onto plane `dst` along `axis` for every node of the other two axes.
-__device__ __forceinline__ bool plane_node(const DevParams& P, int axis, int t, int dst, int src, long long& Ld,
-                                           long long& Ls) {
-  int a, b, na, nb;
-  if (axis == 0) { na = P.ny; nb = P.nz; }
-  else if (axis == 1) { na = P.nx; nb = P.nz; }
-  else { na = P.nx; nb = P.ny; }
-  if (t >= na * nb) return false;
-  a = t / nb; b = t % nb;
-  if (axis == 0) { Ld = lin(P, dst, a, b); Ls = lin(P, src, a, b); }
-  else if (axis == 1) { Ld = lin(P, a, dst, b); Ls = lin(P, a, src, b); }
-  else { Ld = lin(P, a, b, dst); Ls = lin(P, a, b, src); }
-  return true;
-}
-template <typename T>
-__global__ void k_plane_scalar(DevParams P, T* v, int axis, int dst, int src) {
-  long long Ld, Ls;
-  if (plane_node(P, axis, blockIdx.x * blockDim.x + threadIdx.x, dst, src, Ld, Ls)) v[Ld] = v[Ls];
-}
-__global__ void k_plane_u(DevParams P, double* a, double* b, double* c, int axis, int dst, int src) {
-  long long Ld, Ls;
-  if (!plane_node(P, axis, blockIdx.x * blockDim.x + threadIdx.x, dst, src, Ld, Ls)) return;
-  a[Ld] = axis == 0 ? -a[Ls] : a[Ls];
-  b[Ld] = axis == 1 ? -b[Ls] : b[Ls];
-  c[Ld] = axis == 2 ? -c[Ls] : c[Ls];
-}
-__global__ void k_plane_pop(DevParams P, double* f, int axis, int dst, int src) {
-  long long Ld, Ls;
-  if (!plane_node(P, axis, blockIdx.x * blockDim.x + threadIdx.x, dst, src, Ld, Ls)) return;
-  const long long N = P.N;
-  double tmp[19];
-#pragma unroll
-  for (int i = 0; i < 19; i++) {
-    const int s = axis == 0 ? SYMX(i) : (axis == 1 ? SYMY(i) : SYMZ(i));
-    tmp[i] = f[s * N + Ls];
+// ---- mirror planes (symmetry_X/Y/Z_phi/_u/_fi, Source1.f90:1443-1542) ---------
+// The reference copies plane n-1 onto plane n of x, then planes 2 and n-1 onto
+// 1 and n of y, then plane n-1 onto n of z.  A node on several mirror planes
+// ends with the value of the node mirrored in each of those axes, and no source
+// lies on a mirror plane, so one launch over the planes' nodes does all three
+// passes for every array (24 launches of calmacros before; 152^3: 380 us of a
+// 3.4 ms step were plane copies).
+struct MirrorSet {
+  double* scalar[4] = {};   // copied
+  double* vec[2][3] = {};   // the component along a mirrored axis changes sign
+  double* pop[2] = {};      // velocities mirrored
+  int32_t* mask[4] = {};
+  double* low = nullptr;    // also copied onto the wall planes x = 0 and z = 0 from their neighbours
+  int ns = 0, nv = 0, np = 0, nm = 0;
+};
+
+// velocity index of (cx, cy, cz)
+__constant__ unsigned char kDir[27] = {0, 10, 0, 14, 2, 12, 0, 8, 0, 18, 4, 16, 6, 0, 5, 17, 3, 15, 0, 9, 0, 13, 1, 11, 0, 7, 0};
+__device__ __forceinline__ int dir_index(int cx, int cy, int cz) { return kDir[(cx + 1) * 9 + (cy + 1) * 3 + cz + 1]; }
+
+// node (x, y, z) mirrored off the mirror planes; which axes were mirrored
+struct Image {
+  int x, y, z;
+  bool fx, fy, fz;
+  __device__ __forceinline__ int dir(int cx, int cy, int cz) const {
+    return dir_index(fx ? -cx : cx, fy ? -cy : cy, fz ? -cz : cz);
   }
-#pragma unroll
-  for (int i = 0; i < 19; i++) f[i * N + Ld] = tmp[i];
+};
+__device__ __forceinline__ Image image_of(const DevParams& P, int x, int y, int z) {
+  Image m;
+  m.fx = x == P.nx - 1;
+  m.fy = y == 0 || y == P.ny - 1;
+  m.fz = z == P.nz - 1;
+  m.x = m.fx ? P.nx - 2 : x;
+  m.y = y == 0 ? 1 : (m.fy ? P.ny - 2 : y);
+  m.z = m.fz ? P.nz - 2 : z;
+  return m;
 }
 
-int plane_threads(const DevParams& P, int axis) {
-  return axis == 0 ? P.ny * P.nz : (axis == 1 ? P.nx * P.nz : P.nx * P.ny);
+// t-th node of the boundary planes: x = nx-1, y = 0, y = ny-1, z = nz-1 and, with
+// `walls`, x = 0 and z = 0 (nodes on several planes come up once per plane, with
+// the same result)
+__device__ __forceinline__ bool plane_node(const DevParams& P, int t, bool walls, int& x, int& y, int& z) {
+  const int yz = P.ny * P.nz, xz = P.nx * P.nz, xy = P.nx * P.ny;
+  if (t < yz) { x = P.nx - 1; y = t / P.nz; z = t % P.nz; return true; }
+  t -= yz;
+  if (t < 2 * xz) {
+    y = t < xz ? 0 : P.ny - 1;
+    if (t >= xz) t -= xz;
+    x = t / P.nz; z = t % P.nz;
+    return true;
+  }
+  t -= 2 * xz;
+  if (t < xy) { x = t / P.ny; y = t % P.ny; z = P.nz - 1; return true; }
+  t -= xy;
+  if (!walls) return false;
+  if (t < yz) { x = 0; y = t / P.nz; z = t % P.nz; return true; }
+  t -= yz;
+  if (t < xy) { x = t / P.ny; y = t % P.ny; z = 0; return true; }
+  return false;
 }
-template <typename T>
-void mirror_scalar(sym_handle* h, T* v, int axis) {
-  const DevParams& P = h->dp;
-  const int n = axis == 0 ? P.nx : (axis == 1 ? P.ny : P.nz);
-  const unsigned g = blocks_for(plane_threads(P, axis));
-  k_plane_scalar<T><<<g, TPB, 0, h->st>>>(P, v, axis, n - 1, n - 2);
-  if (axis == 1) k_plane_scalar<T><<<g, TPB, 0, h->st>>>(P, v, axis, 0, 1);
+inline long long plane_count(const DevParams& P, bool walls) {
+  const long long yz = (long long)P.ny * P.nz, xz = (long long)P.nx * P.nz, xy = (long long)P.nx * P.ny;
+  return yz + 2 * xz + xy + (walls ? yz + xy : 0);
 }
-void mirror_u(sym_handle* h, double* a, double* b, double* c, int axis) {
-  const DevParams& P = h->dp;
-  const int n = axis == 0 ? P.nx : (axis == 1 ? P.ny : P.nz);
-  const unsigned g = blocks_for(plane_threads(P, axis));
-  k_plane_u<<<g, TPB, 0, h->st>>>(P, a, b, c, axis, n - 1, n - 2);
-  if (axis == 1) k_plane_u<<<g, TPB, 0, h->st>>>(P, a, b, c, axis, 0, 1);
+
+__global__ void __launch_bounds__(TPB) k_mirror(DevParams P, MirrorSet S) {
+  int x, y, z;
+  if (!plane_node(P, blockIdx.x * TPB + threadIdx.x, S.low != nullptr, x, y, z)) return;
+  const Image m = image_of(P, x, y, z);
+  const long long Ld = lin(P, x, y, z), N = P.N;
+  if (S.low) S.low[Ld] = S.low[lin(P, m.x == 0 ? 1 : m.x, m.y, m.z == 0 ? 1 : m.z)];
+  if (!(m.fx || m.fy || m.fz)) return;
+  const long long Ls = lin(P, m.x, m.y, m.z);
+  for (int k = 0; k < S.ns; k++) S.scalar[k][Ld] = S.scalar[k][Ls];
+  for (int k = 0; k < S.nm; k++) S.mask[k][Ld] = S.mask[k][Ls];
+  for (int k = 0; k < S.nv; k++) {
+    const double a = S.vec[k][0][Ls], b = S.vec[k][1][Ls], c = S.vec[k][2][Ls];
+    S.vec[k][0][Ld] = m.fx ? -a : a;
+    S.vec[k][1][Ld] = m.fy ? -b : b;
+    S.vec[k][2][Ld] = m.fz ? -c : c;
+  }
+  for (int k = 0; k < S.np; k++) {
+    double* const f = S.pop[k];
+    double tmp[19];
+#pragma unroll
+    for (int i = 0; i < 19; i++) tmp[i] = f[m.dir(CX(i), CY(i), CZ(i)) * N + Ls];
+#pragma unroll
+    for (int i = 0; i < 19; i++) f[i * N + Ld] = tmp[i];
+  }
 }
-void mirror_pop(sym_handle* h, double* f, int axis) {
-  const DevParams& P = h->dp;
-  const int n = axis == 0 ? P.nx : (axis == 1 ? P.ny : P.nz);
-  const unsigned g = blocks_for(plane_threads(P, axis));
-  k_plane_pop<<<g, TPB, 0, h->st>>>(P, f, axis, n - 1, n - 2);
-  if (axis == 1) k_plane_pop<<<g, TPB, 0, h->st>>>(P, f, axis, 0, 1);
+void mirror(sym_handle* h, const MirrorSet& S) {
+  k_mirror<<<blocks_for(plane_count(h->dp, S.low != nullptr)), TPB, 0, h->st>>>(h->dp, S);
 }
 
 // ---- calmacros (Source1.f90:770-831) --------------------------------------
@@ -137,12 +167,24 @@ __global__ void k_calmacros(DevParams P, const double* __restrict__ ri, const do
   rhoN[L] = (sr - sb) / rh;
 }
 
-void mirror_macros(sym_handle* h, bool with_fi) {
-  for (int ax = 0; ax < 3; ax++) {
-    mirror_scalar(h, h->rhoN, ax); mirror_scalar(h, h->rhoR, ax); mirror_scalar(h, h->rhoB, ax);
-    mirror_scalar(h, h->rho, ax); mirror_u(h, h->ux, h->uy, h->uz, ax);
-    if (with_fi) mirror_pop(h, h->fi, ax);
-  }
+// rho_N, rho_R, rho_B, rho, u and fi; wall_phi: rho_N also onto the wall planes
+void mirror_macros(sym_handle* h, bool wall_phi) {
+  MirrorSet S;
+  S.scalar[S.ns++] = h->rhoR;
+  S.scalar[S.ns++] = h->rhoB;
+  S.scalar[S.ns++] = h->rho;
+  if (wall_phi) S.low = h->rhoN;
+  else S.scalar[S.ns++] = h->rhoN;
+  S.vec[0][0] = h->ux; S.vec[0][1] = h->uy; S.vec[0][2] = h->uz;
+  S.nv = 1;
+  S.pop[S.np++] = h->fi;
+  mirror(h, S);
+}
+void mirror_colours(sym_handle* h) {
+  MirrorSet S;
+  S.pop[S.np++] = h->ri;
+  S.pop[S.np++] = h->bi;
+  mirror(h, S);
 }
 
 // ---- derivatives (Source1.f90:452-597) ------------------------------------
@@ -161,8 +203,8 @@ __global__ void k_pin_fill(DevParams P, const int32_t* __restrict__ pin, const i
   rhoN[L] = v / ws;
 }
 
-__global__ void k_gradient(DevParams P, const int32_t* __restrict__ walls_all, const double* __restrict__ rhoN,
-                           double* gx, double* gy, double* gz, double* nx, double* ny, double* nz, int32_t* flag) {
+__global__ void k_gradient(DevParams P, const sym_particles* __restrict__ S, const int32_t* __restrict__ pout,
+                           const int32_t* __restrict__ walls_all, const double* __restrict__ rhoN, double* gx, double* gy, double* gz, double* nx, double* ny, double* nz, int32_t* flag) {
   int x, y, z;
   if (!range_node(P, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
   const long long L = lin(P, x, y, z);
@@ -180,23 +222,17 @@ __global__ void k_gradient(DevParams P, const int32_t* __restrict__ walls_all, c
     const double fnorm = sqrt(g0 * g0 + g1 * g1 + g2 * g2);
     if (fnorm > P.evap) { n0 = g0 / fnorm; n1 = g1 / fnorm; n2 = g2 / fnorm; fl = 1; }
   }
+  // rotated to the contact angle next to a solid (:535-587)
+  const int pp = fl ? pout[L] : 0;
+  if (pp >= 1) {
+    double nw[3], n[3] = {n0, n1, n2}, v[3];
+    wall_normal_dev(P, S, pp, x, y, z, nw);
+    akai_rotate<double>(P.cita, nw, n, true, v);
+    n0 = v[0]; n1 = v[1]; n2 = v[2];
+    const double fnorm = sqrt(g0 * g0 + g1 * g1 + g2 * g2);
+    g0 = fnorm * v[0]; g1 = fnorm * v[1]; g2 = fnorm * v[2];
+  }
   gx[L] = g0; gy[L] = g1; gz[L] = g2; nx[L] = n0; ny[L] = n1; nz[L] = n2; flag[L] = fl;
-}
-
-__global__ void k_wetting(DevParams P, const sym_particles* __restrict__ S, const int32_t* __restrict__ pout,
-                          const int32_t* __restrict__ flag, double* gx, double* gy, double* gz, double* nx, double* ny,
-                          double* nz) {
-  int x, y, z;
-  if (!range_node(P, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
-  const long long L = lin(P, x, y, z);
-  const int pp = pout[L];
-  if (!(pp >= 1 && flag[L])) return;
-  double nw[3], n[3] = {nx[L], ny[L], nz[L]}, v[3];
-  wall_normal_dev(P, S, pp, x, y, z, nw);
-  akai_rotate<double>(P.cita, nw, n, true, v);
-  nx[L] = v[0]; ny[L] = v[1]; nz[L] = v[2];
-  const double fnorm = sqrt(gx[L] * gx[L] + gy[L] * gy[L] + gz[L] * gz[L]);
-  gx[L] = fnorm * v[0]; gy[L] = fnorm * v[1]; gz[L] = fnorm * v[2];
 }
 
 // ---- collision (Source1.f90:599-695) --------------------------------------
@@ -277,43 +313,54 @@ __global__ void k_recolor(DevParams P, const int32_t* __restrict__ walls_all, co
 }
 
 // ---- boundary (Source1.f90:1544-1592), REFERENCE geometry -------------------
-__global__ void k_bb_bottom(DevParams P, double* ri, double* bi) {  // bottom wall z=1 (1-based)
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P.nx * P.ny) return;
-  const int x = t / P.ny, y = t % P.ny, z = 1;
-  const long long N = P.N, L = lin(P, x, y, z);
+// Mirror planes, then the halfway bounce-back of the bottom wall z = 0 and of
+// the back wall x = 0 (0-based): link i of a node next to a wall comes back as
+// opc(i) of the wall node it enters.  One thread per boundary node gathers its
+// new populations; the reads go to nodes off the mirror planes, and on the wall
+// planes only to velocities that no thread writes.
+__global__ void __launch_bounds__(TPB) k_boundary(DevParams P, double* ri, double* bi) {
+  int x, y, z;
+  if (!plane_node(P, blockIdx.x * TPB + threadIdx.x, true, x, y, z)) return;
+  const long long N = P.N, Ld = lin(P, x, y, z);
+  const Image own = image_of(P, x, y, z);
+  const bool mirrored = own.fx || own.fy || own.fz;
+  const long long Lo = lin(P, own.x, own.y, own.z);
+  double tr[19], tb[19];
 #pragma unroll
-  for (int i = 1; i < 19; i++) {
-    const int zn = wrapi(z + CZ(i), P.nz);
-    if (zn == 0) {
-      const long long Ln = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), zn);
-      ri[OPC(i) * N + Ln] = ri[i * N + L];
-      bi[OPC(i) * N + Ln] = bi[i * N + L];
+  for (int i = 0; i < 19; i++) {
+    // (1,0,-1) of the row beside both walls: the back wall would return what
+    // the bottom wall just put there, its own value
+    const bool back = x == 0 && CX(i) > 0 && !(i == 13 && z == 1);
+    if ((z == 0 && CZ(i) > 0) || back) {
+      const Image m = image_of(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
+      const long long q = m.dir(-CX(i), -CY(i), -CZ(i)) * N + lin(P, m.x, m.y, m.z);
+      tr[i] = ri[q];
+      tb[i] = bi[q];
+    } else if (mirrored) {
+      const long long q = own.dir(CX(i), CY(i), CZ(i)) * N + Lo;
+      tr[i] = ri[q];
+      tb[i] = bi[q];
     }
   }
-}
-__global__ void k_bb_back(DevParams P, double* ri, double* bi) {  // back wall x=1 (1-based)
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P.ny * P.nz) return;
-  const int y = t / P.nz, z = t % P.nz, x = 1;
-  const long long N = P.N, L = lin(P, x, y, z);
 #pragma unroll
-  for (int i = 1; i < 19; i++) {
-    const int xn = wrapi(x + CX(i), P.nx);
-    if (xn == 0) {
-      const long long Ln = lin(P, xn, wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
-      ri[OPC(i) * N + Ln] = ri[i * N + L];
-      bi[OPC(i) * N + Ln] = bi[i * N + L];
+  for (int i = 0; i < 19; i++) {
+    const bool back = x == 0 && CX(i) > 0 && !(i == 13 && z == 1);
+    if ((z == 0 && CZ(i) > 0) || back || mirrored) {
+      ri[i * N + Ld] = tr[i];
+      bi[i * N + Ld] = tb[i];
     }
   }
 }
 
 // ---- streaming (Source1.f90:735-768): periodic pull, i = 1..18 ---------------
+// REST: the velocity at rest is carried over too
+template <bool REST>
 __global__ void k_stream_pull(DevParams P, const double* __restrict__ f, double* __restrict__ ft) {
   const long long L = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (L >= P.N) return;
   const int z = (int)(L % P.nz), y = (int)((L / P.nz) % P.ny), x = (int)(L / ((long long)P.nz * P.ny));
   const long long N = P.N;
+  if (REST) ft[L] = f[L];
 #pragma unroll
   for (int i = 1; i < 19; i++) {
     const long long src = lin(P, wrapi(x - CX(i), P.nx), wrapi(y - CY(i), P.ny), wrapi(z - CZ(i), P.nz));
@@ -408,6 +455,195 @@ __global__ void k_curve2(DevParams P, const sym_particles* __restrict__ S, const
       ri[i * N + L] = ri[j * N + B];
       bi[i * N + L] = bi[j * N + B];
     }
+  }
+}
+
+// ---- whole steps (sym_step, REFERENCE geometry, halfway bounce-back) -------------
+// A run of n steps is the reference's loop body n times, cut between the calls
+// so that passes over the populations fall together (152^3 per step, bytes per
+// node: separate subroutines about 2,700, these about 1,450):
+//   streaming of both colours, curve and the next step's calmacros in one pass
+//   (k_step_macros<true>), and collision with Recolor in one (k_collide_recolor).
+// What no later call of the same run reads is written by the run's last step
+// only (FULL): fi and ffi away from the particles, rho and u, and the mirror
+// planes' copies of them.
+
+// calmacros (:770-831) of the populations (ri, bi); PULL: of the populations
+// that streaming (:735-768) and curve (:990-1034) make of them, which go to
+// (ro, bo) on every node of the arrays.  !FULL: fi only next to particles (the
+// momentum exchange reads it there), no rho and u.
+template <bool PULL, bool FULL>
+__global__ void __launch_bounds__(TPB) k_step_macros(DevParams P, const sym_particles* __restrict__ S,
+                                                     const double* __restrict__ ri, const double* __restrict__ bi,
+                                                     double* __restrict__ ro, double* __restrict__ bo, double* fi,
+                                                     double* rho, double* ux, double* uy, double* uz, double* rhoN,
+                                                     double* rhoR, double* rhoB, const int32_t* __restrict__ walls,
+                                                     const int32_t* __restrict__ walls_all,
+                                                     const int32_t* __restrict__ pout) {
+  const long long N = P.N, L = blockIdx.x * (long long)TPB + threadIdx.x;
+  if (L >= N) return;
+  const unsigned Lu = (unsigned)L, q = Lu / (unsigned)P.nz;
+  const int z = (int)(Lu - q * (unsigned)P.nz), x = (int)(q / (unsigned)P.ny), y = (int)(q - (unsigned)x * P.ny);
+  const bool in = x >= P.lo[0] && x <= P.hi[0] && y >= P.lo[1] && y <= P.hi[1] && z >= P.lo[2] && z <= P.hi[2];
+  if (!PULL && !in) return;
+  const int pp = in ? pout[L] : 0;
+  const bool solid = in && walls_all[L] >= 1;
+  double r[19], b[19];
+  if (PULL) {
+    r[0] = ri[L];
+    b[0] = bi[L];
+#pragma unroll
+    for (int i = 1; i < 19; i++) {
+      const long long src = i * N + lin(P, wrapi(x - CX(i), P.nx), wrapi(y - CY(i), P.ny), wrapi(z - CZ(i), P.nz));
+      r[i] = ri[src];
+      b[i] = bi[src];
+    }
+    if (pp >= 1) {
+      // link i comes from a node of particle pp: this node's own opposite
+      // population, with the wall's velocity
+      const int par = P.par;
+      const double xr = disp(P, (double)(x + P.origin), S->center[0 * par + pp - 1], 0);
+      const double yr = disp(P, (double)(y + P.origin), S->center[1 * par + pp - 1], 1);
+      const double zr = disp(P, (double)(z + P.origin), S->center[2 * par + pp - 1], 2);
+      const double* up = S->up;
+      const double* rp = S->rp;
+      const double uw0 = up[0 * par + pp - 1] + zr * rp[1 * par + pp - 1] - yr * rp[2 * par + pp - 1];
+      const double uw1 = up[1 * par + pp - 1] + xr * rp[2 * par + pp - 1] - zr * rp[0 * par + pp - 1];
+      const double uw2 = up[2 * par + pp - 1] + yr * rp[0 * par + pp - 1] - xr * rp[1 * par + pp - 1];
+      const double cr = rhoR[L], cb = rhoB[L];
+#pragma unroll
+      for (int i = 1; i < 19; i++) {
+        if (walls[lin(P, x - CX(i), y - CY(i), z - CZ(i))] != pp) continue;
+        const double star = uw0 * (double)CX(i) + uw1 * (double)CY(i) + uw2 * (double)CZ(i);
+        r[i] = ri[OPC(i) * N + L] + 6.0 * W(i) * cr * star;
+        b[i] = bi[OPC(i) * N + L] + 6.0 * W(i) * cb * star;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 19; i++) {
+      ro[i * N + L] = r[i];
+      bo[i * N + L] = b[i];
+    }
+    if (!in) return;
+  }
+  if (solid) {
+    rhoN[L] = 0.0;
+    if (FULL) { ux[L] = 0.0; uy[L] = 0.0; uz[L] = 0.0; rho[L] = P.rho0; }
+    return;
+  }
+  if (!PULL) {
+#pragma unroll
+    for (int i = 0; i < 19; i++) {
+      r[i] = ri[i * N + L];
+      b[i] = bi[i * N + L];
+    }
+  }
+  double sr = 0.0, sb = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
+#pragma unroll
+  for (int i = 0; i < 19; i++) {
+    sr = sr + r[i];
+    sb = sb + b[i];
+    if (FULL || pp > 0) fi[i * N + L] = r[i] + b[i];
+    if (FULL) {
+      const double f = r[i] + b[i];
+      if (CX(i)) mx = mx + f * (double)CX(i);
+      if (CY(i)) my = my + f * (double)CY(i);
+      if (CZ(i)) mz = mz + f * (double)CZ(i);
+    }
+  }
+  rhoR[L] = sr; rhoB[L] = sb;
+  const double rh = sr + sb;
+  rhoN[L] = (sr - sb) / rh;
+  if (FULL) {
+    rho[L] = rh;
+    ux[L] = mx / rh; uy[L] = my / rh; uz[L] = mz / rh;
+  }
+}
+
+// collision (:599-695) and Recolor (:697-732) of one node from its populations,
+// in place; the collision in the fused path's arithmetic (nodemath.cuh), bound
+// by memory instead of FP64 issue (the two kernels: 816 + 366 us at 152^3).
+template <bool FULL>
+__global__ void __launch_bounds__(128, 4) k_collide_recolor(
+    DevParams P, const __grid_constant__ TileParams<double> T, const int32_t* __restrict__ walls_all,
+    const int32_t* __restrict__ pout, const int32_t* __restrict__ flag, const double* __restrict__ nxv,
+    const double* __restrict__ nyv, const double* __restrict__ nzv, const double* __restrict__ gx,
+    const double* __restrict__ gy, const double* __restrict__ gz, const double* __restrict__ rhoN, double* ux,
+    double* uy, double* uz, double* fi, double* ffi, double* ri, double* bi) {
+  using namespace fused;
+  const unsigned t = blockIdx.x * 128u + threadIdx.x;
+  const unsigned rz = P.hi[2] - P.lo[2] + 1, ry = P.hi[1] - P.lo[1] + 1;
+  const unsigned q = t / rz;
+  const int z = P.lo[2] + (int)(t - q * rz), x = P.lo[0] + (int)(q / ry), y = P.lo[1] + (int)(q % ry);
+  if (x > P.hi[0]) return;
+  const long long L = lin(P, x, y, z), N = P.N;
+  if (walls_all[L] > 0) return;
+  const int pp = pout[L];
+  const bool fl = flag[L] != 0;
+  double f[19], cr[19];
+#pragma unroll
+  for (int i = 0; i < 19; i++) {
+    cr[i] = ri[i * N + L];
+    f[i] = cr[i] + bi[i * N + L];
+  }
+  const double sr = cr[0] + ((cr[1] + cr[2]) + (cr[3] + cr[4]) + (cr[5] + cr[6])) +
+                    (((cr[7] + cr[10]) + (cr[8] + cr[9])) + ((cr[11] + cr[14]) + (cr[12] + cr[13])) +
+                     ((cr[15] + cr[18]) + (cr[16] + cr[17])));
+  Moments<double> m;
+  to_moments<double, double>(f, m);
+  const double rh = m.rho, sb = rh - sr;
+  double irho, su, sq;
+  node_rates_fused<double>(T, rhoN[L], rh, irho, su, sq);
+  const double n0 = nxv[L], n1 = nyv[L], n2 = nzv[L];
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  if (fl && pp <= 0 && z >= 2 && x >= 2) {   // z>=3 .and. x>=3 (1-based), :624
+    const double kurv = curvature<double, double>(
+        [&](auto ic, double (&d)[3]) {
+          constexpr int i = decltype(ic)::value;
+          const int o = CZ(i) + P.nz * (CY(i) + P.ny * CX(i));
+          d[0] = nxv[L + o] - nxv[L - o];
+          d[1] = nyv[L + o] - nyv[L - o];
+          d[2] = nzv[L + o] - nzv[L - o];
+        },
+        n0, n1, n2);
+    const double val = T.np.half_sigma * kurv;
+    fx = val * gx[L]; fy = val * gy[L]; fz = val * gz[L];
+  }
+  const double u0 = (m.jx + 0.5 * fx) * irho, u1 = (m.jy + 0.5 * fy) * irho, u2 = (m.jz + 0.5 * fz) * irho;
+  if (FULL) { ux[L] = u0; uy[L] = u1; uz[L] = u2; }
+  const NodeParams<double>& np = T.np;
+  relax<double, double>(m, rh, u0, u1, u2, fx, fy, fz, su, np.s_e > 0 ? np.s_e : su, np.s_eps > 0 ? np.s_eps : su,
+                        np.s_q > 0 ? np.s_q : sq, np.s_pi > 0 ? np.s_pi : su, np.s_m > 0 ? np.s_m : sq);
+  from_moments<double, double>(m, f);
+  if (FULL || pp > 0) {
+#pragma unroll
+    for (int i = 0; i < 19; i++) { fi[i * N + L] = f[i]; ffi[i * N + L] = f[i]; }
+  }
+  const bool rzero = sr <= P.evap, bzero = sb <= P.evap;
+  const double ratio = bzero ? 1.0 : (rzero ? 0.0 : sr * irho);
+  const double coef = (rzero || bzero || !fl) ? 0.0 : sr * sb * irho * np.beta;
+#pragma unroll
+  for (int i = 0; i < 19; i++) {
+    double r = ratio * f[i];
+    if (i > 0) r = fma(coef * W(i), n0 * (double)CX(i) + n1 * (double)CY(i) + n2 * (double)CZ(i), r);
+    ri[i * N + L] = r;
+    bi[i * N + L] = f[i] - r;
+  }
+}
+
+// streaming of both colours (every node, the velocity at rest carried over)
+__global__ void __launch_bounds__(TPB) k_stream_both(DevParams P, const double* __restrict__ ri,
+                                                     const double* __restrict__ bi, double* __restrict__ ro,
+                                                     double* __restrict__ bo) {
+  const long long N = P.N, L = blockIdx.x * (long long)TPB + threadIdx.x;
+  if (L >= N) return;
+  const unsigned Lu = (unsigned)L, q = Lu / (unsigned)P.nz;
+  const int z = (int)(Lu - q * (unsigned)P.nz), x = (int)(q / (unsigned)P.ny), y = (int)(q - (unsigned)x * P.ny);
+#pragma unroll
+  for (int i = 0; i < 19; i++) {
+    const long long src = i * N + lin(P, wrapi(x - CX(i), P.nx), wrapi(y - CY(i), P.ny), wrapi(z - CZ(i), P.nz));
+    ro[i * N + L] = ri[src];
+    bo[i * N + L] = bi[src];
   }
 }
 
@@ -599,11 +835,7 @@ int ref_calmacros(sym_handle* h) {
   const DevParams& P = h->dp;
   k_calmacros<<<blocks_for(range_count(P)), TPB, 0, h->st>>>(P, h->ri, h->bi, h->fi, h->rho, h->ux, h->uy, h->uz,
                                                               h->rhoN, h->rhoR, h->rhoB, h->walls_all);
-  if (P.ref) {
-    k_plane_scalar<double><<<blocks_for(plane_threads(P, 2)), TPB, 0, h->st>>>(P, h->rhoN, 2, 0, 1);  // z=1 wall
-    k_plane_scalar<double><<<blocks_for(plane_threads(P, 0)), TPB, 0, h->st>>>(P, h->rhoN, 0, 0, 1);  // x=1 wall
-    mirror_macros(h, true);
-  }
+  if (P.ref) mirror_macros(h, true);
   return check_cuda(h, cudaGetLastError(), "calmacros");
 }
 
@@ -611,13 +843,19 @@ int ref_derivatives(sym_handle* h) {
   const DevParams& P = h->dp;
   const unsigned g = blocks_for(range_count(P));
   k_pin_fill<<<g, TPB, 0, h->st>>>(P, h->pin, h->walls_all, h->rhoN);
-  if (P.ref)
-    for (int ax = 0; ax < 3; ax++) mirror_scalar(h, h->rhoN, ax);
-  k_gradient<<<g, TPB, 0, h->st>>>(P, h->walls_all, h->rhoN, h->gx, h->gy, h->gz, h->nx, h->ny, h->nz, h->flag);
-  k_wetting<<<g, TPB, 0, h->st>>>(P, h->dpart, h->pout, h->flag, h->gx, h->gy, h->gz, h->nx, h->ny, h->nz);
   if (P.ref) {
-    for (int ax = 0; ax < 3; ax++) mirror_u(h, h->nx, h->ny, h->nz, ax);
-    for (int ax = 0; ax < 3; ax++) mirror_u(h, h->gx, h->gy, h->gz, ax);
+    MirrorSet S;
+    S.scalar[S.ns++] = h->rhoN;
+    mirror(h, S);
+  }
+  k_gradient<<<g, TPB, 0, h->st>>>(P, h->dpart, h->pout, h->walls_all, h->rhoN, h->gx, h->gy, h->gz, h->nx, h->ny,
+                                   h->nz, h->flag);
+  if (P.ref) {
+    MirrorSet S;
+    S.vec[0][0] = h->nx; S.vec[0][1] = h->ny; S.vec[0][2] = h->nz;
+    S.vec[1][0] = h->gx; S.vec[1][1] = h->gy; S.vec[1][2] = h->gz;
+    S.nv = 2;
+    mirror(h, S);
   }
   return check_cuda(h, cudaGetLastError(), "derivatives");
 }
@@ -640,17 +878,24 @@ int ref_recolor(sym_handle* h) {
 int ref_boundary(sym_handle* h) {
   const DevParams& P = h->dp;
   if (!P.ref) return SYM_OK;
-  for (int ax = 0; ax < 3; ax++) { mirror_pop(h, h->ri, ax); mirror_pop(h, h->bi, ax); }
-  k_bb_bottom<<<blocks_for((long long)P.nx * P.ny), TPB, 0, h->st>>>(P, h->ri, h->bi);
-  k_bb_back<<<blocks_for((long long)P.ny * P.nz), TPB, 0, h->st>>>(P, h->ri, h->bi);
+  k_boundary<<<blocks_for(plane_count(P, true)), TPB, 0, h->st>>>(P, h->ri, h->bi);
   return check_cuda(h, cudaGetLastError(), "boundary");
 }
 
 int ref_streaming(sym_handle* h, int which) {
   const DevParams& P = h->dp;
-  double* f = which == 0 ? h->ri : h->bi;
-  k_stream_pull<<<blocks_for(P.N), TPB, 0, h->st>>>(P, f, h->ft);
-  cudaMemcpyAsync(f + P.N, h->ft + P.N, sizeof(double) * 18 * P.N, cudaMemcpyDeviceToDevice, h->st);
+  double*& f = which == 0 ? h->ri : h->bi;
+  if (P.ref) {
+    // the streamed populations are the handle's from here on (the old array
+    // becomes the temporary): no copy back of 18 of 19 velocities (152^3: 158 us
+    // per colour)
+    k_stream_pull<true><<<blocks_for(P.N), TPB, 0, h->st>>>(P, f, h->ft);
+    std::swap(f, h->ft);
+  } else {
+    // a CONFIG handle's arrays stay where the fused path's tables point
+    k_stream_pull<false><<<blocks_for(P.N), TPB, 0, h->st>>>(P, f, h->ft);
+    cudaMemcpyAsync(f + P.N, h->ft + P.N, sizeof(double) * 18 * P.N, cudaMemcpyDeviceToDevice, h->st);
+  }
   return check_cuda(h, cudaGetLastError(), "streaming");
 }
 
@@ -662,8 +907,7 @@ int ref_curve(sym_handle* h) {
   else
     k_curve<<<blocks_for(range_count(P)), TPB, 0, h->st>>>(P, h->dpart, h->walls, h->pout, h->ri, h->bi, h->rhoR,
                                                             h->rhoB);
-  if (P.ref)
-    for (int ax = 0; ax < 3; ax++) { mirror_pop(h, h->ri, ax); mirror_pop(h, h->bi, ax); }
+  if (P.ref) mirror_colours(h);
   return check_cuda(h, cudaGetLastError(), "curve");
 }
 
@@ -743,8 +987,66 @@ int soa_to_aos(sym_handle* h, const double* soa, double* aos) {
   return check_cuda(h, cudaGetLastError(), "soa_to_aos");
 }
 
-// exported for particles.cu (mirror sequences used by set_walls/refilling)
-void mirror_int_all(sym_handle* h, int32_t* a, int axis) { mirror_scalar<int32_t>(h, a, axis); }
-void mirror_macros_all(sym_handle* h) { mirror_macros(h, true); }
+// ---- the pieces of a run of steps (see k_step_macros) ----
+namespace {
+void mirror_phase(sym_handle* h, bool wall_phi, bool colours) {
+  MirrorSet S;
+  if (colours) {
+    S.scalar[S.ns++] = h->rhoR;
+    S.scalar[S.ns++] = h->rhoB;
+  }
+  if (wall_phi) S.low = h->rhoN;
+  else S.scalar[S.ns++] = h->rhoN;
+  mirror(h, S);
+}
+}  // namespace
+void mirror_phi(sym_handle* h) { mirror_phase(h, false, false); }
+
+int ref_step_macros(sym_handle* h, bool pull, bool full) {
+  const DevParams& P = h->dp;
+  auto go = [&](auto kern) {
+    kern<<<blocks_for(P.N), TPB, 0, h->st>>>(P, h->dpart, h->ri, h->bi, h->ft, h->ft2, h->fi, h->rho, h->ux, h->uy,
+                                             h->uz, h->rhoN, h->rhoR, h->rhoB, h->walls, h->walls_all, h->pout);
+  };
+  if (pull && full) go(k_step_macros<true, true>);
+  else if (pull) go(k_step_macros<true, false>);
+  else if (full) go(k_step_macros<false, true>);
+  else go(k_step_macros<false, false>);
+  if (pull) {
+    std::swap(h->ri, h->ft);
+    std::swap(h->bi, h->ft2);
+  }
+  if (full) mirror_macros(h, true);
+  else mirror_phase(h, true, true);
+  return check_cuda(h, cudaGetLastError(), "step macros");
+}
+
+int ref_collide_recolor(sym_handle* h, bool full) {
+  const DevParams& P = h->dp;
+  const unsigned g = blocks_for(range_count(P), 128);
+  auto go = [&](auto kern) {
+    kern<<<g, 128, 0, h->st>>>(P, tile_params<double>(P), h->walls_all, h->pout, h->flag, h->nx, h->ny, h->nz, h->gx,
+                               h->gy, h->gz, h->rhoN, h->ux, h->uy, h->uz, h->fi, h->ffi, h->ri, h->bi);
+  };
+  if (full) go(k_collide_recolor<true>);
+  else go(k_collide_recolor<false>);
+  return check_cuda(h, cudaGetLastError(), "collision and recolour");
+}
+
+int ref_stream_both(sym_handle* h) {
+  k_stream_both<<<blocks_for(h->dp.N), TPB, 0, h->st>>>(h->dp, h->ri, h->bi, h->ft, h->ft2);
+  std::swap(h->ri, h->ft);
+  std::swap(h->bi, h->ft2);
+  return check_cuda(h, cudaGetLastError(), "streaming");
+}
+
+// exported for particles.cu (the mirrors of set_walls and refilling)
+void mirror_masks(sym_handle* h) {
+  MirrorSet S;
+  S.mask[0] = h->walls; S.mask[1] = h->walls_all; S.mask[2] = h->pin; S.mask[3] = h->pout;
+  S.nm = 4;
+  mirror(h, S);
+}
+void mirror_macros_all(sym_handle* h) { mirror_macros(h, false); }
 
 }  // namespace symb200

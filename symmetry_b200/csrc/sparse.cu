@@ -143,13 +143,13 @@ __global__ void __launch_bounds__(kT) k_sp_momentum_final(const SpDom* __restric
   part::momentum_final_body(D.P, D.S, D.red, D.nblk_mom, e.pp, sh);
 }
 
-// repulsion then Newton-Euler, one thread per domain with particles
-__global__ void k_sp_move(const SpDom* __restrict__ doms, const int* __restrict__ list, int n) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const SpDom& D = doms[list[t]];
-  part::repulsive_body(D.P, D.S);
-  part::movement_body(D.P, D.S);
+// repulsion then Newton-Euler, one warp per domain with particles, one lane each
+__global__ void k_sp_move(const SpDom* __restrict__ doms, const int* __restrict__ list) {
+  const SpDom& D = doms[list[blockIdx.x]];
+  const int pp = threadIdx.x + 1;
+  if (pp <= D.P.par) part::repulsive_one(D.P, D.S, pp);
+  __syncwarp();
+  if (pp <= D.P.par) part::movement_one(D.P, D.S, pp);
 }
 
 // set_walls, reset: the masks of the previous step lie inside the previous
@@ -586,7 +586,7 @@ void enqueue_plan(SparsePlan* p, int k, cudaStream_t st) {
   go(k_sp_capillary_final, f[SparsePlan::CAPF], 32);
   go(k_sp_momentum, f[SparsePlan::MOM]);
   go(k_sp_momentum_final, f[SparsePlan::MOMF]);
-  if (p->nmove) k_sp_move<<<(p->nmove + 31) / 32, 32, 0, st>>>(D, p->d_move, p->nmove);
+  if (p->nmove) k_sp_move<<<p->nmove, SYM_MAX_PAR, 0, st>>>(D, p->d_move);
   go(k_sp_reset, f[SparsePlan::RESET]);
   go(k_sp_flat, f[SparsePlan::FLAT]);
   for (auto& t : p->mark) go(k_sp_mark, t);

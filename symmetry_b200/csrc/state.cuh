@@ -39,6 +39,14 @@ struct FastState {
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
 };
 
+// A captured piece of canonical steps: the arrays it starts from and those it leaves.
+struct StepGraph {
+  int piece = 0;
+  double *from[4] = {}, *to[4] = {};   // ri, bi, ft, ft2
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+};
+
 }  // namespace symb200
 
 struct sym_handle {
@@ -49,6 +57,7 @@ struct sym_handle {
   size_t N = 0;
   // canonical state (reference arrays, SoA, FP64)
   double *ri = nullptr, *bi = nullptr, *fi = nullptr, *ffi = nullptr, *ft = nullptr;
+  double* ft2 = nullptr;   // second streaming target (runs of steps in REFERENCE geometry, on first use)
   double *rho = nullptr, *ux = nullptr, *uy = nullptr, *uz = nullptr;
   double *rhoN = nullptr, *rhoR = nullptr, *rhoB = nullptr;
   double *nx = nullptr, *ny = nullptr, *nz = nullptr, *gx = nullptr, *gy = nullptr, *gz = nullptr;
@@ -63,9 +72,7 @@ struct sym_handle {
   size_t red_len = 0;
   double* hred = nullptr;           // pinned host scalars
   symb200::FastState fast;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t gexec = nullptr;
-  int graph_steps = 0;
+  std::vector<symb200::StepGraph> graphs;   // canonical steps
   size_t bytes = 0;
   // Every array the handle holds from creation is carved from one device
   // allocation (the slab): one cudaMalloc and one cudaFree per handle, no
@@ -93,6 +100,10 @@ int ref_recolor(sym_handle* h);
 int ref_boundary(sym_handle* h);
 int ref_streaming(sym_handle* h, int which);
 int ref_curve(sym_handle* h);
+// passes of a run of steps (REFERENCE geometry; need ft and ft2)
+int ref_step_macros(sym_handle* h, bool pull, bool full);
+int ref_collide_recolor(sym_handle* h, bool full);
+int ref_stream_both(sym_handle* h);
 int ref_initialization(sym_handle* h);
 int ref_init_fill(sym_handle* h);    // rhoN, rho given -> populations
 int ref_init_thread(sym_handle* h, double radius, double amp, double wavelength, double width, double noise,
@@ -111,7 +122,7 @@ int part_capillary_force2(sym_handle* h);
 int part_momentum(sym_handle* h);
 int part_repulsive(sym_handle* h);
 int part_movement(sym_handle* h);
-int part_refilling(sym_handle* h);
+int part_refilling(sym_handle* h, bool phi_only = false);
 int part_initia_center(sym_handle* h);
 
 // fused fast path, fast.cu
