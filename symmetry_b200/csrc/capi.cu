@@ -113,7 +113,7 @@ int dalloc(sym_handle* h, T** p, size_t n) {
   return e;
 }
 
-size_t reduction_len(const sym_params& p) {
+size_t reduction_len(const sym_params& p, int la_num) {
   const size_t N = (size_t)p.nx * p.ny * p.nz;
   size_t n = (N + 255) / 256 * 5 + 16;
   n = std::max(n, (size_t)p.nx + p.ny + p.nz + 16);
@@ -123,6 +123,8 @@ size_t reduction_len(const sym_params& p) {
     const size_t box = (size_t)(e * e * e);
     n = std::max(n, ((box + 255) / 256) * 6 * (size_t)p.par + 16);
     n = std::max(n, (size_t)32 * 7 * p.par + 16);   // capillary partial sums
+    // a fused step's capillary (256 points per block) and momentum partials side by side
+    n = std::max(n, (((size_t)la_num + 255) / 256 * 7 + (box + 255) / 256 * 6) * (size_t)p.par + 16);
   }
   return n;
 }
@@ -318,7 +320,7 @@ int alloc_state(sym_handle* h) {
       if (!e) e = dalloc(h, pp, NL);
     if (!e) e = dalloc(h, &h->laflag, NL);
   }
-  h->red_len = reduction_len(p);
+  h->red_len = reduction_len(p, h->dp.la_num);
   if (!e) e = dalloc(h, &h->red, h->red_len);
   if (!e && p.mode == SYM_MODE_CONFIG) e = fast_alloc(h);
   return e;

@@ -997,16 +997,13 @@ __device__ __forceinline__ void prep_node(const DevParams& P, const Pad& pd, con
 // densities), which it records in rr_old: the references this step's collide
 // decodes with
 template <typename S>
-__device__ __forceinline__ void refill_import_node(const DevParams& P, const Pad& pd, int pp, S* pops,
-                                                   typename Codec<S>::R* phi_cur, const int32_t* __restrict__ pout,
-                                                   const int32_t* __restrict__ walls_old,
-                                                   const double* __restrict__ ri, const double* __restrict__ bi,
+__device__ __forceinline__ void refill_import_node(const DevParams& P, const Pad& pd, S* pops,
+                                                   typename Codec<S>::R* phi_cur, const double* __restrict__ ri, const double* __restrict__ bi,
                                                    const double* __restrict__ rhoN, Ref* __restrict__ rr_old,
                                                    int x, int y, int z) {
   using R = typename Codec<S>::R;
   const long long L = lin(P, x, y, z);
   const unsigned N = (unsigned)P.N;
-  if (pout[L] != pp || walls_old[L] < 1) return;
   Ref ref{};
   if constexpr (Codec<S>::kRef) {
     double sr = 0.0, sb = 0.0;

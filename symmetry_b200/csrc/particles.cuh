@@ -294,8 +294,39 @@ __device__ __forceinline__ void block_sums(const double (&v)[K], double* sh) {
   }
 }
 
-// Shb (immersed area) and capillary_force2 (Source1.f90:1980-2028).  The
-// 16,380 Lagrange points of a particle are split over kCapBlocks blocks that
+// Shb (immersed area) and capillary_force2 (Source1.f90:1980-2028): what
+// Lagrange point `num` of particle pp adds to the seven sums (force, torque, area)
+__device__ __forceinline__ void capillary_add(const DevParams& P, const sym_particles* __restrict__ S,
+                                              const double* __restrict__ Lax, const double* __restrict__ Lay,
+                                              const double* __restrict__ Laz, const double* __restrict__ La_rhoN,
+                                              const double* __restrict__ La_nx, const double* __restrict__ La_ny,
+                                              const double* __restrict__ La_nz, const int32_t* __restrict__ La_flag,
+                                              const double* __restrict__ ds, int do_tension, int pp, int num,
+                                              double (&acc)[7]) {
+  const int par = P.par;
+  const double cx = PC(S->center, par, pp, 0), cy = PC(S->center, par, pp, 1), cz = PC(S->center, par, pp, 2);
+  const double k = 0.134 * 1.43;
+  const bool right = (P.cita == M_PI / 2.0);
+  const long long q = (long long)num * par + (pp - 1);
+  if (La_rhoN[q] > 0.0) acc[6] += ds[q];
+  if (!do_tension || !La_flag[q]) return;
+  double nw[3] = {Lax[q] - cx, Lay[q] - cy, Laz[q] - cz};
+  const double xr[3] = {nw[0], nw[1], nw[2]};
+  unitization(nw);
+  const double ie[3] = {-La_nx[q], -La_ny[q], -La_nz[q]};
+  double temp[3], nt[3], tt[3];
+  veccross(ie, nw, temp);
+  const double projector = sqrt(temp[0] * temp[0] + temp[1] * temp[1] + temp[2] * temp[2]);
+  veccross(temp, ie, nt);
+  unitization(nt);
+  const double rn = La_rhoN[q];
+  const double om = 1.0 - rn * rn;
+  const double star = 4.5 * k * P.beta * (om * om) * ds[q] * projector;
+  for (int c = 0; c < 3; c++) temp[c] = right ? star * nw[c] * P.sigma : star * nt[c] * P.sigma;
+  veccross(xr, temp, tt);
+  for (int c = 0; c < 3; c++) { acc[c] += temp[c]; acc[3 + c] += tt[c]; }
+}
+// The 16,380 Lagrange points of a particle are split over kCapBlocks blocks that
 // write fixed-order partial sums (part[(pp-1)*kCapBlocks + block][7]); the
 // final pass adds them in block order (deterministic).  Block-level: every
 // thread of the 256-thread block calls it, with kCapShared doubles of shared
@@ -309,31 +340,9 @@ __device__ __forceinline__ void capillary_partial(const DevParams& P, const sym_
                                                   const double* __restrict__ La_nz,
                                                   const int32_t* __restrict__ La_flag, const double* __restrict__ ds,
                                                   int do_tension, double* part, int pp, int blk, double* sh) {
-  const int par = P.par;
-  const double cx = PC(S->center, par, pp, 0), cy = PC(S->center, par, pp, 1), cz = PC(S->center, par, pp, 2);
-  const double k = 0.134 * 1.43;
-  const bool right = (P.cita == M_PI / 2.0);
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int num = blk * 256 + threadIdx.x; num < P.la_num; num += 256 * kCapBlocks) {
-    const long long q = (long long)num * par + (pp - 1);
-    if (La_rhoN[q] > 0.0) acc[6] += ds[q];
-    if (!do_tension || !La_flag[q]) continue;
-    double nw[3] = {Lax[q] - cx, Lay[q] - cy, Laz[q] - cz};
-    const double xr[3] = {nw[0], nw[1], nw[2]};
-    unitization(nw);
-    const double ie[3] = {-La_nx[q], -La_ny[q], -La_nz[q]};
-    double temp[3], nt[3], tt[3];
-    veccross(ie, nw, temp);
-    const double projector = sqrt(temp[0] * temp[0] + temp[1] * temp[1] + temp[2] * temp[2]);
-    veccross(temp, ie, nt);
-    unitization(nt);
-    const double rn = La_rhoN[q];
-    const double om = 1.0 - rn * rn;
-    const double star = 4.5 * k * P.beta * (om * om) * ds[q] * projector;
-    for (int c = 0; c < 3; c++) temp[c] = right ? star * nw[c] * P.sigma : star * nt[c] * P.sigma;
-    veccross(xr, temp, tt);
-    for (int c = 0; c < 3; c++) { acc[c] += temp[c]; acc[3 + c] += tt[c]; }
-  }
+  for (int num = blk * 256 + threadIdx.x; num < P.la_num; num += 256 * kCapBlocks)
+    capillary_add(P, S, Lax, Lay, Laz, La_rhoN, La_nx, La_ny, La_nz, La_flag, ds, do_tension, pp, num, acc);
   block_sums<256, 7>(acc, sh);
   if (threadIdx.x < 7) part[((size_t)(pp - 1) * kCapBlocks + blk) * 7 + threadIdx.x] = sh[threadIdx.x * 256];
 }
@@ -477,16 +486,24 @@ __device__ __forceinline__ void momentum_links_partial(const DevParams& P, int p
       const double uw0 = PC(S->up, par, pp, 0) + zr * PC(S->rp, par, pp, 1) - yr * PC(S->rp, par, pp, 2);
       const double uw1 = PC(S->up, par, pp, 1) + xr * PC(S->rp, par, pp, 2) - zr * PC(S->rp, par, pp, 0);
       const double uw2 = PC(S->up, par, pp, 2) + yr * PC(S->rp, par, pp, 0) - xr * PC(S->rp, par, pp, 1);
+      // the populations of all links are read at once (one after another behind
+      // their conditions, the reads were most of this kernel's time)
+      double f[19], g[19];
 #pragma unroll
       for (int i = 1; i < 19; i++) {
         // the reference's link i (neighbour x - c_i inside, :1193-1203) is
-        // bit OPC(i) of the mask; i ascending as there
+        // bit OPC(i) of the mask
+        const bool has = e.y >> OPC(i) & 1u;
+        f[i] = has ? fi[i * N + L] : 0.0;
+        g[i] = has ? ffi[OPC(i) * N + L] : 0.0;
+      }
+#pragma unroll
+      for (int i = 1; i < 19; i++) {   // i ascending as there
         if (!(e.y >> OPC(i) & 1u)) continue;
         const int j = OPC(i);
-        const double f = fi[i * N + L], g = ffi[j * N + L];
-        const double fmx = ((double)CX(i) - uw0) * f - ((double)CX(j) - uw0) * g;
-        const double fmy = ((double)CY(i) - uw1) * f - ((double)CY(j) - uw1) * g;
-        const double fmz = ((double)CZ(i) - uw2) * f - ((double)CZ(j) - uw2) * g;
+        const double fmx = ((double)CX(i) - uw0) * f[i] - ((double)CX(j) - uw0) * g[i];
+        const double fmy = ((double)CY(i) - uw1) * f[i] - ((double)CY(j) - uw1) * g[i];
+        const double fmz = ((double)CZ(i) - uw2) * f[i] - ((double)CZ(j) - uw2) * g[i];
         a[0] = a[0] - fmx; a[1] = a[1] - fmy; a[2] = a[2] - fmz;
         a[3] = a[3] - (yr * fmz - zr * fmy);
         a[4] = a[4] - (zr * fmx - xr * fmz);
@@ -613,14 +630,12 @@ __device__ __forceinline__ void movement_one(const DevParams& P, sym_particles* 
 }
 
 // ---- refilling (Source1.f90:1351-1418) --------------------------------------------
-__device__ __forceinline__ void refill_node(const DevParams& P, int pp, const sym_particles* __restrict__ S,
-                                            const int32_t* __restrict__ pout, const int32_t* __restrict__ walls_old,
-                                            double* rho, double* rhoN, double* rhoR, double* rhoB, double* ux,
+// the values of uncovered node (x,y,z), which belongs to particle pp
+__device__ __forceinline__ void refill_values(const DevParams& P, int pp, const sym_particles* __restrict__ S,
+                                              const int32_t* __restrict__ walls_old, double* rho, double* rhoN, double* rhoR, double* rhoB, double* ux,
                                             double* uy, double* uz, double* ri, double* bi, double* fi, int x, int y,
                                             int z) {
-  if (!in_range(P, x, y, z)) return;
   const long long L = lin(P, x, y, z), N = P.N;
-  if (pout[L] != pp || walls_old[L] < 1) return;
   const int par = P.par;
   const double xr = disp(P, (double)(x + P.origin), PC(S->center_old, par, pp, 0), 0);
   const double yr = disp(P, (double)(y + P.origin), PC(S->center_old, par, pp, 1), 1);
@@ -642,6 +657,17 @@ __device__ __forceinline__ void refill_node(const DevParams& P, int pp, const sy
     const double r = feq_srt<double>(i, R, u0, u1, u2, usqr), bb = feq_srt<double>(i, B, u0, u1, u2, usqr);
     ri[i * N + L] = r; bi[i * N + L] = bb; fi[i * N + L] = r + bb;
   }
+}
+
+__device__ __forceinline__ void refill_node(const DevParams& P, int pp, const sym_particles* __restrict__ S,
+                                            const int32_t* __restrict__ pout, const int32_t* __restrict__ walls_old,
+                                            double* rho, double* rhoN, double* rhoR, double* rhoB, double* ux,
+                                            double* uy, double* uz, double* ri, double* bi, double* fi, int x, int y,
+                                            int z) {
+  if (!in_range(P, x, y, z)) return;
+  const long long L = lin(P, x, y, z);
+  if (pout[L] != pp || walls_old[L] < 1) return;
+  refill_values(P, pp, S, walls_old, rho, rhoN, rhoR, rhoB, ux, uy, uz, ri, bi, fi, x, y, z);
 }
 
 }  // namespace part

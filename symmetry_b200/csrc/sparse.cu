@@ -2,31 +2,31 @@
 // :237-243 and the pin fill of derivatives :467-492) for every domain of a
 // batch, or the one domain of sym_step, at once.
 //
-// Each subroutine is one launch for all domains: a block table maps every
-// block of the launch to (domain, particle, block within that particle's
-// work), and a per-domain descriptor holds the domain's parameters, arrays
-// and particle boxes.  Per step, in the reference's order:
-//   prep            canonical views of the fused state on each particle box
-//   lagrange        Lagrange points (Lagrange_points :1799-1978)
-//   capillary       immersed area and capillary force, fixed-order partials
-//                   (:1864-1866, capillary_force2 :1980-2028), then the sums
-//   momentum        momentum exchange over the link lists (warp-shuffle
-//                   partials per box block), then the sums (:1178-1261)
-//   move            repulsion and Newton-Euler, one thread per domain
-//                   (:1594-1671, :1263-1349)
-//   set_walls       masks (:326-395): reset on the previous box, flat wall
-//                   planes, sphere marks, pin/pout and the link lists of the
-//                   next step's momentum
-//   refilling       uncovered nodes (:1351-1418) and into the fused state
-//   pin fill        fictitious phi on solid nodes next to fluid
+// A block table maps every block of a launch to (domain, particle, block
+// within that particle's work), and a per-domain descriptor holds the domain's
+// parameters, arrays and particle boxes.  The work is a chain of short,
+// latency-bound kernels, so what does not depend on one another shares a launch
+// (6 a step; one per subroutine, 14, took twice as long).  In the reference's
+// order:
+//   prep      canonical views of the fused state on each particle box
+//   forces    Lagrange points (Lagrange_points :1799-1978) with the immersed
+//             area and capillary force (:1864-1866, capillary_force2
+//             :1980-2028), fixed-order partials per block; beside them the
+//             momentum exchange over the link lists (warp-shuffle partials per
+//             box block, :1178-1261)
+//   move      the sums of both, repulsion and Newton-Euler, one block per
+//             domain (:1594-1671, :1263-1349)
+//   masks     set_walls (:326-395): on the previous box the new masks, flat
+//             wall planes, sphere marks
+//   pins      pin/pout and the link lists of the next step's momentum; beside
+//             them refilling (uncovered nodes, :1351-1418) and into the fused
+//             state
+//   pin fill  fictitious phi on solid nodes next to fluid
 // and, after the collide kernel, with the interpolated bounce-back:
-//   curve2          links into a particle re-set with the link fraction
-//                   (:1036-1101)
-// Masks, refills and sums are written per particle in the same order as the
-// per-handle kernels of particles.cu, so results are those of the drop-in
-// path bit for bit -- except the momentum sums, which add the same per-node
-// terms in another order (over the links instead of a box-wide tree): equal
-// to rounding.
+//   curve2    links into a particle re-set with the link fraction
+//             (:1036-1101)
+// Masks and refills are those of the per-handle kernels of particles.cu bit for
+// bit; the sums add the same terms in another fixed order: equal to rounding.
 #include <algorithm>
 #include <cstring>
 #include <string>
@@ -53,7 +53,7 @@ struct SpDom {
   double *gx, *gy, *gz, *nx, *ny, *nz;
   double *lax, *lay, *laz, *larhon, *lanx, *lany, *lanz, *lads;
   int32_t* laflag;
-  double* red;           // capillary partials, then momentum partials
+  double *red, *red_mom;   // partial sums of the capillary force and of the momentum exchange
   void* pops;            // fused populations of this step
   void* phic;            // this step's phase field (pin-filled below)
   void* phip;            // the previous step's phase field
@@ -67,7 +67,7 @@ struct SpDom {
   long long link_blocks;
   int* status;
   Box bprep, bmom, bmark, bpin, bref, bpfill;
-  long long nblk_mom;
+  long long nblk_mom, nblk_lag;
   int full_reset;        // more than one particle: masks reset on the whole domain
   int pad_;
 };
@@ -90,13 +90,6 @@ __global__ void __launch_bounds__(kT, 4) k_sp_prep(const SpDom* __restrict__ dom
                D.rhoR, D.rhoB, D.fi, D.gx, D.gy, D.gz, D.nx, D.ny, D.nz, D.rr_old, x, y, z);
 }
 
-__global__ void __launch_bounds__(kT, 4) k_sp_lagrange(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  part::lagrange_point(D.P, D.S, D.walls, D.rhoN, D.gx, D.gy, D.gz, D.nx, D.ny, D.nz, D.lax, D.lay, D.laz, D.larhon,
-                       D.lanx, D.lany, D.lanz, D.laflag, D.lads, e.b * kT + threadIdx.x, e.pp, D.ltab);
-}
-
 // the Lagrange points' sin/cos table of a domain, once per plan
 __global__ void __launch_bounds__(kT) k_sp_lagrange_table(const SpDom* __restrict__ doms,
                                                            const Blk* __restrict__ map) {
@@ -108,121 +101,185 @@ __global__ void __launch_bounds__(kT) k_sp_lagrange_table(const SpDom* __restric
   part::lagrange_trig(D.P, num, t[0], t[1], t[2], t[3]);
 }
 
-__global__ void __launch_bounds__(kT) k_sp_capillary(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  __shared__ double sh[part::kCapShared];
+// Lagrange points [b kT, (b+1) kT) of a particle and their capillary sums (v = 0),
+// or the momentum exchange over the link list of one block of its box (v = 1;
+// the list was written by the previous step's set_walls, or by the import)
+constexpr int kLagShared = 8 * 7;
+__global__ void __launch_bounds__(kT, 2) k_sp_forces(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
+  __shared__ double sh[kLagShared];
   const Blk e = map[blockIdx.x];
   const SpDom& D = doms[e.d];
-  part::capillary_partial(D.P, D.S, D.lax, D.lay, D.laz, D.larhon, D.lanx, D.lany, D.lanz, D.laflag, D.lads, 1,
-                          D.red, e.pp, e.b, sh);
-}
-
-// immersed area (Lagrange_points) and capillary force and torque
-// (capillary_force2) of one particle from the same partials
-__global__ void k_sp_capillary_final(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  part::capillary_final_body(D.P, D.S, D.red, 1, 1, e.pp, threadIdx.x);
-}
-
-// momentum exchange over the link list of one block of the particle's box
-// (written by the previous step's set_walls, or by the import)
-__global__ void __launch_bounds__(kT) k_sp_momentum(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  __shared__ double sh[8 * 6];
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  const long long seg = (long long)(e.pp - 1) * D.link_blocks + e.b;
-  part::momentum_links_partial(D.P, e.pp, D.S, D.pout, D.fi, D.ffi, D.links + seg * kT, D.nlinks[seg], D.red,
-                               D.nblk_mom, e.b, sh);
-}
-
-__global__ void __launch_bounds__(kT) k_sp_momentum_final(const SpDom* __restrict__ doms,
-                                                          const Blk* __restrict__ map) {
-  __shared__ double sh[kT];
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  part::momentum_final_body(D.P, D.S, D.red, D.nblk_mom, e.pp, sh);
-}
-
-// repulsion then Newton-Euler, one warp per domain with particles, one lane each
-__global__ void k_sp_move(const SpDom* __restrict__ doms, const int* __restrict__ list) {
-  const SpDom& D = doms[list[blockIdx.x]];
-  const int pp = threadIdx.x + 1;
-  if (pp <= D.P.par) part::repulsive_one(D.P, D.S, pp);
-  __syncwarp();
-  if (pp <= D.P.par) part::movement_one(D.P, D.S, pp);
-}
-
-// set_walls, reset: the masks of the previous step lie inside the previous
-// box of the particle (pout reaches one link beyond the sphere), or, with
-// more than one particle, anywhere: then the whole domain is reset
-__global__ void __launch_bounds__(kT) k_sp_reset(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  long long L;
-  if (D.full_reset) {
-    L = (long long)e.b * kT + threadIdx.x;
-    if (L >= D.P.N) return;
-  } else {
-    int x, y, z;
-    if (!part::box_node(D.P, D.bpin, D.S->center_old, 1, (long long)e.b * kT + threadIdx.x, x, y, z)) return;
-    L = lin(D.P, x, y, z);
+  if (e.v) {
+    const long long seg = (long long)(e.pp - 1) * D.link_blocks + e.b;
+    part::momentum_links_partial(D.P, e.pp, D.S, D.pout, D.fi, D.ffi, D.links + seg * kT, D.nlinks[seg], D.red_mom,
+                                 D.nblk_mom, e.b, sh);
+    return;
   }
-  part::walls_reset_node(L, D.walls, D.walls_old, D.walls_all, D.pin, D.pout);
+  const int num = e.b * kT + threadIdx.x;
+  double acc[7] = {0, 0, 0, 0, 0, 0, 0};
+  if (num < D.P.la_num) {
+    part::lagrange_point(D.P, D.S, D.walls, D.rhoN, D.gx, D.gy, D.gz, D.nx, D.ny, D.nz, D.lax, D.lay, D.laz, D.larhon,
+                         D.lanx, D.lany, D.lanz, D.laflag, D.lads, num, e.pp, D.ltab);
+    part::capillary_add(D.P, D.S, D.lax, D.lay, D.laz, D.larhon, D.lanx, D.lany, D.lanz, D.laflag, D.lads, 1, e.pp,
+                        num, acc);
+  }
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int c = 0; c < 7; c++) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
+    if (lane == 0) sh[warp * 7 + c] = acc[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < 7) {
+    double v = 0.0;
+    for (int w = 0; w < kT / 32; w++) v += sh[w * 7 + threadIdx.x];
+    D.red[((long long)(e.pp - 1) * D.nblk_lag + e.b) * 7 + threadIdx.x] = v;
+  }
 }
 
-// set_walls, flat wetting walls (CONFIG): the planes x = 0 and x = nx-1 are
-// solid at every step, so their previous mask (walls_old) is solid too
-__global__ void __launch_bounds__(kT) k_sp_flat(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  const int t = e.b * kT + threadIdx.x;
-  if (t >= D.P.ny * D.P.nz) return;
-  const int y = t / D.P.nz, z = t % D.P.nz;
-  const long long a = lin(D.P, 0, y, z), b = lin(D.P, D.P.nx - 1, y, z);
-  D.walls[a] = D.P.par + 1; D.walls_all[a] = 10; D.walls_old[a] = 10;
-  D.walls[b] = D.P.par + 2; D.walls_all[b] = 10; D.walls_old[b] = 10;
+// the sums of the partials, then repulsion and Newton-Euler: one block per
+// domain with particles, one warp per (particle, component) sum -- lanes in
+// strides, then a shuffle tree: a fixed order -- and one thread per particle
+__global__ void __launch_bounds__(kT) k_sp_move(const SpDom* __restrict__ doms, const int* __restrict__ list) {
+  const SpDom& D = doms[list[blockIdx.x]];
+  const int par = D.P.par;
+  const unsigned lane = threadIdx.x & 31u;
+  for (int s = threadIdx.x >> 5; s < 13 * par; s += kT / 32) {
+    const int pp = s / 13, c = s % 13;
+    const bool cap = c < 7;
+    const double* part = cap ? D.red + (long long)pp * D.nblk_lag * 7 + c
+                             : D.red_mom + (long long)pp * D.nblk_mom * 6 + (c - 7);
+    const long long n = cap ? D.nblk_lag : D.nblk_mom;
+    const int w = cap ? 7 : 6;
+    double v = 0.0;
+    for (long long b = lane; b < n; b += 32) v += part[b * w];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) {
+      if (c < 3) D.S->tension[c * par + pp] = v;
+      else if (c < 6) D.S->tension_t[(c - 3) * par + pp] = v;
+      else if (c == 6) D.S->shb[pp] = v;
+      else if (c < 10) D.S->fp[(c - 7) * par + pp] = v;
+      else D.S->tp[(c - 10) * par + pp] = v;
+    }
+  }
+  __syncthreads();
+  const int pp = threadIdx.x + 1;
+  if (pp <= par) part::repulsive_one(D.P, D.S, pp);
+  __syncthreads();
+  if (pp <= par) part::movement_one(D.P, D.S, pp);
 }
 
-__global__ void __launch_bounds__(kT) k_sp_mark(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
+// set_walls.  One particle (v = 0): the masks of the previous step lie inside the
+// particle's previous box (pout reaches one link beyond the sphere), where each
+// node becomes what it is now -- flat wall, sphere, fluid.  v = 1: the flat
+// wetting walls, solid at every step, so their previous mask is solid too.
+// v = 2: marks on the sphere's present box (where it left the previous one).
+// More than one particle: v = 3 clears the whole domain, and the marks (v = 2)
+// follow in a launch of their own.  Threads that meet on a node write the same.
+__global__ void __launch_bounds__(kT) k_sp_masks(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
   const Blk e = map[blockIdx.x];
   const SpDom& D = doms[e.d];
+  const DevParams& P = D.P;
+  const double r2 = P.rad * P.rad;
+  const long long t = (long long)e.b * kT + threadIdx.x;
   int x, y, z;
-  if (!part::box_node(D.P, D.bmark, D.S->center, e.pp, (long long)e.b * kT + threadIdx.x, x, y, z)) return;
-  part::walls_mark_node(D.P, D.S, e.pp, D.P.rad * D.P.rad, x, y, z, D.walls, D.walls_all);
-}
-
-// pin/pout of the flat walls: v = 0 the plane x = 1 (wall x = 0), v = 1 the
-// plane x = nx-2 (wall x = nx-1)
-__global__ void __launch_bounds__(kT) k_sp_pin_plane(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  const int t = e.b * kT + threadIdx.x;
-  if (t >= D.P.ny * D.P.nz) return;
-  const int xp = e.v == 0 ? 1 : D.P.nx - 2, id = D.P.par + 1 + e.v;
-  part::pinpout_node(D.P, xp, t / D.P.nz, t % D.P.nz, id, D.walls, D.walls_all, D.pin, D.pout);
+  if (e.v == 0) {
+    if (!part::box_node(P, D.bpin, D.S->center_old, 1, t, x, y, z)) return;
+    const long long L = lin(P, x, y, z);
+    const bool flat = P.wall_x && (x == 0 || x == P.nx - 1);
+    const bool in = part::inside(P, D.S, 1, r2, x, y, z);
+    D.walls_old[L] = flat ? 10 : D.walls_all[L];
+    D.walls_all[L] = in || flat ? 10 : 0;
+    D.walls[L] = in ? 1 : (flat ? P.par + (x == 0 ? 1 : 2) : 0);
+    D.pin[L] = 0;
+    D.pout[L] = 0;
+  } else if (e.v == 1) {
+    if (t >= 2LL * P.ny * P.nz) return;
+    const int side = t >= (long long)P.ny * P.nz;
+    const int u = (int)(t - (long long)side * P.ny * P.nz);
+    x = side ? P.nx - 1 : 0; y = u / P.nz; z = u % P.nz;
+    const long long L = lin(P, x, y, z);
+    int id = P.par + 1 + side;
+    for (int q = 1; q <= P.par; q++)
+      if (part::inside(P, D.S, q, r2, x, y, z)) id = q;
+    D.walls[L] = id; D.walls_all[L] = 10; D.walls_old[L] = 10;
+  } else if (e.v == 2) {
+    if (!part::box_node(P, D.bmark, D.S->center, e.pp, t, x, y, z)) return;
+    part::walls_mark_last(P, D.S, e.pp, r2, x, y, z, D.walls, D.walls_all);
+  } else {
+    if (t >= P.N) return;
+    const int xp = (int)(t / ((long long)P.ny * P.nz));
+    if (P.wall_x && (xp == 0 || xp == P.nx - 1)) {   // their marks are v = 1's
+      D.pin[t] = 0;
+      D.pout[t] = 0;
+    } else {
+      part::walls_reset_node(t, D.walls, D.walls_old, D.walls_all, D.pin, D.pout);
+    }
+  }
 }
 
 // pin/pout of particle pp on one block of its box, and that block's link list
-// for the next step's momentum (every thread takes part in the compaction)
-__global__ void __launch_bounds__(kT) k_sp_pin_box(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
+// for the next step's momentum (v = 0; every thread takes part in the
+// compaction); pin/pout of the flat walls (v = 1 the plane x = 1, v = 2 the
+// plane x = nx-2; a node also next to a particle is the particle's); refilling
+// (v = 3) with the import of each refilled node into the fused state: a
+// refilled node's import reads only what its own refill wrote, no refill reads a
+// refilled node (it averages fluid neighbours only), and the particle it
+// belongs to -- the last one next to it -- is read off the masks, not off pout
+template <typename S>
+__global__ void __launch_bounds__(kT, 2) k_sp_pins(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
+  using R = typename Codec<S>::R;
   __shared__ int sh[8];
   const Blk e = map[blockIdx.x];
   const SpDom& D = doms[e.d];
+  const DevParams& P = D.P;
+  const long long t = (long long)e.b * kT + threadIdx.x;
   int x, y, z;
-  bool has = false;
-  unsigned L = 0, mask = 0;
-  if (part::box_node(D.P, D.bpin, D.S->center, e.pp, (long long)e.b * kT + threadIdx.x, x, y, z) &&
-      part::in_range(D.P, x, y, z)) {
-    part::pinpout_node(D.P, x, y, z, e.pp, D.walls, D.walls_all, D.pin, D.pout);
-    const long long l = lin(D.P, x, y, z);
-    if (D.walls_all[l] == 0) {
-      mask = part::link_mask(D.P, x, y, z, e.pp, D.walls);
-      has = mask != 0;
-      L = (unsigned)l;
+  if (e.v == 0) {
+    bool has = false;
+    unsigned L = 0, mask = 0;
+    if (part::box_node(P, D.bpin, D.S->center, e.pp, t, x, y, z) && part::in_range(P, x, y, z)) {
+      part::pinpout_particles(P, x, y, z, D.walls, D.walls_all, D.pin, D.pout);
+      const long long l = lin(P, x, y, z);
+      if (D.walls_all[l] == 0) {
+        mask = part::link_mask(P, x, y, z, e.pp, D.walls);
+        has = mask != 0;
+        L = (unsigned)l;
+      }
     }
+    const long long seg = (long long)(e.pp - 1) * D.link_blocks + e.b;
+    part::link_compact(has, L, mask, D.links + seg * kT, D.nlinks + seg, sh);
+  } else if (e.v <= 2) {
+    if (t >= (long long)P.ny * P.nz) return;
+    x = e.v == 1 ? 1 : P.nx - 2; y = (int)(t / P.nz); z = (int)(t % P.nz);
+    const long long L = lin(P, x, y, z);
+    if (D.walls_all[L] != 0) return;
+    const int id = P.par + e.v;
+    bool mine = false, particle = false;
+    for (int i = 1; i < 19; i++) {
+      const long long nb = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
+      const int w = D.walls[nb];
+      if (w == id) { D.pin[nb] = id; mine = true; }
+      particle |= w >= 1 && w <= P.par;
+    }
+    if (mine && !particle) D.pout[L] = id;
+  } else {
+    if (!part::box_node(P, D.bref, D.S->center_old, e.pp, t, x, y, z) || !part::in_range(P, x, y, z)) return;
+    const long long L = lin(P, x, y, z);
+    if (D.walls_old[L] < 1 || D.walls_all[L] != 0) return;
+    int owner = 0;
+    for (int i = 1; i < 19; i++) {
+      const int w =
+          D.walls[lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz))];
+      if (w >= 1 && w <= P.par) owner = max(owner, w);
+    }
+    if (owner != e.pp) return;
+    part::refill_values(P, e.pp, D.S, D.walls_old, D.rho, D.rhoN, D.rhoR, D.rhoB, D.ux, D.uy, D.uz, D.ri, D.bi, D.fi,
+                        x, y, z);
+    refill_import_node<S>(P, D.pd, (S*)D.pops, (R*)D.phic, D.ri, D.bi, D.rhoN, D.rr_old, x, y, z);
   }
-  const long long seg = (long long)(e.pp - 1) * D.link_blocks + e.b;
-  part::link_compact(has, L, mask, D.links + seg * kT, D.nlinks + seg, sh);
 }
 
 // the link lists of particle pp from the current masks (after an import)
@@ -247,41 +304,20 @@ __global__ void __launch_bounds__(kT) k_links_build(DevParams P, part::Box b, in
   part::link_compact(has, L, mask, links + seg * kT, nlinks + seg, sh);
 }
 
-// refilling (uncovered nodes, :1351-1418) and the import of each refilled
-// node into the fused state, by the same thread: a refilled node's import
-// reads only what its own refill wrote, and no refill reads a refilled node
-// (it averages fluid neighbours only), so nodes need no ordering
-template <typename S>
-__global__ void __launch_bounds__(kT) k_sp_refill_import(const SpDom* __restrict__ doms,
-                                                         const Blk* __restrict__ map) {
-  using R = typename Codec<S>::R;
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
-  int x, y, z;
-  if (!part::box_node(D.P, D.bref, D.S->center_old, e.pp, (long long)e.b * kT + threadIdx.x, x, y, z)) return;
-  part::refill_node(D.P, e.pp, D.S, D.pout, D.walls_old, D.rho, D.rhoN, D.rhoR, D.rhoB, D.ux, D.uy, D.uz, D.ri,
-                    D.bi, D.fi, x, y, z);
-  refill_import_node<S>(D.P, D.pd, e.pp, (S*)D.pops, (R*)D.phic, D.pout, D.walls_old, D.ri, D.bi, D.rhoN,
-                        D.rr_old, x, y, z);
-}
-
-// pin fill of the flat walls: v = 0 the plane x = 0, v = 1 the plane x = nx-1
+// pin fill of a particle's solid nodes (v = 0) or of a flat wall (v = 1 the plane
+// x = 0, v = 2 the plane x = nx-1): a fill reads fluid nodes only
 template <typename R>
-__global__ void __launch_bounds__(kT) k_sp_pinfill_plane(const SpDom* __restrict__ doms,
-                                                         const Blk* __restrict__ map) {
+__global__ void __launch_bounds__(kT) k_sp_pinfill(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
   const Blk e = map[blockIdx.x];
   const SpDom& D = doms[e.d];
-  const int t = e.b * kT + threadIdx.x;
-  if (t >= D.P.ny * D.P.nz) return;
-  pinfill_node<R>(D.P, D.pd, (R*)D.phic, D.pin, D.walls_all, e.v == 0 ? 0 : D.P.nx - 1, t / D.P.nz, t % D.P.nz);
-}
-
-template <typename R>
-__global__ void __launch_bounds__(kT) k_sp_pinfill_box(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
-  const Blk e = map[blockIdx.x];
-  const SpDom& D = doms[e.d];
+  const long long t = (long long)e.b * kT + threadIdx.x;
   int x, y, z;
-  if (!part::box_node(D.P, D.bpfill, D.S->center, e.pp, (long long)e.b * kT + threadIdx.x, x, y, z)) return;
+  if (e.v == 0) {
+    if (!part::box_node(D.P, D.bpfill, D.S->center, e.pp, t, x, y, z)) return;
+  } else {
+    if (t >= (long long)D.P.ny * D.P.nz) return;
+    x = e.v == 1 ? 0 : D.P.nx - 1; y = (int)(t / D.P.nz); z = (int)(t % D.P.nz);
+  }
   pinfill_node<R>(D.P, D.pd, (R*)D.phic, D.pin, D.walls_all, x, y, z);
 }
 
@@ -358,15 +394,14 @@ long long nblocks(long long n) { return (n + kT - 1) / kT; }
 struct SparsePlan {
   int storage = -1;
   SpDom* d_dom[2] = {nullptr, nullptr};   // per parity
-  // block tables, one per launch; several launches per particle index keep
-  // the per-particle order of the masks and refills
-  enum { PREP, LAG, CAP, CAPF, MOM, MOMF, RESET, FLAT, PINPLANE, PFPLANE, PFBOX, CURVE2, NFIX };
+  // block tables, one per launch
+  // (MARK: domains of several particles, whose masks are cleared first)
+  enum { PREP, FORCES, MASKS, MARK, PINS, PINFILL, CURVE2, NFIX };
   struct Table {
     Blk* d = nullptr;
     int n = 0;
   };
   Table fix[NFIX];
-  std::vector<Table> mark, pin, refill;   // [particle index - 1]
   int* d_move = nullptr;   // domains with particles
   double* d_ltab = nullptr;   // Lagrange sin/cos tables of every domain with particles
   int nmove = 0;
@@ -401,6 +436,7 @@ SpDom make_dom(sym_handle* h, int cur, int pc) {
   d.lax = h->lax; d.lay = h->lay; d.laz = h->laz; d.larhon = h->larhon;
   d.lanx = h->lanx; d.lany = h->lany; d.lanz = h->lanz; d.lads = h->lads; d.laflag = h->laflag;
   d.red = h->red;
+  d.red_mom = h->red + (size_t)h->dp.par * nblocks(h->dp.la_num) * 7;
   d.pops = popp(h, cur);
   d.phic = phip(h, pc);
   d.phip = phip(h, 1 - pc);
@@ -419,6 +455,7 @@ SpDom make_dom(sym_handle* h, int cur, int pc) {
   d.bref = part::sphere_box(h->dp, 4.0);
   d.bpfill = part::sphere_box(h->dp, 2.0);
   d.nblk_mom = nblocks(d.bmom.count());
+  d.nblk_lag = nblocks(h->dp.la_num);
   d.full_reset = h->dp.par > 1 ? 1 : 0;
   return d;
 }
@@ -431,9 +468,6 @@ void sparse_plan_free(SparsePlan* p) {
     if (p->d_dom[k]) cudaFree(p->d_dom[k]);
   for (auto& t : p->fix)
     if (t.d) cudaFree(t.d);
-  for (auto* v : {&p->mark, &p->pin, &p->refill})
-    for (auto& t : *v)
-      if (t.d) cudaFree(t.d);
   if (p->d_move) cudaFree(p->d_move);
   if (p->d_ltab) cudaFree(p->d_ltab);
   delete p;
@@ -464,52 +498,38 @@ SparsePlan* sparse_plan_build(const std::vector<sym_handle*>& doms, const std::v
   std::vector<Blk> ltb;            // blocks of the one-time Lagrange table launch
   std::vector<long long> ltoff;    // each domain's table offset (doubles), -1 without particles
   long long ltlen = 0;
-  int maxpar = 0;
   std::vector<int> move;
   for (int i = 0; i < n; i++) {
     sym_handle* h = doms[i];
     for (int k = 0; k < 2; k++) dd[k].push_back(make_dom(h, (cur0[i] + k) & 1, (pc0[i] + k) & 1));
     const SpDom& D = dd[0].back();
     const DevParams& P = h->dp;
-    const int plane_blk = (int)nblocks((long long)P.ny * P.nz);
+    auto blocks = [&](int table, long long n, int pp, int v) {
+      for (long long b = 0; b < nblocks(n); b++) tb[table].push_back({i, pp, (int)b, v});
+    };
+    const long long plane = (long long)P.ny * P.nz;
     if (P.wall_x)
-      for (int v = 0; v < 2; v++)
-        for (int b = 0; b < plane_blk; b++) tb[SparsePlan::PFPLANE].push_back({i, 0, b, v});
+      for (int v = 1; v <= 2; v++) blocks(SparsePlan::PINFILL, plane, 0, v);
     ltoff.push_back(P.par > 0 ? ltlen : -1);
     if (P.par <= 0) continue;
     for (long long b = 0; b < nblocks(P.la_num); b++) ltb.push_back({i, 0, (int)b, 0});
     ltlen += 4LL * P.la_num;
-    maxpar = std::max(maxpar, P.par);
     move.push_back(i);
     if (P.wall_x) {
-      for (int b = 0; b < plane_blk; b++) tb[SparsePlan::FLAT].push_back({i, 0, b, 0});
-      for (int v = 0; v < 2; v++)
-        for (int b = 0; b < plane_blk; b++) tb[SparsePlan::PINPLANE].push_back({i, 0, b, v});
+      blocks(SparsePlan::MASKS, 2 * plane, 0, 1);
+      for (int v = 1; v <= 2; v++) blocks(SparsePlan::PINS, plane, 0, v);
     }
-    if (D.full_reset) {
-      for (long long b = 0; b < nblocks(P.N); b++) tb[SparsePlan::RESET].push_back({i, 0, (int)b, 0});
-    } else {
-      for (long long b = 0; b < nblocks(D.bpin.count()); b++) tb[SparsePlan::RESET].push_back({i, 1, (int)b, 0});
-    }
+    if (D.full_reset) blocks(SparsePlan::MASKS, P.N, 0, 3);
+    else blocks(SparsePlan::MASKS, D.bpin.count(), 1, 0);
     for (int pp = 1; pp <= P.par; pp++) {
-      for (long long b = 0; b < nblocks(D.bprep.count()); b++) tb[SparsePlan::PREP].push_back({i, pp, (int)b, 0});
-      for (long long b = 0; b < nblocks(P.la_num); b++) tb[SparsePlan::LAG].push_back({i, pp, (int)b, 0});
-      for (int b = 0; b < part::kCapBlocks; b++) tb[SparsePlan::CAP].push_back({i, pp, b, 0});
-      tb[SparsePlan::CAPF].push_back({i, pp, 0, 0});
-      for (long long b = 0; b < D.nblk_mom; b++) tb[SparsePlan::MOM].push_back({i, pp, (int)b, 0});
-      tb[SparsePlan::MOMF].push_back({i, pp, 0, 0});
-      for (long long b = 0; b < nblocks(D.bpfill.count()); b++) tb[SparsePlan::PFBOX].push_back({i, pp, (int)b, 0});
-      if (P.bounce)
-        for (long long b = 0; b < nblocks(D.bmom.count()); b++) tb[SparsePlan::CURVE2].push_back({i, pp, (int)b, 0});
-    }
-  }
-  std::vector<std::vector<Blk>> mk(maxpar), pn(maxpar), rf(maxpar);
-  for (int i = 0; i < n; i++) {
-    const SpDom& D = dd[0][i];
-    for (int pp = 1; pp <= doms[i]->dp.par; pp++) {
-      for (long long b = 0; b < nblocks(D.bmark.count()); b++) mk[pp - 1].push_back({i, pp, (int)b, 0});
-      for (long long b = 0; b < nblocks(D.bpin.count()); b++) pn[pp - 1].push_back({i, pp, (int)b, 0});
-      for (long long b = 0; b < nblocks(D.bref.count()); b++) rf[pp - 1].push_back({i, pp, (int)b, 0});
+      blocks(SparsePlan::PREP, D.bprep.count(), pp, 0);
+      blocks(SparsePlan::FORCES, P.la_num, pp, 0);
+      blocks(SparsePlan::FORCES, D.bmom.count(), pp, 1);
+      blocks(D.full_reset ? SparsePlan::MARK : SparsePlan::MASKS, D.bmark.count(), pp, 2);
+      blocks(SparsePlan::PINS, D.bpin.count(), pp, 0);
+      blocks(SparsePlan::PINS, D.bref.count(), pp, 3);
+      blocks(SparsePlan::PINFILL, D.bpfill.count(), pp, 0);
+      if (P.bounce) blocks(SparsePlan::CURVE2, D.bmom.count(), pp, 0);
     }
   }
   int e = SYM_OK;
@@ -532,14 +552,6 @@ SparsePlan* sparse_plan_build(const std::vector<sym_handle*>& doms, const std::v
     cudaMemcpyAsync(p->d_dom[k], dd[k].data(), sizeof(SpDom) * n, cudaMemcpyHostToDevice, st);
   }
   for (int t = 0; t < SparsePlan::NFIX && !e; t++) e = plan_table(p->fix[t], tb[t], st);
-  p->mark.resize(maxpar);
-  p->pin.resize(maxpar);
-  p->refill.resize(maxpar);
-  for (int q = 0; q < maxpar && !e; q++) {
-    e = plan_table(p->mark[q], mk[q], st);
-    if (!e) e = plan_table(p->pin[q], pn[q], st);
-    if (!e) e = plan_table(p->refill[q], rf[q], st);
-  }
   if (!e && !move.empty()) {
     p->nmove = (int)move.size();
     if (cudaMalloc(&p->d_move, sizeof(int) * move.size()) != cudaSuccess) {
@@ -564,8 +576,6 @@ SparsePlan* sparse_plan_build(const std::vector<sym_handle*>& doms, const std::v
   // launches per step
   int l = 0;
   for (auto& t : p->fix) l += t.n ? 1 : 0;
-  for (auto* v : {&p->mark, &p->pin, &p->refill})
-    for (auto& t : *v) l += t.n ? 1 : 0;
   l += p->nmove ? 1 : 0;
   p->launches = l;
   return p;
@@ -581,20 +591,12 @@ void enqueue_plan(SparsePlan* p, int k, cudaStream_t st) {
     if (t.n) kern<<<t.n, threads, 0, st>>>(D, t.d);
   };
   go(k_sp_prep<S>, f[SparsePlan::PREP]);
-  go(k_sp_lagrange, f[SparsePlan::LAG]);
-  go(k_sp_capillary, f[SparsePlan::CAP]);
-  go(k_sp_capillary_final, f[SparsePlan::CAPF], 32);
-  go(k_sp_momentum, f[SparsePlan::MOM]);
-  go(k_sp_momentum_final, f[SparsePlan::MOMF]);
-  if (p->nmove) k_sp_move<<<p->nmove, SYM_MAX_PAR, 0, st>>>(D, p->d_move);
-  go(k_sp_reset, f[SparsePlan::RESET]);
-  go(k_sp_flat, f[SparsePlan::FLAT]);
-  for (auto& t : p->mark) go(k_sp_mark, t);
-  go(k_sp_pin_plane, f[SparsePlan::PINPLANE]);
-  for (auto& t : p->pin) go(k_sp_pin_box, t);
-  for (auto& t : p->refill) go(k_sp_refill_import<S>, t);
-  go(k_sp_pinfill_plane<R>, f[SparsePlan::PFPLANE]);
-  go(k_sp_pinfill_box<R>, f[SparsePlan::PFBOX]);
+  go(k_sp_forces, f[SparsePlan::FORCES]);
+  if (p->nmove) k_sp_move<<<p->nmove, kT, 0, st>>>(D, p->d_move);
+  go(k_sp_masks, f[SparsePlan::MASKS]);
+  go(k_sp_masks, f[SparsePlan::MARK]);
+  go(k_sp_pins<S>, f[SparsePlan::PINS]);
+  go(k_sp_pinfill<R>, f[SparsePlan::PINFILL]);
 }
 }  // namespace
 
