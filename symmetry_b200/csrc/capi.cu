@@ -227,18 +227,16 @@ int canonical_piece(sym_handle* h, int piece) {
   int e;
   if ((e = ref_step_macros(h, piece == MID || piece == TAIL, last))) return e;
   if (h->p.par > 0) {
-    if ((e = part_lagrange_points(h))) return e;
-    if ((e = part_capillary_force2(h))) return e;
+    if ((e = part_lagrange_capillary(h))) return e;
     if ((e = part_momentum(h))) return e;
-    if ((e = part_repulsive(h))) return e;
-    if ((e = part_movement(h))) return e;
+    if ((e = part_repulsive_movement(h))) return e;
   }
   if ((e = part_set_walls(h))) return e;
   if (h->p.par > 0)
     if ((e = part_refilling(h, !last))) return e;
-  if ((e = ref_derivatives(h))) return e;
+  if ((e = ref_derivatives(h, !last))) return e;
   if ((e = ref_collide_recolor(h, last))) return e;
-  if ((e = ref_boundary(h))) return e;
+  if ((e = ref_boundary(h, last))) return e;
   if (!last) return SYM_OK;
   if ((e = ref_stream_both(h))) return e;
   return ref_curve(h);

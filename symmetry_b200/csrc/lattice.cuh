@@ -382,4 +382,26 @@ __device__ __forceinline__ void wall_normal_dev(const PT& P, const sym_particles
   }
 }
 
+// f(L, fx, fy, fz) for every mirror image of interior node (x, y, z) on the mirror
+// planes (fx: mirrored in x, ...), and with `walls` also for its copies on the
+// wall planes x = 0 and z = 0: what a node's own kernel writes there needs no
+// pass over the planes (on z planes, whose nodes lie a row apart, that is one
+// sector per value; here it is the neighbour of the row's own write).
+template <typename F>
+__device__ __forceinline__ void for_images(const DevParams& P, int x, int y, int z, bool walls, F&& f) {
+  const bool edge = x == P.nx - 2 || y == 1 || y == P.ny - 2 || z == P.nz - 2 || (walls && (x == 1 || z == 1));
+  if (!edge) return;
+  int xs[3] = {x, 0, 0}, ys[3] = {y, 0, 0}, zs[3] = {z, 0, 0}, nx = 1, ny = 1, nz = 1;
+  if (x == P.nx - 2) xs[nx++] = P.nx - 1;
+  if (walls && x == 1) xs[nx++] = 0;
+  if (y == 1) ys[ny++] = 0;
+  if (y == P.ny - 2) ys[ny++] = P.ny - 1;
+  if (z == P.nz - 2) zs[nz++] = P.nz - 1;
+  if (walls && z == 1) zs[nz++] = 0;
+  for (int a = 0; a < nx; a++)
+    for (int b = 0; b < ny; b++)
+      for (int c = 0; c < nz; c++)
+        if (a | b | c) f(lin(P, xs[a], ys[b], zs[c]), xs[a] == P.nx - 1, b > 0, zs[c] == P.nz - 1);
+}
+
 }  // namespace symb200

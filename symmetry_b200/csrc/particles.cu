@@ -9,7 +9,6 @@ namespace symb200 {
 
 void mirror_masks(sym_handle* h);
 void mirror_macros_all(sym_handle* h);
-void mirror_phi(sym_handle* h);
 
 namespace {
 
@@ -102,6 +101,11 @@ __global__ void k_momentum_final(DevParams P, sym_particles* S, const double* pa
 __global__ void k_repulsive(DevParams P, sym_particles* S) {   // one thread per particle
   if ((int)threadIdx.x < P.par) repulsive_one(P, S, threadIdx.x + 1);
 }
+__global__ void k_repulsive_movement(DevParams P, sym_particles* S) {
+  if ((int)threadIdx.x < P.par) repulsive_one(P, S, threadIdx.x + 1);
+  __syncwarp();
+  if ((int)threadIdx.x < P.par) movement_one(P, S, threadIdx.x + 1);
+}
 __global__ void k_movement(DevParams P, sym_particles* S) {
   if ((int)threadIdx.x < P.par) movement_one(P, S, threadIdx.x + 1);
 }
@@ -112,11 +116,16 @@ __global__ void k_movement(DevParams P, sym_particles* S) {
 __global__ void k_refill(DevParams P, Box b, const sym_particles* __restrict__ S,
                          const int32_t* __restrict__ pout, const int32_t* __restrict__ walls_old, double* rho,
                          double* rhoN, double* rhoR, double* rhoB, double* ux, double* uy, double* uz, double* ri,
-                         double* bi, double* fi) {
+                         double* bi, double* fi, bool images) {
   int x, y, z;
   const int pp = blockIdx.y + 1;
   if (!box_node(P, b, S->center_old, pp, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
   refill_node(P, pp, S, pout, walls_old, rho, rhoN, rhoR, rhoB, ux, uy, uz, ri, bi, fi, x, y, z);
+  if (!images || !in_range(P, x, y, z)) return;
+  const long long L = lin(P, x, y, z);
+  if (pout[L] != pp || walls_old[L] < 1) return;
+  const double phi = rhoN[L];
+  for_images(P, x, y, z, false, [&](long long Li, bool, bool, bool) { rhoN[Li] = phi; });
 }
 
 // ---- initia_center (Source1.f90:926-976), REFERENCE geometry ----------------------
@@ -194,6 +203,26 @@ int part_capillary_force2(sym_handle* h) {
   return check_cuda(h, cudaGetLastError(), "capillary_force2");
 }
 
+// Lagrange_points and capillary_force2 with one pass for area, force and torque;
+// repulsive and movement in one launch (inside a step)
+int part_lagrange_capillary(sym_handle* h) {
+  const DevParams& P = h->dp;
+  if (P.par == 0) return SYM_OK;
+  dim3 g(blocks_for(P.la_num, 128), P.par);
+  k_lagrange<<<g, 128, 0, h->st>>>(P, h->dpart, h->walls, h->rhoN, h->gx, h->gy, h->gz, h->nx, h->ny, h->nz, h->lax,
+                                   h->lay, h->laz, h->larhon, h->lanx, h->lany, h->lanz, h->laflag, h->lads);
+  if ((size_t)kCapBlocks * 7 * P.par > h->red_len) return set_error(h, SYM_ERR_STATE, "capillary scratch too small");
+  k_capillary<<<dim3(kCapBlocks, P.par), 256, 0, h->st>>>(P, h->dpart, h->lax, h->lay, h->laz, h->larhon, h->lanx,
+                                                           h->lany, h->lanz, h->laflag, h->lads, 1, h->red);
+  k_capillary_final<<<P.par, 32, 0, h->st>>>(P, h->dpart, h->red, 1, 1);
+  return check_cuda(h, cudaGetLastError(), "Lagrange points and capillary force");
+}
+int part_repulsive_movement(sym_handle* h) {
+  if (h->dp.par == 0) return SYM_OK;
+  k_repulsive_movement<<<1, SYM_MAX_PAR, 0, h->st>>>(h->dp, h->dpart);
+  return check_cuda(h, cudaGetLastError(), "repulsion and movement");
+}
+
 int part_momentum(sym_handle* h) {
   const DevParams& P = h->dp;
   if (P.par == 0) return SYM_OK;
@@ -218,16 +247,16 @@ int part_movement(sym_handle* h) {
   return check_cuda(h, cudaGetLastError(), "movement");
 }
 
-// phi_only: only rho_N goes onto the mirror planes (inside a run of steps)
-int part_refilling(sym_handle* h, bool phi_only) {
+// in_run: only rho_N of the refilled nodes goes onto the mirror planes (a later
+// step of the same run writes the rest)
+int part_refilling(sym_handle* h, bool in_run) {
   const DevParams& P = h->dp;
   if (P.par == 0) return SYM_OK;
   const Box b = sphere_box(h, 4.0);
   k_refill<<<dim3(blocks_for(b.count()), P.par), TPB, 0, h->st>>>(P, b, h->dpart, h->pout, h->walls_old, h->rho,
                                                                   h->rhoN, h->rhoR, h->rhoB, h->ux, h->uy, h->uz,
-                                                                  h->ri, h->bi, h->fi);
-  if (P.ref && phi_only) mirror_phi(h);
-  else if (P.ref) mirror_macros_all(h);
+                                                                  h->ri, h->bi, h->fi, P.ref && in_run);
+  if (P.ref && !in_run) mirror_macros_all(h);
   return check_cuda(h, cudaGetLastError(), "refilling");
 }
 

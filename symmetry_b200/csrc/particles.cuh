@@ -48,10 +48,10 @@ __device__ __forceinline__ bool box_node(const DevParams& P, const Box& b, const
                                          long long t, int& x, int& y, int& z) {
   if (t >= b.count()) return false;
   int id[3];
-  id[2] = (int)(t % b.n[2]);
-  t /= b.n[2];
-  id[1] = (int)(t % b.n[1]);
-  id[0] = (int)(t / b.n[1]);
+  const unsigned u = (unsigned)t, q = u / (unsigned)b.n[2], r = q / (unsigned)b.n[1];   // (count < 2^32: inside a domain)
+  id[2] = (int)(u - q * (unsigned)b.n[2]);
+  id[1] = (int)(q - r * (unsigned)b.n[1]);
+  id[0] = (int)r;
   const int dims[3] = {P.nx, P.ny, P.nz};
   int v[3];
   for (int k = 0; k < 3; k++) {
@@ -378,16 +378,29 @@ __device__ __forceinline__ void momentum_partial(const DevParams& P, const Box& 
       const double uw0 = PC(S->up, par, pp, 0) + zr * PC(S->rp, par, pp, 1) - yr * PC(S->rp, par, pp, 2);
       const double uw1 = PC(S->up, par, pp, 1) + xr * PC(S->rp, par, pp, 2) - zr * PC(S->rp, par, pp, 0);
       const double uw2 = PC(S->up, par, pp, 2) + yr * PC(S->rp, par, pp, 0) - xr * PC(S->rp, par, pp, 1);
+      // the neighbours' masks, then the populations of the links, are read
+      // together, not one link after another
+      bool link[19];
+      double f[19], g[19];
+#pragma unroll
       for (int i = 1; i < 19; i++) {
         const int xb = P.ref ? x - CX(i) : wrapi(x - CX(i), P.nx);
         const int yb = P.ref ? y - CY(i) : wrapi(y - CY(i), P.ny);
         const int zb = P.ref ? z - CZ(i) : wrapi(z - CZ(i), P.nz);
-        if (walls[lin(P, xb, yb, zb)] != pp) continue;
+        link[i] = walls[lin(P, xb, yb, zb)] == pp;
+      }
+#pragma unroll
+      for (int i = 1; i < 19; i++) {
+        f[i] = link[i] ? fi[i * N + L] : 0.0;
+        g[i] = link[i] ? ffi[OPC(i) * N + L] : 0.0;
+      }
+#pragma unroll
+      for (int i = 1; i < 19; i++) {
+        if (!link[i]) continue;
         const int j = OPC(i);
-        const double f = fi[i * N + L], g = ffi[j * N + L];
-        const double fmx = ((double)CX(i) - uw0) * f - ((double)CX(j) - uw0) * g;
-        const double fmy = ((double)CY(i) - uw1) * f - ((double)CY(j) - uw1) * g;
-        const double fmz = ((double)CZ(i) - uw2) * f - ((double)CZ(j) - uw2) * g;
+        const double fmx = ((double)CX(i) - uw0) * f[i] - ((double)CX(j) - uw0) * g[i];
+        const double fmy = ((double)CY(i) - uw1) * f[i] - ((double)CY(j) - uw1) * g[i];
+        const double fmz = ((double)CZ(i) - uw2) * f[i] - ((double)CZ(j) - uw2) * g[i];
         a[0] = a[0] - fmx; a[1] = a[1] - fmy; a[2] = a[2] - fmz;
         a[3] = a[3] - (yr * fmz - zr * fmy);
         a[4] = a[4] - (zr * fmx - xr * fmz);
@@ -571,61 +584,72 @@ __device__ __forceinline__ void repulsive_one(const DevParams& P, sym_particles*
 }
 
 // ---- movement (Source1.f90:1263-1349) of particle pp, after every particle's
-// repulsive_one -------------------------------------------------------------------
+// repulsive_one; its state is read and written once (changed in place, the chain
+// of memory round trips was the kernel's 12 us) -------------------------------------
 __device__ __forceinline__ void movement_one(const DevParams& P, sym_particles* S, int pp) {
   const int par = P.par;
-  auto A = [&](double* a, int pp, int k) -> double& { return a[k * par + pp - 1]; };
+  double c0[3], c[3], up[3], rp[3], fp[3], tp[3], fre[3], ten[3], tent[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int q = k * par + pp - 1;
+    c0[k] = S->center0[q]; c[k] = S->center[q];
+    up[k] = S->up[q]; rp[k] = S->rp[q];
+    fp[k] = S->fp[q]; tp[k] = S->tp[q]; fre[k] = S->fre[q];
+    ten[k] = S->tension[q]; tent[k] = S->tension_t[q];
+  }
   if (P.ref) {
-    {
-      if (fabs(A(S->center0, pp, 0) - ((double)P.nx - 0.5)) < 0.1) {
-        A(S->fp, pp, 0) = 0.0; A(S->fp, pp, 1) = 2.0 * A(S->fp, pp, 1); A(S->fp, pp, 2) = 2.0 * A(S->fp, pp, 2);
-        A(S->tp, pp, 0) = 2.0 * A(S->tp, pp, 0); A(S->tp, pp, 1) = 0.0; A(S->tp, pp, 2) = 0.0;
-        A(S->fre, pp, 0) = 0.0;
-        A(S->tension, pp, 0) = 0.0; A(S->tension, pp, 1) = A(S->tension, pp, 1) * 2.0;
-        A(S->tension, pp, 2) = A(S->tension, pp, 2) * 2.0;
-        A(S->tension_t, pp, 0) = 2.0 * A(S->tension_t, pp, 0);
-        A(S->tension_t, pp, 1) = 0.0; A(S->tension_t, pp, 2) = 0.0;
+    // a particle that started on a mirror plane: the force along the plane's
+    // normal and the torques along the plane vanish, the others double
+    auto mirrored = [&](int axis) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        if (k == axis) {
+          fp[k] = 0.0; ten[k] = 0.0; fre[k] = 0.0;
+        } else {
+          fp[k] = 2.0 * fp[k];
+          ten[k] = ten[k] * 2.0;
+        }
       }
-      const double c0y = A(S->center0, pp, 1);
-      if (fabs(c0y - ((double)P.ny - 0.5)) < 0.1 || fabs(c0y - 1.5) < 0.1) {
-        A(S->fp, pp, 0) = 2.0 * A(S->fp, pp, 0); A(S->fp, pp, 1) = 0.0; A(S->fp, pp, 2) = 2.0 * A(S->fp, pp, 2);
-        A(S->tp, pp, 0) = 0.0; A(S->tp, pp, 1) = 2.0 * A(S->tp, pp, 1); A(S->tp, pp, 2) = 0.0;
-        A(S->fre, pp, 1) = 0.0;
-        A(S->tension, pp, 0) = 2.0 * A(S->tension, pp, 0); A(S->tension, pp, 1) = 0.0;
-        A(S->tension, pp, 2) = 2.0 * A(S->tension, pp, 2);
-        A(S->tension_t, pp, 0) = 0.0; A(S->tension_t, pp, 1) = 0.0; A(S->tension_t, pp, 2) = 0.0;
-      }
-      if (fabs(A(S->center0, pp, 2) - ((double)P.nz - 0.5)) < 0.1) {
-        A(S->fp, pp, 0) = 2.0 * A(S->fp, pp, 0); A(S->fp, pp, 1) = 2.0 * A(S->fp, pp, 1); A(S->fp, pp, 2) = 0.0;
-        A(S->tp, pp, 0) = 0.0; A(S->tp, pp, 1) = 0.0; A(S->tp, pp, 2) = 2.0 * A(S->tp, pp, 2);
-        A(S->fre, pp, 2) = 0.0;
-        A(S->tension, pp, 0) = A(S->tension, pp, 0) * 2.0; A(S->tension, pp, 1) = A(S->tension, pp, 1) * 2.0;
-        A(S->tension, pp, 2) = 0.0;
-        A(S->tension_t, pp, 0) = 0.0; A(S->tension_t, pp, 1) = 0.0;
-        A(S->tension_t, pp, 2) = 2.0 * A(S->tension_t, pp, 2);
-      }
+    };
+    if (fabs(c0[0] - ((double)P.nx - 0.5)) < 0.1) {
+      mirrored(0);
+      tp[0] = 2.0 * tp[0]; tp[1] = 0.0; tp[2] = 0.0;
+      tent[0] = 2.0 * tent[0]; tent[1] = 0.0; tent[2] = 0.0;
     }
-    {
-      if (pp == par / 3 + 1) {
-        double t = (A(S->tension, pp, 0) + A(S->tension, pp, 2)) / 2.0;
-        A(S->tension, pp, 0) = t; A(S->tension, pp, 2) = t;
-        A(S->tension_t, pp, 1) = 0.0;
-        t = (A(S->fp, pp, 0) + A(S->fp, pp, 2)) / 2.0;
-        A(S->fp, pp, 0) = t; A(S->fp, pp, 2) = t;
-        A(S->tp, pp, 1) = 0.0;
-        t = (A(S->fre, pp, 0) + A(S->fre, pp, 2)) / 2.0;
-        A(S->fre, pp, 0) = t; A(S->fre, pp, 2) = t;
-      }
+    if (fabs(c0[1] - ((double)P.ny - 0.5)) < 0.1 || fabs(c0[1] - 1.5) < 0.1) {
+      mirrored(1);
+      tp[0] = 0.0; tp[1] = 2.0 * tp[1]; tp[2] = 0.0;
+      tent[0] = 0.0; tent[1] = 0.0; tent[2] = 0.0;
+    }
+    if (fabs(c0[2] - ((double)P.nz - 0.5)) < 0.1) {
+      mirrored(2);
+      tp[0] = 0.0; tp[1] = 0.0; tp[2] = 2.0 * tp[2];
+      tent[0] = 0.0; tent[1] = 0.0; tent[2] = 2.0 * tent[2];
+    }
+    if (pp == par / 3 + 1) {
+      double t = (ten[0] + ten[2]) / 2.0;
+      ten[0] = t; ten[2] = t;
+      tent[1] = 0.0;
+      t = (fp[0] + fp[2]) / 2.0;
+      fp[0] = t; fp[2] = t;
+      tp[1] = 0.0;
+      t = (fre[0] + fre[2]) / 2.0;
+      fre[0] = t; fre[2] = t;
     }
   }
   const double m = P.mass, I = P.inertia;
-  for (int c = 0; c < 3; c++) {
-    double f = A(S->fp, pp, c) + A(S->fre, pp, c) + A(S->tension, pp, c);
-    if (!P.ref) f = f + m * P.body[c];
-    A(S->up, pp, c) = A(S->up, pp, c) + f / m;
-    A(S->rp, pp, c) = A(S->rp, pp, c) + (A(S->tp, pp, c) + A(S->tension_t, pp, c)) / I;
-    A(S->center_old, pp, c) = A(S->center, pp, c);
-    A(S->center, pp, c) = A(S->center, pp, c) + A(S->up, pp, c) + 0.5 * f / m;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int q = k * par + pp - 1;
+    double f = fp[k] + fre[k] + ten[k];
+    if (!P.ref) f = f + m * P.body[k];
+    up[k] = up[k] + f / m;
+    S->up[q] = up[k];
+    S->rp[q] = rp[k] + (tp[k] + tent[k]) / I;
+    S->center_old[q] = c[k];
+    S->center[q] = c[k] + up[k] + 0.5 * f / m;
+    S->fp[q] = fp[k]; S->tp[q] = tp[k]; S->fre[q] = fre[k];
+    S->tension[q] = ten[k]; S->tension_t[q] = tent[k];
   }
 }
 

@@ -21,13 +21,13 @@ inline unsigned blocks_for(long long n, int tpb = TPB) { return (unsigned)((n + 
 
 // thread t -> node of the update range (z fastest)
 __device__ __forceinline__ bool range_node(const DevParams& P, long long t, int& x, int& y, int& z) {
-  const int rx = P.hi[0] - P.lo[0] + 1, ry = P.hi[1] - P.lo[1] + 1, rz = P.hi[2] - P.lo[2] + 1;
-  if (t >= (long long)rx * ry * rz) return false;
-  z = P.lo[2] + (int)(t % rz);
-  t /= rz;
-  y = P.lo[1] + (int)(t % ry);
-  x = P.lo[0] + (int)(t / ry);
-  return true;
+  // (32-bit arithmetic: a domain has at most 4e9 nodes)
+  const unsigned ry = P.hi[1] - P.lo[1] + 1, rz = P.hi[2] - P.lo[2] + 1;
+  const unsigned u = (unsigned)t, q = u / rz, r = q / ry;
+  z = P.lo[2] + (int)(u - q * rz);
+  y = P.lo[1] + (int)(q - r * ry);
+  x = P.lo[0] + (int)r;
+  return t <= 0xffffffffLL && x <= P.hi[0];
 }
 inline long long range_count(const DevParams& P) {
   return (long long)(P.hi[0] - P.lo[0] + 1) * (P.hi[1] - P.lo[1] + 1) * (P.hi[2] - P.lo[2] + 1);
@@ -111,14 +111,30 @@ __global__ void __launch_bounds__(TPB) k_mirror(DevParams P, MirrorSet S) {
   if (S.low) S.low[Ld] = S.low[lin(P, m.x == 0 ? 1 : m.x, m.y, m.z == 0 ? 1 : m.z)];
   if (!(m.fx || m.fy || m.fz)) return;
   const long long Ls = lin(P, m.x, m.y, m.z);
-  for (int k = 0; k < S.ns; k++) S.scalar[k][Ld] = S.scalar[k][Ls];
-  for (int k = 0; k < S.nm; k++) S.mask[k][Ld] = S.mask[k][Ls];
-  for (int k = 0; k < S.nv; k++) {
-    const double a = S.vec[k][0][Ls], b = S.vec[k][1][Ls], c = S.vec[k][2][Ls];
-    S.vec[k][0][Ld] = m.fx ? -a : a;
-    S.vec[k][1][Ld] = m.fy ? -b : b;
-    S.vec[k][2][Ld] = m.fz ? -c : c;
+  // every array's value is read before the first is written (the planes of z are
+  // one sector per value: latency, not bandwidth)
+  double v[4 + 6];
+  int32_t k4[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (k < S.ns) v[k] = S.scalar[k][Ls];
+    if (k < S.nm) k4[k] = S.mask[k][Ls];
   }
+#pragma unroll
+  for (int k = 0; k < 6; k++)
+    if (k / 3 < S.nv) v[4 + k] = S.vec[k / 3][k % 3][Ls];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (k < S.ns) S.scalar[k][Ld] = v[k];
+    if (k < S.nm) S.mask[k][Ld] = k4[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 6; k++)
+    if (k / 3 < S.nv) {
+      const bool flip = k % 3 == 0 ? m.fx : (k % 3 == 1 ? m.fy : m.fz);
+      S.vec[k / 3][k % 3][Ld] = flip ? -v[4 + k] : v[4 + k];
+    }
+#pragma unroll 1
   for (int k = 0; k < S.np; k++) {
     double* const f = S.pop[k];
     double tmp[19];
@@ -188,21 +204,40 @@ void mirror_colours(sym_handle* h) {
 }
 
 // ---- derivatives (Source1.f90:452-597) ------------------------------------
-__global__ void k_pin_fill(DevParams P, const int32_t* __restrict__ pin, const int32_t* __restrict__ walls_all,
-                           double* rhoN) {
-  int x, y, z;
-  if (!range_node(P, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
-  const long long L = lin(P, x, y, z);
-  if (pin[L] <= 0) return;
-  double ws = 0.0, v = 0.0;
-#pragma unroll
-  for (int i = 1; i < 19; i++) {
-    const long long nb = nbr(P, x, y, z, i);
-    if (walls_all[nb] <= 0) { ws = ws + W(i); v = v + W(i) * rhoN[nb]; }
+// images: the filled node's images on the mirror planes too.  Four nodes per
+// thread: nearly all of them only read their mask (152^3: 22 us with one, bound
+// by the launch of 13,000 blocks)
+__global__ void __launch_bounds__(TPB) k_pin_fill(DevParams P, const int32_t* __restrict__ pin,
+                                                  const int32_t* __restrict__ walls_all, double* rhoN, bool images) {
+  const long long L0 = 4 * (blockIdx.x * (long long)TPB + threadIdx.x);
+  int p[4] = {0, 0, 0, 0};
+  if (L0 + 4 <= P.N) {   // (pin starts on a 256-byte boundary)
+    const int4 v = *reinterpret_cast<const int4*>(pin + L0);
+    p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w;
+  } else {
+    for (int k = 0; k < 4; k++)
+      if (L0 + k < P.N) p[k] = pin[L0 + k];
   }
-  rhoN[L] = v / ws;
+#pragma unroll 1
+  for (int k = 0; k < 4; k++) {
+    if (p[k] <= 0) continue;
+    const long long L = L0 + k;
+    const unsigned Lu = (unsigned)L, q = Lu / (unsigned)P.nz;
+    const int z = (int)(Lu - q * (unsigned)P.nz), x = (int)(q / (unsigned)P.ny), y = (int)(q - (unsigned)x * P.ny);
+    if (x < P.lo[0] || x > P.hi[0] || y < P.lo[1] || y > P.hi[1] || z < P.lo[2] || z > P.hi[2]) continue;
+    double ws = 0.0, v = 0.0;
+#pragma unroll
+    for (int i = 1; i < 19; i++) {
+      const long long nb = nbr(P, x, y, z, i);
+      if (walls_all[nb] <= 0) { ws = ws + W(i); v = v + W(i) * rhoN[nb]; }
+    }
+    rhoN[L] = v / ws;
+    if (images) for_images(P, x, y, z, false, [&](long long Li, bool, bool, bool) { rhoN[Li] = v / ws; });
+  }
 }
 
+// REF: no neighbour of an updated node is across a periodic face
+template <bool REF>
 __global__ void k_gradient(DevParams P, const sym_particles* __restrict__ S, const int32_t* __restrict__ pout,
                            const int32_t* __restrict__ walls_all, const double* __restrict__ rhoN, double* gx, double* gy, double* gz, double* nx, double* ny, double* nz, int32_t* flag) {
   int x, y, z;
@@ -213,7 +248,7 @@ __global__ void k_gradient(DevParams P, const sym_particles* __restrict__ S, con
   if (walls_all[L] <= 0) {
 #pragma unroll
     for (int i = 1; i < 19; i++) {
-      const double val = W(i) * rhoN[nbr(P, x, y, z, i)];
+      const double val = W(i) * rhoN[REF ? L + CZ(i) + P.nz * (CY(i) + (long long)P.ny * CX(i)) : nbr(P, x, y, z, i)];
       if (CX(i)) g0 = g0 + val * (double)CX(i);
       if (CY(i)) g1 = g1 + val * (double)CY(i);
       if (CZ(i)) g2 = g2 + val * (double)CZ(i);
@@ -233,6 +268,11 @@ __global__ void k_gradient(DevParams P, const sym_particles* __restrict__ S, con
     g0 = fnorm * v[0]; g1 = fnorm * v[1]; g2 = fnorm * v[2];
   }
   gx[L] = g0; gy[L] = g1; gz[L] = g2; nx[L] = n0; ny[L] = n1; nz[L] = n2; flag[L] = fl;
+  if (REF)
+    for_images(P, x, y, z, false, [&](long long Li, bool fx, bool fy, bool fz) {
+      gx[Li] = fx ? -g0 : g0; gy[Li] = fy ? -g1 : g1; gz[Li] = fz ? -g2 : g2;
+      nx[Li] = fx ? -n0 : n0; ny[Li] = fy ? -n1 : n1; nz[Li] = fz ? -n2 : n2;
+    });
 }
 
 // ---- collision (Source1.f90:599-695) --------------------------------------
@@ -318,6 +358,14 @@ __global__ void k_recolor(DevParams P, const int32_t* __restrict__ walls_all, co
 // opc(i) of the wall node it enters.  One thread per boundary node gathers its
 // new populations; the reads go to nodes off the mirror planes, and on the wall
 // planes only to velocities that no thread writes.
+// FULL: every velocity of every boundary node.  Otherwise (inside a run of
+// steps) a node on mirror planes only gets the velocities that enter the domain;
+// those that leave it or run along the planes reach no interior node, and the
+// run's last step writes them all.  Nodes of the wall planes, whose populations
+// along the walls a run carries from step to step, get all of theirs, and
+// (1,0,-1) of the plane x = nx-1 wraps to the row beside both walls, where no
+// bounce-back replaces it.
+template <bool FULL>
 __global__ void __launch_bounds__(TPB) k_boundary(DevParams P, double* ri, double* bi) {
   int x, y, z;
   if (!plane_node(P, blockIdx.x * TPB + threadIdx.x, true, x, y, z)) return;
@@ -325,6 +373,11 @@ __global__ void __launch_bounds__(TPB) k_boundary(DevParams P, double* ri, doubl
   const Image own = image_of(P, x, y, z);
   const bool mirrored = own.fx || own.fy || own.fz;
   const long long Lo = lin(P, own.x, own.y, own.z);
+  const bool all = FULL || x == 0 || z == 0;
+  auto enters = [&](int cx, int cy, int cz) {
+    return (x == P.nx - 1 && (cx < 0 || (cx > 0 && cy == 0 && cz < 0))) || (y == 0 && cy > 0) ||
+           (y == P.ny - 1 && cy < 0) || (z == P.nz - 1 && cz < 0);
+  };
   double tr[19], tb[19];
 #pragma unroll
   for (int i = 0; i < 19; i++) {
@@ -336,7 +389,7 @@ __global__ void __launch_bounds__(TPB) k_boundary(DevParams P, double* ri, doubl
       const long long q = m.dir(-CX(i), -CY(i), -CZ(i)) * N + lin(P, m.x, m.y, m.z);
       tr[i] = ri[q];
       tb[i] = bi[q];
-    } else if (mirrored) {
+    } else if (mirrored && (all || enters(CX(i), CY(i), CZ(i)))) {
       const long long q = own.dir(CX(i), CY(i), CZ(i)) * N + Lo;
       tr[i] = ri[q];
       tb[i] = bi[q];
@@ -345,7 +398,7 @@ __global__ void __launch_bounds__(TPB) k_boundary(DevParams P, double* ri, doubl
 #pragma unroll
   for (int i = 0; i < 19; i++) {
     const bool back = x == 0 && CX(i) > 0 && !(i == 13 && z == 1);
-    if ((z == 0 && CZ(i) > 0) || back || mirrored) {
+    if ((z == 0 && CZ(i) > 0) || back || (mirrored && (all || enters(CX(i), CY(i), CZ(i))))) {
       ri[i * N + Ld] = tr[i];
       bi[i * N + Ld] = tb[i];
     }
@@ -378,13 +431,21 @@ __global__ void k_curve(DevParams P, const sym_particles* __restrict__ S, const 
   const int pp = pout[L];
   if (pp < 1) return;
   const int par = P.par;
-#pragma unroll 1
+  // the neighbours' masks are read together, not one per link
+  int wbs[19];
+  long long Bs[19];
+#pragma unroll
   for (int i = 1; i < 19; i++) {
     const int xb = P.ref ? x - CX(i) : wrapi(x - CX(i), P.nx);
     const int yb = P.ref ? y - CY(i) : wrapi(y - CY(i), P.ny);
     const int zb = P.ref ? z - CZ(i) : wrapi(z - CZ(i), P.nz);
-    const long long B = lin(P, xb, yb, zb);
-    const int wb = walls[B];
+    Bs[i] = lin(P, xb, yb, zb);
+    wbs[i] = walls[Bs[i]];
+  }
+#pragma unroll
+  for (int i = 1; i < 19; i++) {
+    const long long B = Bs[i];
+    const int wb = wbs[i];
     const bool flat = !P.ref && wb > par;
     if (wb == pp || flat) {
       double star = 0.0;
@@ -839,24 +900,22 @@ int ref_calmacros(sym_handle* h) {
   return check_cuda(h, cudaGetLastError(), "calmacros");
 }
 
-int ref_derivatives(sym_handle* h) {
+// mirrored: rho_N is already on the mirror planes (inside a run of steps)
+int ref_derivatives(sym_handle* h, bool mirrored) {
   const DevParams& P = h->dp;
   const unsigned g = blocks_for(range_count(P));
-  k_pin_fill<<<g, TPB, 0, h->st>>>(P, h->pin, h->walls_all, h->rhoN);
-  if (P.ref) {
+  k_pin_fill<<<blocks_for((P.N + 3) / 4), TPB, 0, h->st>>>(P, h->pin, h->walls_all, h->rhoN, mirrored);
+  if (P.ref && !mirrored) {
     MirrorSet S;
     S.scalar[S.ns++] = h->rhoN;
     mirror(h, S);
   }
-  k_gradient<<<g, TPB, 0, h->st>>>(P, h->dpart, h->pout, h->walls_all, h->rhoN, h->gx, h->gy, h->gz, h->nx, h->ny,
-                                   h->nz, h->flag);
-  if (P.ref) {
-    MirrorSet S;
-    S.vec[0][0] = h->nx; S.vec[0][1] = h->ny; S.vec[0][2] = h->nz;
-    S.vec[1][0] = h->gx; S.vec[1][1] = h->gy; S.vec[1][2] = h->gz;
-    S.nv = 2;
-    mirror(h, S);
-  }
+  auto go = [&](auto kern) {
+    kern<<<g, TPB, 0, h->st>>>(P, h->dpart, h->pout, h->walls_all, h->rhoN, h->gx, h->gy, h->gz, h->nx, h->ny, h->nz,
+                               h->flag);
+  };
+  if (P.ref) go(k_gradient<true>);
+  else go(k_gradient<false>);
   return check_cuda(h, cudaGetLastError(), "derivatives");
 }
 
@@ -875,10 +934,11 @@ int ref_recolor(sym_handle* h) {
   return check_cuda(h, cudaGetLastError(), "recolor");
 }
 
-int ref_boundary(sym_handle* h) {
+int ref_boundary(sym_handle* h, bool full) {
   const DevParams& P = h->dp;
   if (!P.ref) return SYM_OK;
-  k_boundary<<<blocks_for(plane_count(P, true)), TPB, 0, h->st>>>(P, h->ri, h->bi);
+  if (full) k_boundary<true><<<blocks_for(plane_count(P, true)), TPB, 0, h->st>>>(P, h->ri, h->bi);
+  else k_boundary<false><<<blocks_for(plane_count(P, true)), TPB, 0, h->st>>>(P, h->ri, h->bi);
   return check_cuda(h, cudaGetLastError(), "boundary");
 }
 
@@ -988,20 +1048,6 @@ int soa_to_aos(sym_handle* h, const double* soa, double* aos) {
 }
 
 // ---- the pieces of a run of steps (see k_step_macros) ----
-namespace {
-void mirror_phase(sym_handle* h, bool wall_phi, bool colours) {
-  MirrorSet S;
-  if (colours) {
-    S.scalar[S.ns++] = h->rhoR;
-    S.scalar[S.ns++] = h->rhoB;
-  }
-  if (wall_phi) S.low = h->rhoN;
-  else S.scalar[S.ns++] = h->rhoN;
-  mirror(h, S);
-}
-}  // namespace
-void mirror_phi(sym_handle* h) { mirror_phase(h, false, false); }
-
 int ref_step_macros(sym_handle* h, bool pull, bool full) {
   const DevParams& P = h->dp;
   auto go = [&](auto kern) {
@@ -1016,8 +1062,15 @@ int ref_step_macros(sym_handle* h, bool pull, bool full) {
     std::swap(h->ri, h->ft);
     std::swap(h->bi, h->ft2);
   }
-  if (full) mirror_macros(h, true);
-  else mirror_phase(h, true, true);
+  if (full) {
+    mirror_macros(h, true);
+  } else {   // (images written by the kernel itself cost it 60 us in divergence, the pass 10)
+    MirrorSet S;
+    S.scalar[S.ns++] = h->rhoR;
+    S.scalar[S.ns++] = h->rhoB;
+    S.low = h->rhoN;
+    mirror(h, S);
+  }
   return check_cuda(h, cudaGetLastError(), "step macros");
 }
 

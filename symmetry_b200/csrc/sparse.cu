@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kT) k_sp_lagrange_table(const SpDom* __restric
 // or the momentum exchange over the link list of one block of its box (v = 1;
 // the list was written by the previous step's set_walls, or by the import)
 constexpr int kLagShared = 8 * 7;
-__global__ void __launch_bounds__(kT, 2) k_sp_forces(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
+__global__ void __launch_bounds__(kT, 4) k_sp_forces(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
   __shared__ double sh[kLagShared];
   const Blk e = map[blockIdx.x];
   const SpDom& D = doms[e.d];
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kT) k_sp_masks(const SpDom* __restrict__ doms,
 // refilled node (it averages fluid neighbours only), and the particle it
 // belongs to -- the last one next to it -- is read off the masks, not off pout
 template <typename S>
-__global__ void __launch_bounds__(kT, 2) k_sp_pins(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
+__global__ void __launch_bounds__(kT, 4) k_sp_pins(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
   using R = typename Codec<S>::R;
   __shared__ int sh[8];
   const Blk e = map[blockIdx.x];

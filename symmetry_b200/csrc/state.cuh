@@ -94,10 +94,10 @@ void dev_release(sym_handle* h, void* p);               // frees only what did n
 
 // canonical (reference-structured) kernels, ref_kernels.cu
 int ref_calmacros(sym_handle* h);
-int ref_derivatives(sym_handle* h);
+int ref_derivatives(sym_handle* h, bool mirrored = false);
 int ref_collision(sym_handle* h);
 int ref_recolor(sym_handle* h);
-int ref_boundary(sym_handle* h);
+int ref_boundary(sym_handle* h, bool full = true);
 int ref_streaming(sym_handle* h, int which);
 int ref_curve(sym_handle* h);
 // passes of a run of steps (REFERENCE geometry; need ft and ft2)
@@ -122,7 +122,9 @@ int part_capillary_force2(sym_handle* h);
 int part_momentum(sym_handle* h);
 int part_repulsive(sym_handle* h);
 int part_movement(sym_handle* h);
-int part_refilling(sym_handle* h, bool phi_only = false);
+int part_refilling(sym_handle* h, bool in_run = false);
+int part_lagrange_capillary(sym_handle* h);   // both subroutines in one go
+int part_repulsive_movement(sym_handle* h);
 int part_initia_center(sym_handle* h);
 
 // fused fast path, fast.cu
