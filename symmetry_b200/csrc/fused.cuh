@@ -924,12 +924,19 @@ __device__ __forceinline__ void pinfill_node(const DevParams& P, const Pad& pd, 
                                              int x, int y, int z) {
   const long long L = lin(P, x, y, z);
   if (pin[L] <= 0) return;
-  R ws = R(0), v = R(0);
+  // masks and values of all neighbours are read together (one after another
+  // behind its mask, each a round trip to memory)
+  int wall[19];
+  R ph[19];
 #pragma unroll
   for (int i = 1; i < 19; i++) {
-    const long long nb = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
-    if (walls_all[nb] <= 0) { ws = ws + R(W(i)); v = v + R(W(i)) * phi[pd.idx(x + CX(i), y + CY(i), z + CZ(i))]; }
+    wall[i] = walls_all[lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz))];
+    ph[i] = phi[pd.idx(x + CX(i), y + CY(i), z + CZ(i))];
   }
+  R ws = R(0), v = R(0);
+#pragma unroll
+  for (int i = 1; i < 19; i++)
+    if (wall[i] <= 0) { ws = ws + R(W(i)); v = v + R(W(i)) * ph[i]; }
   phi_store<R>(P, pd, phi, x, y, z, v / ws);
 }
 
@@ -950,23 +957,28 @@ __device__ __forceinline__ void prep_node(const DevParams& P, const Pad& pd, con
   using R = typename Codec<S>::R;
   const long long L = lin(P, x, y, z);
   const unsigned N = (unsigned)P.N;
+  // masks and populations are read together, not one behind the other
   const Ref rref = Codec<S>::kRef ? rr_old[pd.idx(x, y, z)] : Ref{};
-  if (walls_all[L] > 0) {
+  const int wall = walls_all[L], near = pout[L];
+  R pr[19], pb[19];
+  unroll19([&](auto ic) {
+    constexpr int i = decltype(ic)::value;
+    Codec<S>::template load<i>(pops, N, (unsigned)L, rref, pr[i], pb[i]);
+  });
+  if (wall > 0) {
     rhoN[L] = 0.0;
     gx[L] = 0.0; gy[L] = 0.0; gz[L] = 0.0; nxv[L] = 0.0; nyv[L] = 0.0; nzv[L] = 0.0;
     return;
   }
   // fi is read only by the momentum exchange, at nodes with links into a
   // particle (pout > 0): written there only
-  const bool links = pout[L] > 0;
+  const bool links = near > 0;
   R sr = R(0), sb = R(0);
   unroll19([&](auto ic) {
     constexpr int i = decltype(ic)::value;
-    R r, b;
-    Codec<S>::template load<i>(pops, N, (unsigned)L, rref, r, b);
-    if (links) fi[(size_t)i * N + L] = (double)(r + b);
-    sr = sr + r;
-    sb = sb + b;
+    if (links) fi[(size_t)i * N + L] = (double)(pr[i] + pb[i]);
+    sr = sr + pr[i];
+    sb = sb + pb[i];
   });
   rhoR[L] = (double)sr; rhoB[L] = (double)sb;
   rhoN[L] = (double)phi_cur[pd.idx(x, y, z)];
@@ -983,7 +995,7 @@ __device__ __forceinline__ void prep_node(const DevParams& P, const Pad& pd, con
   R n0 = R(0), n1 = R(0), n2 = R(0);
   if (fn > R(P.evap)) {
     n0 = g0 / fn; n1 = g1 / fn; n2 = g2 / fn;
-    const int q = pout[L];
+    const int q = near;
     if (q >= 1) {
       wet_rotate<R>(P, Sp, q, x, y, z, n0, n1, n2);
       g0 = fn * n0; g1 = fn * n1; g2 = fn * n2;

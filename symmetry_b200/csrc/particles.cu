@@ -48,7 +48,7 @@ __global__ void k_walls_pinpout_box(DevParams P, Box b, const sym_particles* __r
                                     int32_t* pin, int32_t* pout) {
   int x, y, z;
   if (!box_node(P, b, S->center, blockIdx.y + 1, blockIdx.x * (long long)blockDim.x + threadIdx.x, x, y, z)) return;
-  pinpout_particles(P, x, y, z, walls, walls_all, pin, pout);
+  pinpout_particles(P, x, y, z, blockIdx.y + 1, walls, walls_all, pin, pout);
 }
 __global__ void k_walls_pinpout_plane(DevParams P, int xplane, int id, const int32_t* __restrict__ walls,
                                       const int32_t* __restrict__ walls_all, int32_t* pin, int32_t* pout) {

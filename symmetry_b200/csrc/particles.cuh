@@ -121,23 +121,32 @@ __device__ __forceinline__ void pinpout_node(const DevParams& P, int x, int y, i
 }
 
 // pin and pout of node (x,y,z) next to any particles: pout names the last of them
-// (the threads of several particles' boxes write the same values)
-__device__ __forceinline__ void pinpout_particles(const DevParams& P, int x, int y, int z,
-                                                  const int32_t* __restrict__ walls,
-                                                  const int32_t* __restrict__ walls_all, int32_t* pin, int32_t* pout) {
-  if (!in_range(P, x, y, z)) return;
+// (the threads of several particles' boxes write the same values).  Returns the
+// node's links into particle `id`: bit i set when the neighbour x + c_i is its.
+__device__ __forceinline__ unsigned pinpout_particles(const DevParams& P, int x, int y, int z, int id,
+                                                      const int32_t* __restrict__ walls,
+                                                      const int32_t* __restrict__ walls_all, int32_t* pin,
+                                                      int32_t* pout) {
+  if (!in_range(P, x, y, z)) return 0;
   const long long L = lin(P, x, y, z);
-  if (walls_all[L] != 0) return;
+  const int own = walls_all[L];
+  int w[19];
+#pragma unroll
+  for (int i = 1; i < 19; i++)
+    w[i] = walls[lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz))];
+  if (own != 0) return 0;
   int last = 0;
+  unsigned links = 0;
+#pragma unroll
   for (int i = 1; i < 19; i++) {
-    const long long nb = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
-    const int w = walls[nb];
-    if (w >= 1 && w <= P.par) {
-      pin[nb] = w;
-      last = w > last ? w : last;
+    if (w[i] >= 1 && w[i] <= P.par) {
+      pin[lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz))] = w[i];
+      last = w[i] > last ? w[i] : last;
+      if (w[i] == id) links |= 1u << i;
     }
   }
   if (last) pout[L] = last;
+  return links;
 }
 
 // ---- Lagrange_points (Source1.f90:1799-1978) ----------------------------------
@@ -212,12 +221,25 @@ __device__ __forceinline__ void lagrange_point(const DevParams& P, const sym_par
     iy0 = lag_idx(P, y0, P.ny, 1); iy1 = lag_idx(P, y0 + 1, P.ny, 1);
     iz0 = lag_idx(P, z0, P.nz, 2); iz1 = lag_idx(P, z0 + 1, P.nz, 2);
     double wsum = 0.0, acc = 0.0;
+    // four corners at a time, mask and values read together (read behind the
+    // mask, corner after corner, they were most of the kernel's time)
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const long long xf = x0 + EX[i], yf = y0 + EY[i], zf = z0 + EZ[i];
-      const long long F = lin(P, EX[i] ? ix1 : ix0, EY[i] ? iy1 : iy0, EZ[i] ? iz1 : iz0);
-      if (walls[F] <= 0) {
-        const double star = rhoN[F] + gx[F] * (lx - (double)xf) + gy[F] * (ly - (double)yf) + gz[F] * (lz - (double)zf);
+    for (int h = 0; h < 8; h += 4) {
+      int wall[4];
+      double c0[4], c1[4], c2[4], c3[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int i = h + k;
+        const long long F = lin(P, EX[i] ? ix1 : ix0, EY[i] ? iy1 : iy0, EZ[i] ? iz1 : iz0);
+        wall[k] = walls[F];
+        c0[k] = rhoN[F]; c1[k] = gx[F]; c2[k] = gy[F]; c3[k] = gz[F];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int i = h + k;
+        const long long xf = x0 + EX[i], yf = y0 + EY[i], zf = z0 + EZ[i];
+        if (wall[k] > 0) continue;
+        const double star = c0[k] + c1[k] * (lx - (double)xf) + c2[k] * (ly - (double)yf) + c3[k] * (lz - (double)zf);
         const double dis = (double)(xf - lx) * (double)(xf - lx) + ((double)yf - ly) * ((double)yf - ly) +
                            ((double)zf - lz) * ((double)zf - lz);
         const double w = 1.0 / dis;
@@ -239,14 +261,24 @@ __device__ __forceinline__ void lagrange_point(const DevParams& P, const sym_par
     double mn = 100.0;
     long long G = lin(P, ix0, iy0, iz0);   // corner 0 unless a nearer one qualifies
 #pragma unroll 1
-    for (int i = 0; i < 8; i++) {
-      const int ex = ((i + 1) >> 1) & 1, ey = (i >> 1) & 1, ez = (i >> 2) & 1;   // EX[i], EY[i], EZ[i]
-      const long long xf = x0 + ex, yf = y0 + ey, zf = z0 + ez;
-      const bool inside = P.ref ? (xf <= P.nx && yf >= 1 && yf <= P.ny && zf <= P.nz) : true;
-      if (!inside) continue;
-      const long long F = lin(P, ex ? ix1 : ix0, ey ? iy1 : iy0, ez ? iz1 : iz0);
-      if (walls[F] <= 0) {
-        if (fabs(nxv[F] * nxv[F] + nyv[F] * nyv[F] + nzv[F] * nzv[F]) > 0.0) {
+    for (int h = 0; h < 8; h += 4) {
+      int wall[4];
+      double c1[4], c2[4], c3[4];
+      long long Fs[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        // EX, EY of corner h + k do not depend on h; EZ is 0 below 4
+        const long long F = lin(P, EX[k] ? ix1 : ix0, EY[k] ? iy1 : iy0, h ? iz1 : iz0);
+        Fs[k] = F;
+        wall[k] = walls[F];
+        c1[k] = nxv[F]; c2[k] = nyv[F]; c3[k] = nzv[F];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const long long xf = x0 + EX[k], yf = y0 + EY[k], zf = z0 + (h ? 1 : 0), F = Fs[k];
+        const bool inside = P.ref ? (xf <= P.nx && yf >= 1 && yf <= P.ny && zf <= P.nz) : true;
+        if (!inside || wall[k] > 0) continue;
+        if (fabs(c1[k] * c1[k] + c2[k] * c2[k] + c3[k] * c3[k]) > 0.0) {
           const double dis = ((double)xf - lx) * ((double)xf - lx) + ((double)yf - ly) * ((double)yf - ly) +
                              ((double)zf - lz) * ((double)zf - lz);
           if (sqrt(dis) < mn) { mn = sqrt(dis); G = F; }
@@ -669,9 +701,20 @@ __device__ __forceinline__ void refill_values(const DevParams& P, int pp, const 
   const double u2 = PC(S->up, par, pp, 2) + yr * PC(S->rp, par, pp, 0) - xr * PC(S->rp, par, pp, 1);
   ux[L] = u0; uy[L] = u1; uz[L] = u2;
   double sr = 0.0, sb = 0.0, num = 0.0;
-  for (int i = 1; i < 19; i++) {
-    const long long nb = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
-    if (walls_old[nb] <= 0) { sr = sr + rhoR[nb]; sb = sb + rhoB[nb]; num = num + 1.0; }
+#pragma unroll
+  for (int h = 1; h < 19; h += 9) {   // nine neighbours at a time, mask and densities together
+    int wall[9];
+    double nr[9], nb_[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+      const int i = h + k;
+      const long long nb = lin(P, wrapi(x + CX(i), P.nx), wrapi(y + CY(i), P.ny), wrapi(z + CZ(i), P.nz));
+      wall[k] = walls_old[nb];
+      nr[k] = rhoR[nb]; nb_[k] = rhoB[nb];
+    }
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      if (wall[k] <= 0) { sr = sr + nr[k]; sb = sb + nb_[k]; num = num + 1.0; }
   }
   const double R = sr / num, B = sb / num, rh = R + B;
   rhoR[L] = R; rhoB[L] = B; rho[L] = rh; rhoN[L] = (R - B) / rh;

@@ -80,7 +80,7 @@ struct Blk {
 
 // ---- kernels -------------------------------------------------------------------
 template <typename S>
-__global__ void __launch_bounds__(kT, 4) k_sp_prep(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
+__global__ void __launch_bounds__(kT, 2) k_sp_prep(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
   using R = typename Codec<S>::R;
   const Blk e = map[blockIdx.x];
   const SpDom& D = doms[e.d];
@@ -240,14 +240,10 @@ __global__ void __launch_bounds__(kT, 4) k_sp_pins(const SpDom* __restrict__ dom
   if (e.v == 0) {
     bool has = false;
     unsigned L = 0, mask = 0;
-    if (part::box_node(P, D.bpin, D.S->center, e.pp, t, x, y, z) && part::in_range(P, x, y, z)) {
-      part::pinpout_particles(P, x, y, z, D.walls, D.walls_all, D.pin, D.pout);
-      const long long l = lin(P, x, y, z);
-      if (D.walls_all[l] == 0) {
-        mask = part::link_mask(P, x, y, z, e.pp, D.walls);
-        has = mask != 0;
-        L = (unsigned)l;
-      }
+    if (part::box_node(P, D.bpin, D.S->center, e.pp, t, x, y, z)) {
+      mask = part::pinpout_particles(P, x, y, z, e.pp, D.walls, D.walls_all, D.pin, D.pout);
+      has = mask != 0;
+      L = (unsigned)lin(P, x, y, z);
     }
     const long long seg = (long long)(e.pp - 1) * D.link_blocks + e.b;
     part::link_compact(has, L, mask, D.links + seg * kT, D.nlinks + seg, sh);
