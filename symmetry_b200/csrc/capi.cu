@@ -235,7 +235,7 @@ int canonical_piece(sym_handle* h, int piece) {
   if (h->p.par > 0)
     if ((e = part_refilling(h, !last))) return e;
   if ((e = ref_derivatives(h, !last))) return e;
-  if ((e = ref_collide_recolor(h, last))) return e;
+  if ((e = ref_collide_recolor(h, last, piece == MID))) return e;
   if ((e = ref_boundary(h, last))) return e;
   if (!last) return SYM_OK;
   if ((e = ref_stream_both(h))) return e;
@@ -277,8 +277,13 @@ int run_piece(sym_handle* h, int piece) {
 }
 
 int canonical_steps(sym_handle* h, int nsteps) {
-  // the second streaming target: without room for it the steps run one by one
+  // the second streaming target and its marks: without room for them the steps
+  // run one by one
   bool runs = h->dp.ref && !h->p.bounce;
+  if (runs && !h->kept && dalloc(h, &h->kept, h->N)) {
+    h->kept = nullptr;
+    runs = false;
+  }
   if (runs && !h->ft2 && dalloc(h, &h->ft2, 19 * h->N)) {
     h->ft2 = nullptr;
     runs = false;
@@ -453,7 +458,7 @@ int sym_destroy(sym_handle* h) {
     cudaGraphDestroy(g.graph);
   }
   fast_free(h);
-  void* ptrs[] = {h->ri, h->bi, h->fi, h->ffi, h->ft, h->ft2, h->rho, h->ux, h->uy, h->uz, h->rhoN, h->rhoR, h->rhoB,
+  void* ptrs[] = {h->ri, h->bi, h->fi, h->ffi, h->ft, h->ft2, h->kept, h->rho, h->ux, h->uy, h->uz, h->rhoN, h->rhoR, h->rhoB,
                   h->nx, h->ny, h->nz, h->gx, h->gy, h->gz, h->flag, h->walls, h->walls_old, h->walls_all,
                   h->pin, h->pout, h->dpart, h->lax, h->lay, h->laz, h->larhon, h->lanx, h->lany, h->lanz,
                   h->lads, h->laflag, h->red};

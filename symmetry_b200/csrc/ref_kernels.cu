@@ -289,7 +289,7 @@ __global__ void k_gradient(DevParams P, const sym_particles* __restrict__ S, con
   if (walls_all[L] <= 0) {
 #pragma unroll
     for (int i = 1; i < 19; i++) {
-      const double val = W(i) * rhoN[REF ? L + CZ(i) + P.nz * (CY(i) + (long long)P.ny * CX(i)) : nbr(P, x, y, z, i)];
+      const double val = W(i) * (REF ? (rhoN + L)[CZ(i) + P.nz * (CY(i) + P.ny * CX(i))] : rhoN[nbr(P, x, y, z, i)]);
       if (CX(i)) g0 = g0 + val * (double)CX(i);
       if (CY(i)) g1 = g1 + val * (double)CY(i);
       if (CZ(i)) g2 = g2 + val * (double)CZ(i);
@@ -569,23 +569,28 @@ __global__ void k_curve2(DevParams P, const sym_particles* __restrict__ S, const
 // ---- whole steps (sym_step, REFERENCE geometry, halfway bounce-back) -------------
 // A run of n steps is the reference's loop body n times, cut between the calls
 // so that passes over the populations fall together (152^3 per step, bytes per
-// node: separate subroutines about 2,700, these about 1,450):
+// node: separate subroutines about 2,700, these about 1,150):
 //   streaming of both colours, curve and the next step's calmacros in one pass
 //   (k_step_macros<true>), and collision with Recolor in one (k_collide_recolor).
+//   Both passes pull the streamed populations from the ones boundary left; only
+//   those that curve, refilling or the walls' carry-over make or need are
+//   written in between (`kept`: boundary planes, solids, nodes next to a
+//   particle), so a step reads the populations twice and writes them once.
 // What no later call of the same run reads is written by the run's last step
 // only (FULL): fi and ffi away from the particles, rho and u, and the mirror
 // planes' copies of them.
 
 // calmacros (:770-831) of the populations (ri, bi); PULL: of the populations
 // that streaming (:735-768) and curve (:990-1034) make of them, which go to
-// (ro, bo) on every node of the arrays.  !FULL: fi only next to particles (the
-// momentum exchange reads it there), no rho and u.
+// (ro, bo) on every node (FULL) or on those it marks in kept.  !FULL: fi only
+// next to particles (the momentum exchange reads it there), no rho and u.
 template <bool PULL, bool FULL>
 __global__ void __launch_bounds__(TPB) k_step_macros(DevParams P, const sym_particles* __restrict__ S,
                                                      const double* __restrict__ ri, const double* __restrict__ bi,
-                                                     double* __restrict__ ro, double* __restrict__ bo, double* fi,
-                                                     double* rho, double* ux, double* uy, double* uz, double* rhoN,
-                                                     double* rhoR, double* rhoB, const int32_t* __restrict__ walls,
+                                                     double* __restrict__ ro, double* __restrict__ bo,
+                                                     unsigned char* __restrict__ kept, double* fi, double* rho,
+                                                     double* ux, double* uy, double* uz, double* rhoN, double* rhoR,
+                                                     double* rhoB, const int32_t* __restrict__ walls,
                                                      const int32_t* __restrict__ walls_all,
                                                      const int32_t* __restrict__ pout) {
   const long long N = P.N, L = blockIdx.x * (long long)TPB + threadIdx.x;
@@ -598,13 +603,18 @@ __global__ void __launch_bounds__(TPB) k_step_macros(DevParams P, const sym_part
   const bool solid = in && walls_all[L] >= 1;
   double r[19], b[19];
   if (PULL) {
-    r[0] = ri[L];
-    b[0] = bi[L];
+    // 32-bit offsets along each axis, from one pointer per velocity
+    const int sx = P.ny * P.nz, sy = P.nz;
+    const int ox[3] = {x + 1 < P.nx ? sx : -(P.nx - 1) * sx, 0, x > 0 ? -sx : (P.nx - 1) * sx};
+    const int oy[3] = {y + 1 < P.ny ? sy : -(P.ny - 1) * sy, 0, y > 0 ? -sy : (P.ny - 1) * sy};
+    const int oz[3] = {z + 1 < P.nz ? 1 : -(P.nz - 1), 0, z > 0 ? -1 : P.nz - 1};
+    const double* const rL = ri + L;
+    const double* const bL = bi + L;
 #pragma unroll
-    for (int i = 1; i < 19; i++) {
-      const long long src = i * N + lin(P, wrapi(x - CX(i), P.nx), wrapi(y - CY(i), P.ny), wrapi(z - CZ(i), P.nz));
-      r[i] = ri[src];
-      b[i] = bi[src];
+    for (int i = 0; i < 19; i++) {
+      const int o = ox[CX(i) + 1] + oy[CY(i) + 1] + oz[CZ(i) + 1];
+      r[i] = (rL + i * N)[o];
+      b[i] = (bL + i * N)[o];
     }
     if (pp >= 1) {
       // link i comes from a node of particle pp: this node's own opposite
@@ -627,11 +637,15 @@ __global__ void __launch_bounds__(TPB) k_step_macros(DevParams P, const sym_part
         b[i] = bi[OPC(i) * N + L] + 6.0 * W(i) * cb * star;
       }
     }
+    const bool keep = !in || solid || pp >= 1;
+    if (FULL || keep) {
 #pragma unroll
-    for (int i = 0; i < 19; i++) {
-      ro[i * N + L] = r[i];
-      bo[i * N + L] = b[i];
+      for (int i = 0; i < 19; i++) {
+        ro[i * N + L] = r[i];
+        bo[i * N + L] = b[i];
+      }
     }
+    if (!FULL) kept[L] = keep;
     if (!in) return;
   }
   if (solid) {
@@ -668,16 +682,20 @@ __global__ void __launch_bounds__(TPB) k_step_macros(DevParams P, const sym_part
   }
 }
 
-// collision (:599-695) and Recolor (:697-732) of one node from its populations,
-// in place; the collision in the fused path's arithmetic (nodemath.cuh), bound
-// by memory instead of FP64 issue (the two kernels: 816 + 366 us at 152^3).
-template <bool FULL>
+// collision (:599-695) and Recolor (:697-732) of one node from its populations
+// (ri, bi), in place; the collision in the fused path's arithmetic
+// (nodemath.cuh), bound by memory instead of FP64 issue (the two kernels: 816 +
+// 366 us at 152^3).  PULL: the populations of nodes that k_step_macros did not
+// keep are streamed here from (rs, bs), without curve, which they were not part
+// of; a node that has become solid since gets them unchanged.
+template <bool FULL, bool PULL>
 __global__ void __launch_bounds__(128, 4) k_collide_recolor(
     DevParams P, const __grid_constant__ TileParams<double> T, const int32_t* __restrict__ walls_all,
     const int32_t* __restrict__ pout, const int32_t* __restrict__ flag, const double* __restrict__ nxv,
     const double* __restrict__ nyv, const double* __restrict__ nzv, const double* __restrict__ gx,
     const double* __restrict__ gy, const double* __restrict__ gz, const double* __restrict__ rhoN, double* ux,
-    double* uy, double* uz, double* fi, double* ffi, double* ri, double* bi) {
+    double* uy, double* uz, double* fi, double* ffi, double* ri, double* bi, const double* __restrict__ rs,
+    const double* __restrict__ bs, const unsigned char* __restrict__ kept) {
   using namespace fused;
   const unsigned t = blockIdx.x * 128u + threadIdx.x;
   const unsigned rz = P.hi[2] - P.lo[2] + 1, ry = P.hi[1] - P.lo[1] + 1;
@@ -685,15 +703,31 @@ __global__ void __launch_bounds__(128, 4) k_collide_recolor(
   const int z = P.lo[2] + (int)(t - q * rz), x = P.lo[0] + (int)(q / ry), y = P.lo[1] + (int)(q % ry);
   if (x > P.hi[0]) return;
   const long long L = lin(P, x, y, z), N = P.N;
-  if (walls_all[L] > 0) return;
+  const bool solid = walls_all[L] > 0;
+  const bool pull = PULL && !kept[L];
+  if (solid && !pull) return;
   const int pp = pout[L];
   const bool fl = flag[L] != 0;
   double f[19], cr[19];
+  const double* const fr = pull ? rs : ri;
+  const double* const fb = pull ? bs : bi;
 #pragma unroll
   for (int i = 0; i < 19; i++) {
-    cr[i] = ri[i * N + L];
-    f[i] = cr[i] + bi[i * N + L];
+    // an updated node's neighbours are inside the arrays
+    const long long o = i * N + L - (pull ? CZ(i) + P.nz * (CY(i) + P.ny * CX(i)) : 0);
+    cr[i] = fr[o];
+    f[i] = fb[o];
   }
+  if (solid) {
+#pragma unroll
+    for (int i = 0; i < 19; i++) {
+      ri[i * N + L] = cr[i];
+      bi[i * N + L] = f[i];
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 19; i++) f[i] = cr[i] + f[i];
   const double sr = cr[0] + ((cr[1] + cr[2]) + (cr[3] + cr[4]) + (cr[5] + cr[6])) +
                     (((cr[7] + cr[10]) + (cr[8] + cr[9])) + ((cr[11] + cr[14]) + (cr[12] + cr[13])) +
                      ((cr[15] + cr[18]) + (cr[16] + cr[17])));
@@ -1098,8 +1132,8 @@ int soa_to_aos(sym_handle* h, const double* soa, double* aos) {
 int ref_step_macros(sym_handle* h, bool pull, bool full) {
   const DevParams& P = h->dp;
   auto go = [&](auto kern) {
-    kern<<<blocks_for(P.N), TPB, 0, h->st>>>(P, h->dpart, h->ri, h->bi, h->ft, h->ft2, h->fi, h->rho, h->ux, h->uy,
-                                             h->uz, h->rhoN, h->rhoR, h->rhoB, h->walls, h->walls_all, h->pout);
+    kern<<<blocks_for(P.N), TPB, 0, h->st>>>(P, h->dpart, h->ri, h->bi, h->ft, h->ft2, h->kept, h->fi, h->rho, h->ux,
+                                             h->uy, h->uz, h->rhoN, h->rhoR, h->rhoB, h->walls, h->walls_all, h->pout);
   };
   if (pull && full) go(k_step_macros<true, true>);
   else if (pull) go(k_step_macros<true, false>);
@@ -1121,15 +1155,18 @@ int ref_step_macros(sym_handle* h, bool pull, bool full) {
   return check_cuda(h, cudaGetLastError(), "step macros");
 }
 
-int ref_collide_recolor(sym_handle* h, bool full) {
+// pulled: ref_step_macros(pull, !full) ran before it
+int ref_collide_recolor(sym_handle* h, bool full, bool pulled) {
   const DevParams& P = h->dp;
   const unsigned g = blocks_for(range_count(P), 128);
   auto go = [&](auto kern) {
     kern<<<g, 128, 0, h->st>>>(P, tile_params<double>(P), h->walls_all, h->pout, h->flag, h->nx, h->ny, h->nz, h->gx,
-                               h->gy, h->gz, h->rhoN, h->ux, h->uy, h->uz, h->fi, h->ffi, h->ri, h->bi);
+                               h->gy, h->gz, h->rhoN, h->ux, h->uy, h->uz, h->fi, h->ffi, h->ri, h->bi, h->ft, h->ft2,
+                               h->kept);
   };
-  if (full) go(k_collide_recolor<true>);
-  else go(k_collide_recolor<false>);
+  if (full) go(k_collide_recolor<true, false>);
+  else if (pulled) go(k_collide_recolor<false, true>);
+  else go(k_collide_recolor<false, false>);
   return check_cuda(h, cudaGetLastError(), "collision and recolour");
 }
 

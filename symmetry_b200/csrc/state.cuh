@@ -58,6 +58,7 @@ struct sym_handle {
   // canonical state (reference arrays, SoA, FP64)
   double *ri = nullptr, *bi = nullptr, *fi = nullptr, *ffi = nullptr, *ft = nullptr;
   double* ft2 = nullptr;   // second streaming target (runs of steps in REFERENCE geometry, on first use)
+  unsigned char* kept = nullptr;   // with ft2: nodes whose streamed populations are in ri, bi (k_step_macros)
   double *rho = nullptr, *ux = nullptr, *uy = nullptr, *uz = nullptr;
   double *rhoN = nullptr, *rhoR = nullptr, *rhoB = nullptr;
   double *nx = nullptr, *ny = nullptr, *nz = nullptr, *gx = nullptr, *gy = nullptr, *gz = nullptr;
@@ -100,9 +101,9 @@ int ref_recolor(sym_handle* h);
 int ref_boundary(sym_handle* h, bool full = true);
 int ref_streaming(sym_handle* h, int which);
 int ref_curve(sym_handle* h);
-// passes of a run of steps (REFERENCE geometry; need ft and ft2)
+// passes of a run of steps (REFERENCE geometry; need ft, ft2 and kept)
 int ref_step_macros(sym_handle* h, bool pull, bool full);
-int ref_collide_recolor(sym_handle* h, bool full);
+int ref_collide_recolor(sym_handle* h, bool full, bool pulled);
 int ref_stream_both(sym_handle* h);
 int ref_initialization(sym_handle* h);
 int ref_init_fill(sym_handle* h);    // rhoN, rho given -> populations

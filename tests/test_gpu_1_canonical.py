@@ -212,3 +212,26 @@ def test_reference_steps_leave_every_array(runs):
         e = rel_l2(L.get(f), o.arr(f))
         assert e <= 1e-10, (f, e)
     compare_particles(o, L, 12, 1e-9)
+
+
+def test_reference_run_covers_and_refills_nodes():
+    """Inside a run the streamed populations of a node are stored only next to
+    solids; particles that move half a node per step cover nodes whose
+    populations were not stored and uncover others, in every kind of step of a
+    run.  The same parity targets as above."""
+    p = params.reference_params(48, 88, 48)
+    o = setup_reference(p)
+    s = o.particles
+    params.particles_set(s, "up", 12, [(-0.5 + 0.02 * k, 0.04 * k - 0.2, -0.45) for k in range(12)])
+    L = Lattice(p)
+    copy_oracle_to_lattice(o, L)
+    before = L.get("walls_all").copy()
+    o.step(6)
+    L.step(6)
+    compare_masks(o, L)
+    after = L.get("walls_all")
+    assert ((before > 0) & (after == 0)).any() and ((before == 0) & (after > 0)).any()
+    for f in [f for f in SCALARS if f not in ("n_x", "n_y", "n_z")] + POPS:
+        e = rel_l2(L.get(f), o.arr(f))
+        assert e <= 1e-10, (f, e)
+    compare_particles(o, L, 12, 1e-9)
