@@ -209,8 +209,10 @@ struct Acc<float> {
 // densities (the phase field then reads 2 values per node) or the phase field
 // re-reads the populations (38 per node).  The accumulation costs arithmetic
 // (warp shuffles, a shared-memory exchange, atomics), the re-read costs
-// bytes: FP64 storage, bound by memory, accumulates; the 16-bit and FP32
-// storages, bound by instruction issue, re-read.
+// bytes: FP64 storage, bound by memory, accumulates; the 16-bit storage, bound
+// by arithmetic, re-reads, and FP32 does (accumulating was measured slower for
+// both with one node per thread: +2.7 ms of collide for -0.4 ms of phase on 45 M
+// nodes in 16 bits).
 template <typename S>
 constexpr bool kAccumulate = sizeof(S) == 8;
 
@@ -256,16 +258,22 @@ __device__ __forceinline__ void phase_node(const DevParams& P, const Pad& pd, co
     const unsigned N = (unsigned)P.N;
     if constexpr (Codec<S>::kRef) {
       const Ref ref = rr_old[pd.idx(x, y, z)];
-      R sr = R(0), sb = R(0);
-      unroll19([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        R r, b;
-        Codec<S>::template load<i>(pops, N, Lu, ref, r, b);
-        sr = sr + r;
-        sb = sb + b;
-      });
-      v = qdiv<R>(sr - sb, sr + sb);
-      nref = ref_pair(float(sr), float(sb));
+      // the deviations summed by weight, both of a velocity in one packed addition,
+      // and decoded once, as the collide kernel does (decoding every velocity was
+      // bound by instruction issue: 527 instructions a node)
+      const __half2* const in = reinterpret_cast<const __half2*>(pops) + Lu;
+      const F2 rest(__half22float2(in[0]));
+      F2 axis(__half22float2(in[N])), diag(__half22float2(in[7 * N]));
+#pragma unroll
+      for (unsigned i = 2; i < 7; i++) axis = axis + F2(__half22float2(in[i * N]));
+#pragma unroll
+      for (unsigned i = 8; i < 19; i++) diag = diag + F2(__half22float2(in[i * N]));
+      const F2 dev = vfma(F2(float(W(0) / 4096.0)), rest,
+                          vfma(F2(float(W(1) / 4096.0)), axis, F2(float(W(7) / 4096.0)) * diag));
+      // sr is exactly rho or 0 in a pure phase
+      const float rho = ref.x + dev[0], sr = fmaf(ref.y, rho, dev[1]), sb = rho - sr;
+      v = qdiv<R>(sr - sb, rho);
+      nref = make_float2(rho, sr / rho);
     } else {
       R sr = R(0), sf = R(0);
       unroll19([&](auto ic) {

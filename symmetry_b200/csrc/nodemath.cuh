@@ -8,9 +8,10 @@
 // f_i + f_opc(i), an odd row only f_i - f_opc(i), and within each kind the
 // rows are combinations of the same three axis sums and three face sums.  That
 // takes about a third of the operations of the rows written out pair by pair
-// (256x256x256 FP64 collide, bound by FP64 issue and its latency at 16 warps
-// per SM: 2260 -> 2060 us together with the curvature's six sums, the split
-// normals and one reciprocal square root per normal).
+// (256x256x256 FP64 collide 2260 -> 2060 us together with the curvature's six
+// sums, the split normals and one reciprocal square root per normal; what bounds
+// it now is the latency of its loads at 16 warps per SM, the FP64 pipe is 25 %
+// busy).
 #pragma once
 #include "lattice.cuh"
 
