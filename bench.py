@@ -74,11 +74,12 @@ def b_phase(storage):
 
 # DRAM bytes per node of one collide launch, dram__bytes_read.sum +
 # dram__bytes_write.sum from one ncu capture divided by the nodes of the
-# launch: profiles/k_collide_batch_fp16_mix24.md (16-bit, batched kernel) and
-# profiles/k_collide_fp64_thread_128x128x256.md (FP64, single-domain kernel;
-# the batched kernel runs the same tile code).  The traffic per node does not
-# depend on the number of nodes, so it scales to a full launch.
-COLLIDE_TRAFFIC_B_PER_NODE = {"fp16": 224.7, "fp64": 704.2}
+# launch: profiles/k_collide_batch_fp16_mix24.md (16-bit, uneven domains in the
+# batched kernel) and profiles/k_collide_thread_128x128x256.md (FP64,
+# single-domain kernel; the batched kernel runs the same tile code).  The
+# traffic per node does not depend on the number of nodes, so it scales to a
+# full launch.
+COLLIDE_TRAFFIC_B_PER_NODE = {"fp16": 224.7, "fp64": 648.0}
 
 
 def collide_traffic(storage, nodes):
