@@ -67,6 +67,18 @@ __device__ __forceinline__ bool box_node(const DevParams& P, const Box& b, const
   x = v[0]; y = v[1]; z = v[2];
   return true;
 }
+// whether box_node comes up with node (x, y, z)
+__device__ __forceinline__ bool in_box(const DevParams& P, const Box& b, const double* centre, int pp, int x, int y,
+                                       int z) {
+  const int dims[3] = {P.nx, P.ny, P.nz}, v[3] = {x, y, z};
+  for (int k = 0; k < 3; k++) {
+    if (b.full[k]) continue;
+    int q = v[k] - (int)floor(centre[k * P.par + pp - 1] - (double)P.origin - P.rad - b.margin);
+    if (!P.ref && !(k == 0 && P.wall_x)) q = ((q % dims[k]) + dims[k]) % dims[k];
+    if (q < 0 || q >= b.n[k]) return false;
+  }
+  return true;
+}
 __device__ __forceinline__ bool in_range(const DevParams& P, int x, int y, int z) {
   return x >= P.lo[0] && x <= P.hi[0] && y >= P.lo[1] && y <= P.hi[1] && z >= P.lo[2] && z <= P.hi[2];
 }

@@ -175,9 +175,11 @@ __global__ void __launch_bounds__(kT) k_sp_move(const SpDom* __restrict__ doms, 
 // particle's previous box (pout reaches one link beyond the sphere), where each
 // node becomes what it is now -- flat wall, sphere, fluid.  v = 1: the flat
 // wetting walls, solid at every step, so their previous mask is solid too.
-// v = 2: marks on the sphere's present box (where it left the previous one).
+// v = 2: marks on the part of the sphere's present box that the previous one does
+// not hold -- a node of both is v = 0's alone, which reads its previous mask.
 // More than one particle: v = 3 clears the whole domain, and the marks (v = 2)
-// follow in a launch of their own.  Threads that meet on a node write the same.
+// follow in a launch of their own.  Otherwise threads that meet on a node write
+// the same, and none reads what another writes.
 __global__ void __launch_bounds__(kT) k_sp_masks(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
   const Blk e = map[blockIdx.x];
   const SpDom& D = doms[e.d];
@@ -207,6 +209,7 @@ __global__ void __launch_bounds__(kT) k_sp_masks(const SpDom* __restrict__ doms,
     D.walls[L] = id; D.walls_all[L] = 10; D.walls_old[L] = 10;
   } else if (e.v == 2) {
     if (!part::box_node(P, D.bmark, D.S->center, e.pp, t, x, y, z)) return;
+    if (!D.full_reset && part::in_box(P, D.bpin, D.S->center_old, 1, x, y, z)) return;
     part::walls_mark_last(P, D.S, e.pp, r2, x, y, z, D.walls, D.walls_all);
   } else {
     if (t >= P.N) return;

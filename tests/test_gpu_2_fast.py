@@ -5,6 +5,8 @@ masks bit-exact, particle trajectories <= 1e-9.  FP32 and FP16 shifted storage:
 relative L2 velocity error against FP64 <= 1e-3 (the precision target), with
 the measured errors printed.
 """
+import itertools
+
 import numpy as np
 import pytest
 
@@ -232,3 +234,38 @@ def test_get_macros_leaves_stepping_state_untouched(storage):
         ref = c.get(k)
         scale = max(np.abs(ref[fluid]).max(), 1e-300)
         assert np.abs(m[k][fluid] - ref[fluid]).max() <= 1e-12 * scale, k
+
+
+@pytest.mark.parametrize("rad,centre,up", [
+    (3.28, (13.39, 12.67, 13.44), (0.31, -0.30, -0.07)),
+    (2.2, (12.3, 11.51, 9.34), (0.38, -0.31, 0.15)),
+    (2.61, (13.68, 9.12, 0.11), (0.12, -0.21, -0.38)),
+])
+def test_fast_fp64_node_uncovered_beside_a_covered_one(rad, centre, up):
+    """A sphere that moves by a third of a node uncovers nodes next to nodes it
+    covers in the same step.  The uncovered node's refill averages the
+    neighbours that were fluid before (walls_old, the newly covered one among
+    them).  A heavy sphere keeps its velocity; FP64 parity bounds of this
+    file, the masks exact."""
+    w = configs.c2_wall_particle(nx=28, ny=25, nz=32, rad=rad, centre=centre, z0=6.0, z1=20.0)
+    w.params.mass *= 1e4
+    w.params.inertia *= 1e4
+    w.particles[0]["up"] = list(up)
+    met = False
+    for steps in (1, 2, 3):
+        o, L = fast_run(w, steps, with_oracle=False)
+        before = o.arr("walls_all").copy()
+        for _ in range(steps):
+            before = o.arr("walls_all").copy()
+            o.step(1)
+        uncovered = (before > 0) & (o.arr("walls_all") == 0)
+        covered = (before == 0) & (o.arr("walls_all") > 0)
+        links = [d for d in itertools.product((-1, 0, 1), repeat=3) if 1 <= sum(map(abs, d)) <= 2]
+        met = met or any((uncovered & np.roll(covered, d, (0, 1, 2))).any() for d in links)
+        o.call("calmacros")
+        compare_masks(o, L, ["walls", "walls_old", "walls_all", "pin", "pout"])
+        e = errors(o, L, mask=o.arr("walls_all") == 0)
+        assert max(e.values()) <= 1e-10, e
+        compare_particles(o, L, 1, 1e-9)
+        L.close()
+    assert met
