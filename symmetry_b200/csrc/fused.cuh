@@ -558,7 +558,19 @@ __device__ __forceinline__ void collide_tile(const TileParams<double>& P, const 
           const R rf = rsqrt(g2s);
           fn = g2s * rf;
           n0 = g0 * rf; n1 = g1 * rf; n2 = g2 * rf;
-          if (solid && id >= 1) wet_rotate<R>(P, Sp, id, wrapi(xp, P.nx), y, z, n0, n1, n2);
+          if (solid && id >= 1) {
+            // the rotation has to know a gradient along the wall's normal, whose
+            // unit vector is exactly 1 there (the reference's quotient) and with
+            // rsqrt may be an ulp to either side
+            const R m = fmax(fabs(g0), fmax(fabs(g1), fabs(g2)));
+            if (m * m == g2s) {
+              fn = m;
+              if (fabs(g0) == m) n0 = copysign(R(1), g0);
+              if (fabs(g1) == m) n1 = copysign(R(1), g1);
+              if (fabs(g2) == m) n2 = copysign(R(1), g2);
+            }
+            wet_rotate<R>(P, Sp, id, wrapi(xp, P.nx), y, z, n0, n1, n2);
+          }
         }
       }
       sm.n.set(s, py, pz, n0, n1, n2, fn);

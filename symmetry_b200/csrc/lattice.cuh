@@ -325,8 +325,9 @@ __device__ __forceinline__ void veccross(const double a[3], const double b[3], d
 // cos(acos(.)) and sin(acos(.)) for unit vectors) with sin(theta) held at or
 // above sin(1e-5) at both ends: in single precision nw.n rounds to exactly +-1
 // for angles up to ~3.5e-4, where the acos form divides by sin(0) = 0.
-// FP64 takes them the same way without the bound: the reference's division by
-// sin(0) for parallel vectors stays what it is.
+// FP64 takes them by algebra without the bound.  Its ends are the reference's:
+// of parallel vectors sin(acos(1)) = 0 divides, of opposite ones
+// sin(acos(-1)) = sin(M_PI) = 1.2e-16 does, which leaves the result finite.
 template <typename R>
 __device__ __forceinline__ void akai_rotate_sc(R sc, R cc, const R nw[3], const R n[3], bool guard, R out[3]);
 template <typename R>
@@ -349,14 +350,20 @@ __device__ __forceinline__ void akai_rotate_sc(R sc, R cc, const R nw[3], const 
     }
   } else {
     // cos(acos(c)) and sin(acos(c)) by algebra: c, and sqrt((1 - c)(1 + c)), whose
-    // first factor is exact near 1 (the three functions one after another are
-    // several hundred dependent FP64 operations)
+    // factors are exact near 1 and -1 (the three functions one after another are
+    // several hundred dependent FP64 operations).  Where c rounds to -1 the
+    // second factor has nothing left: the sine of the double nearest pi; the
+    // dot product of two rounded unit vectors may also fall below -1.
     if (guard && mx < R(1e-5)) {
       ct = R(0.99999999995);   // cos, sin of 1e-5 (1 - 5e-11 + 4e-22, 1e-5 - 1.7e-16)
       st = R(9.9999999998333333e-06);
     } else {
       ct = nw[0] * n[0] + nw[1] * n[1] + nw[2] * n[2];
       st = sqrt((R(1) - ct) * (R(1) + ct));
+      if (ct <= R(-1)) {
+        ct = R(-1);
+        st = R(1.2246467991473532e-16);
+      }
     }
   }
   const R a1 = cc - sc * ct / st;

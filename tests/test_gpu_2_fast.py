@@ -10,9 +10,9 @@ import itertools
 import numpy as np
 import pytest
 
-from oracle.oracle import setup_workload as orc_setup
+from oracle.oracle import Oracle, setup_workload as orc_setup
 from symmetry_b200 import configs
-from symmetry_b200.lib import Lattice
+from symmetry_b200.lib import Lattice, setup_workload
 from tests.common import compare_masks, compare_particles, copy_oracle_to_lattice, rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -269,3 +269,62 @@ def test_fast_fp64_node_uncovered_beside_a_covered_one(rad, centre, up):
         compare_particles(o, L, 1, 1e-9)
         L.close()
     assert met
+
+
+def wall_layer(side, cita_deg):
+    """A noise-free layer along both wetting walls: red (side 1), whose wall
+    nodes' normals are exactly opposite to the walls', or blue (side -1),
+    exactly parallel."""
+    nx, ny, nz = 24, 10, 36
+    p = configs.config_params(nx, ny, nz, tau_r=0.9, sigma=5e-3, wall_x=True, cita_deg=cita_deg)
+    x = np.arange(nx, dtype=np.float64)[:, None, None]
+    phi = side * np.tanh(4.0 - np.minimum(x, nx - 1 - x)) * np.ones((nx, ny, nz))
+    o = Oracle(p)
+    o.call("set_walls")
+    o.init_phase(phi, np.ones_like(phi))
+    o.call("derivatives")
+    return p, o
+
+
+@pytest.mark.parametrize("cita_deg", [30.0, 60.0, 90.0, 120.0])
+@pytest.mark.parametrize("side", [1, -1])
+@pytest.mark.parametrize("storage", [0, 1, 2])
+def test_layer_along_a_wetting_wall(storage, side, cita_deg):
+    """Contact-angle rotation of a normal opposite or parallel to the wall's:
+    finite through 20 steps in every storage, derivatives (FP64 in every
+    storage) as the oracle's to the per-call bound 1e-12, and the fused FP64
+    step to 1e-10 after one step.  (Later steps multiply rounding: the
+    rotation of a normal within 1e-5 of the wall's divides by sin(1e-5).)"""
+    p, o = wall_layer(side, cita_deg)
+    p.storage = storage
+    L = Lattice(p)
+    copy_oracle_to_lattice(o, L)
+    L.call("derivatives")
+    for f in ("n_x", "n_y", "n_z", "gradx", "grady", "gradz"):
+        assert np.abs(L.get(f) - o.arr(f)).max() <= 1e-12, f
+    copy_oracle_to_lattice(o, L)
+    L.step(1)
+    o.step(1)
+    m = L.macros()
+    assert all(np.isfinite(v).all() for v in m.values())
+    if storage == 0:
+        fluid = o.arr("walls_all") == 0
+        r, b = o.arr("ri").sum(-1), o.arr("bi").sum(-1)
+        phi = np.where(fluid, (r - b) / (r + b), 0.0)
+        assert np.abs(m["rho_N"] - phi).max() <= 1e-10
+    L.step(19)
+    assert all(np.isfinite(v).all() for v in L.macros().values())
+    L.close()
+
+
+@pytest.mark.parametrize("storage", ["fp64", "fp16"])
+def test_noisy_thread_between_wetting_walls_stays_finite(storage):
+    """A served job between wetting walls far from its thread: noise clipped at
+    the pure phase leaves a few wall nodes' gradients exactly along the
+    normal, opposite to it."""
+    w = next(j.workload for j in configs.c5_jobs(storage=storage) if j.workload.name == "c5_0013")
+    assert w.params.wall_x and w.params.par == 0
+    L = setup_workload(w)
+    L.step(20)
+    assert all(np.isfinite(v).all() for v in L.macros().values())
+    L.close()
