@@ -919,6 +919,7 @@ inline int split_extent(int nx, int cap) {
 inline int best_extent(const std::vector<long long>& columns, const std::vector<int>& nx, int cap, long long slots) {
   int best = 1;
   double least = 1e300;
+  cap = std::min(cap, kMaxExtent);   // a caller's "no limit" may be any number
   for (int x = 1; x <= cap; x++) {
     double sum = 0.0, longest = 0.0;
     for (size_t i = 0; i < nx.size(); i++) {

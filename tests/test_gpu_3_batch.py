@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from symmetry_b200 import configs
-from symmetry_b200.lib import Batch, setup_workload
+from symmetry_b200.lib import Batch, Server, job_spec, setup_workload
 from symmetry_b200.params import particles_get
 
 pytestmark = pytest.mark.gpu
@@ -132,3 +132,28 @@ def test_batch_sizes_of_the_descriptor_tables(storage, n):
         assert np.array_equal(a.get("ri"), members[k].get("ri")), k
         assert np.array_equal(a.get("bi"), members[k].get("bi")), k
     B.close()
+
+
+def test_tile_extent_without_a_limit():
+    """An extent far beyond any domain (a caller's "no limit") costs nothing
+    and changes nothing, in a batch and in the server."""
+    w = configs.c1_thread(nx=20, ny=20, nz=64, radius=4.0)
+    alone, member = setup_workload(w), setup_workload(w)
+    alone.step(6)
+    B = Batch([member])
+    B.set_xchunk(0, 2 ** 31 - 1)
+    B.step(6)
+    assert B.xchunk(0) == 2 ** 31 - 1
+    assert np.array_equal(alone.get("ri"), member.get("ri"))
+    B.close()
+    done = []
+    for x in (None, 2 ** 31 - 1):
+        S = Server(slots=2, check_every=10)
+        for size_class in range(3):
+            if x:
+                S.set_xchunk(size_class, x)
+        i = S.submit(job_spec(w, 20))
+        S.run_until_idle()
+        done.append(S.result(i))
+        S.close()
+    assert done[0].status == done[1].status == 3 and done[0].steps == done[1].steps == 20
