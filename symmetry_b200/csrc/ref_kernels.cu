@@ -737,14 +737,18 @@ __global__ void __launch_bounds__(128, 4) k_collide_recolor(
     }
     return;
   }
+  auto sum = [](const double (&c)[19]) {
+    return c[0] + ((c[1] + c[2]) + (c[3] + c[4]) + (c[5] + c[6])) +
+           (((c[7] + c[10]) + (c[8] + c[9])) + ((c[11] + c[14]) + (c[12] + c[13])) + ((c[15] + c[18]) + (c[16] + c[17])));
+  };
+  // each colour's own sum: as a difference of densities the smaller one would
+  // carry the rounding of the larger (at EVAP_LIM 1e-9 of itself)
+  const double sr = sum(cr), sb = sum(f);
 #pragma unroll
   for (int i = 0; i < 19; i++) f[i] = cr[i] + f[i];
-  const double sr = cr[0] + ((cr[1] + cr[2]) + (cr[3] + cr[4]) + (cr[5] + cr[6])) +
-                    (((cr[7] + cr[10]) + (cr[8] + cr[9])) + ((cr[11] + cr[14]) + (cr[12] + cr[13])) +
-                     ((cr[15] + cr[18]) + (cr[16] + cr[17])));
   Moments<double> m;
   to_moments<double, double>(f, m);
-  const double rh = m.rho, sb = rh - sr;
+  const double rh = m.rho;
   double irho, su, sq;
   node_rates_fused<double>(T, rhoN[L], rh, irho, su, sq);
   const double n0 = nxv[L], n1 = nyv[L], n2 = nzv[L];

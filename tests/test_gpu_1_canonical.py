@@ -235,3 +235,35 @@ def test_reference_run_covers_and_refills_nodes():
         e = rel_l2(L.get(f), o.arr(f))
         assert e <= 1e-10, (f, e)
     compare_particles(o, L, 12, 1e-9)
+
+
+@pytest.mark.parametrize("minority", ["bi", "ri"])
+@pytest.mark.parametrize("steps", [1, 2])
+def test_reference_step_at_the_evaporation_limit(steps, minority):
+    """A colour of density 1e-8 (1 +- 1e-11) in one of density 0.05: whether it
+    is above EVAP_LIM decides if a node's minority colour empties, so each
+    colour's density must have its own 16 digits.  A wrong decision is off by
+    1e-8 w_i; a right one to the rounding of the majority's populations."""
+    p = params.reference_params(20, 24, 22)
+    p.par = 0
+    o = Oracle(p)
+    rng = np.random.default_rng(8)
+    shape = (p.nx, p.ny, p.nz)
+    small = 1e-8 * (1.0 + 1e-11 * rng.uniform(0.1, 1.0, shape) * rng.choice([-1.0, 1.0], shape))
+    large = 0.05 * (1.0 + 1e-3 * rng.uniform(-1.0, 1.0, shape))
+    w = np.array([1 / 3] + [1 / 18] * 6 + [1 / 36] * 12)
+    o.call("set_walls")
+    o.init_phase(np.ones(shape), np.full(shape, p.rho0))
+    o.call("derivatives")
+    f = w * (1.0 + 0.01 * rng.uniform(-1.0, 1.0, shape + (19,)))
+    f /= f.sum(-1, keepdims=True)
+    o.arr(minority)[...] = f * small[..., None]
+    o.arr("ri" if minority == "bi" else "bi")[...] = f * large[..., None]
+    L = Lattice(p)
+    copy_oracle_to_lattice(o, L)
+    o.step(1)
+    emptied = (o.arr(minority) == 0.0).mean()   # the oracle's first step decides both ways
+    assert 0.05 < emptied < 0.95
+    o.step(steps - 1)
+    L.step(steps)
+    assert np.abs(L.get(minority) - o.arr(minority)).max() <= 1e-14
