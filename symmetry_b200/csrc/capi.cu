@@ -1,4 +1,5 @@
 // capi.cu -- extern "C" entry points declared in include/symmetry.h.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -242,15 +243,28 @@ int canonical_piece(sym_handle* h, int piece) {
   return ref_curve(h);
 }
 
-// launches a piece, captured on its first use from the present arrangement of
-// the arrays (streaming leaves them permuted)
-int run_piece(sym_handle* h, int piece) {
+// The graph of a piece from the present arrangement of the arrays (streaming
+// leaves them permuted), captured on first use; the arrays are then arranged as
+// the piece leaves them.  Steps alone come back to two arrangements; a driver
+// that streams one colour between them meets up to 24 of each piece, so a handle
+// keeps the kMaxGraphs graphs used last.
+constexpr size_t kMaxGraphs = 48;
+int take_piece(sym_handle* h, int piece, cudaGraphExec_t* exec) {
   double** const cur[4] = {&h->ri, &h->bi, &h->ft, &h->ft2};
-  StepGraph* g = nullptr;
-  for (StepGraph& q : h->graphs)
-    if (q.piece == piece && q.from[0] == h->ri && q.from[1] == h->bi && q.from[2] == h->ft && q.from[3] == h->ft2)
-      g = &q;
-  if (!g) {
+  std::vector<StepGraph>& gs = h->graphs;   // the one used last at the end
+  size_t at = 0;
+  while (at < gs.size() && !(gs[at].piece == piece && gs[at].from[0] == h->ri && gs[at].from[1] == h->bi &&
+                             gs[at].from[2] == h->ft && gs[at].from[3] == h->ft2))
+    at++;
+  if (at < gs.size()) {
+    std::rotate(gs.begin() + at, gs.begin() + at + 1, gs.end());
+  } else {
+    if (gs.size() >= kMaxGraphs) {
+      // (calls end synchronised: the one dropped is not running)
+      cudaGraphExecDestroy(gs.front().exec);
+      cudaGraphDestroy(gs.front().graph);
+      gs.erase(gs.begin());
+    }
     StepGraph q;
     q.piece = piece;
     for (int k = 0; k < 4; k++) q.from[k] = *cur[k];
@@ -268,11 +282,11 @@ int run_piece(sym_handle* h, int piece) {
       if (q.graph) cudaGraphDestroy(q.graph);
       return e;
     }
-    h->graphs.push_back(q);
-    g = &h->graphs.back();
+    gs.push_back(q);
   }
-  if (int e = check_cuda(h, cudaGraphLaunch(g->exec, h->st), "graph launch")) return e;
-  for (int k = 0; k < 4; k++) *cur[k] = g->to[k];
+  const StepGraph& g = gs.back();
+  *exec = g.exec;
+  for (int k = 0; k < 4; k++) *cur[k] = g.to[k];
   return SYM_OK;
 }
 
@@ -288,9 +302,26 @@ int canonical_steps(sym_handle* h, int nsteps) {
     h->ft2 = nullptr;
     runs = false;
   }
-  for (int t = 0; t < nsteps; t++) {
-    const int piece = !runs ? STEP : (nsteps == 1 ? ONLY : (t == 0 ? HEAD : (t + 1 < nsteps ? MID : TAIL)));
-    if (int e = run_piece(h, piece)) return e;
+  auto piece = [&](int t) {
+    return !runs ? STEP : (nsteps == 1 ? ONLY : (t == 0 ? HEAD : (t + 1 < nsteps ? MID : TAIL)));
+  };
+  cudaGraphExec_t exec;
+  // every graph of the call exists before the first is launched: a failed
+  // capture leaves the state as it was (arrangements recur after 6 steps)
+  double* const first[4] = {h->ri, h->bi, h->ft, h->ft2};
+  int e = SYM_OK;
+  for (int t = 0; t < nsteps && !e; t++) {
+    e = take_piece(h, piece(t), &exec);
+    if (t == 6 && nsteps > 8) t += (nsteps - 8) / 6 * 6;
+  }
+  h->ri = first[0]; h->bi = first[1]; h->ft = first[2]; h->ft2 = first[3];
+  for (int t = 0; t < nsteps && !e; t++) {
+    e = take_piece(h, piece(t), &exec);
+    if (!e) e = check_cuda(h, cudaGraphLaunch(exec, h->st), "graph launch");
+  }
+  if (e) {
+    cudaStreamSynchronize(h->st);
+    return e;
   }
   return check_cuda(h, cudaStreamSynchronize(h->st), "step");
 }

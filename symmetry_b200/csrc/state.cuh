@@ -73,7 +73,7 @@ struct sym_handle {
   size_t red_len = 0;
   double* hred = nullptr;           // pinned host scalars
   symb200::FastState fast;
-  std::vector<symb200::StepGraph> graphs;   // canonical steps
+  std::vector<symb200::StepGraph> graphs;   // canonical steps, the one used last at the end
   size_t bytes = 0;
   // Every array the handle holds from creation is carved from one device
   // allocation (the slab): one cudaMalloc and one cudaFree per handle, no

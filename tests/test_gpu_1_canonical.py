@@ -267,3 +267,28 @@ def test_reference_step_at_the_evaporation_limit(steps, minority):
     o.step(steps - 1)
     L.step(steps)
     assert np.abs(L.get(minority) - o.arr(minority)).max() <= 1e-14
+
+
+@pytest.mark.parametrize("bounce", [0, 1])
+def test_reference_steps_between_streaming_calls(bounce):
+    """Streaming one colour leaves the arrays in another arrangement, and a
+    handle keeps a bounded number of captured steps: runs of 1 to 9 steps
+    between single streaming calls meet every arrangement of the arrays, more
+    than are kept.  Every run has the oracle's result, relative L2 1e-10."""
+    p = params.reference_params(9, 7, 8)
+    p.par, p.bounce = 0, bounce
+    o = Oracle(p)
+    rng = np.random.default_rng(4)
+    shape = (p.nx, p.ny, p.nz)
+    o.call("set_walls")
+    o.init_phase(0.02 * rng.uniform(-1.0, 1.0, shape), p.rho0 * (1.0 + 1e-3 * rng.uniform(-1.0, 1.0, shape)))
+    o.call("derivatives")
+    L = Lattice(p)
+    for k in range(60):
+        which, n = int(rng.integers(2)), int(rng.integers(1, 10))
+        copy_oracle_to_lattice(o, L)
+        for s in (o, L):
+            s.streaming(which)
+            s.step(n)
+        for f in ("ri", "bi", "rho", "rho_N"):
+            assert rel_l2(L.get(f), o.arr(f)) <= 1e-10, (k, f)
