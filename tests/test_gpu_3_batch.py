@@ -134,6 +134,53 @@ def test_batch_sizes_of_the_descriptor_tables(storage, n):
     B.close()
 
 
+@pytest.mark.parametrize("storage,rows", [("fp64", 8), ("fp32", 16), ("fp16", 16)])
+def test_long_marches_do_not_change_results(storage, rows):
+    """Long marches along x (the rings of phi, normals and reference pairs used
+    over and over, densities carried over many planes) are taken only where a
+    batch has columns enough to fill the GPU with them.  With one CTA per SM a
+    domain of 1,520 columns of 40 planes is marched whole; the domains beside
+    it (walls and sphere, and more planes than one tile) share its extent.
+    Exact: every extent gives the same populations bit for bit, and those of
+    the domains stepped alone with their own short tiles."""
+    big = configs.c1_thread(nx=40, ny=40 * rows, nz=1216, radius=9.0, storage=storage)
+    ws = [
+        configs.c2_wall_particle(nx=40, ny=27, nz=45, rad=4.0, centre=(20.3, 12.1, 16.0), z0=16.0, z1=32.0,
+                                 storage=storage),
+        configs.c1_thread(nx=83, ny=19, nz=37, radius=4.0, storage=storage),
+    ]
+    sms = 148
+
+    def columns(w):
+        return -(-w.params.ny // rows) * -(-w.params.nz // 32)
+
+    runs, fields = [], []
+    for cap in (64, 5):
+        members = [setup_workload(w) for w in [big] + ws]
+        B = Batch(members)
+        B.set_ctas_per_sm(1)
+        for i in range(len(members)):
+            B.set_xchunk(i, cap)
+        B.step(7)
+        info = B.info()
+        assert info["grid"] == sms
+        tiles = {64: [1, 1, 3], 5: [8, 8, 17]}[cap]   # of 40, 40 and 83 planes
+        assert info["tiles"] == sum(t * columns(w) for t, w in zip(tiles, [big] + ws)), info
+        runs.append([state(m) for m in members[1:]])
+        fields.append(members[0].macros())
+        B.close()
+        for m in members:
+            m.close()
+    for k in fields[0]:
+        assert np.array_equal(fields[0][k], fields[1][k]), k
+    for w, long, short in zip(ws, *runs):
+        L = setup_workload(w)
+        L.step(7)
+        for a, b, c in zip(long, short, state(L)):
+            if a is not None:
+                assert np.array_equal(a, b) and np.array_equal(a, c), w.name
+
+
 def test_tile_extent_without_a_limit():
     """An extent far beyond any domain (a caller's "no limit") costs nothing
     and changes nothing, in a batch and in the server."""
