@@ -50,7 +50,7 @@ struct DomainDesc {
 };
 
 struct TileEntry {
-  int dom, z0, y0, xa, xb, cost, r0, r1;
+  int dom, z0, y0, xa, xb, cost;
 };
 
 
@@ -68,18 +68,15 @@ __global__ void __launch_bounds__(256) k_phase_batch(const DomainDesc* __restric
     phase_node<S, false>(D.P, D.pd, (const S*)D.pin, (R*)D.phic, D.walls_all, D.rr_old, D.rr_new, L);
 }
 
-template <typename S>
 __global__ void __launch_bounds__(256) k_finalize_batch(const DomainDesc* __restrict__ descs,
                                                         const int2* __restrict__ blk) {
-  using R = typename Codec<S>::R;
-  using AT = typename Acc<R>::T;
   const int2 e = blk[blockIdx.x];
   const DomainDesc& D = descs[e.x];
   const long long L = (long long)e.y * 256 + threadIdx.x;
   if (D.solid)
-    finalize_nodes<S, true, 1>(D.P, D.pd, (AT*)D.acc, (R*)D.phic, D.walls_all, D.rr_new, D.status, L);
+    finalize_nodes<true, 1>(D.P, D.pd, (Acc::T*)D.acc, (double*)D.phic, D.walls_all, D.status, L);
   else
-    finalize_nodes<S, false, 1>(D.P, D.pd, (AT*)D.acc, (R*)D.phic, D.walls_all, D.rr_new, D.status, L);
+    finalize_nodes<false, 1>(D.P, D.pd, (Acc::T*)D.acc, (double*)D.phic, D.walls_all, D.status, L);
 }
 
 // What the collide kernel reads of one domain.
@@ -93,7 +90,7 @@ struct TileDesc {
   const sym_particles* Sp;
   double* ffi;
   const Ref* rr_old;
-  typename Acc<typename Codec<S>::R>::T* acc;
+  Acc::T* acc;
   int* status;
   const CUtensorMap *tm_phi, *tm_ref;
   int solid;
@@ -268,7 +265,7 @@ TileDesc<S> tile_desc(const DomainDesc& d) {
   t.pin = (const S*)d.pin; t.pnext = (S*)d.pnext;
   t.walls = d.walls; t.walls_all = d.walls_all; t.pout = d.pout;
   t.Sp = d.Sp; t.ffi = d.ffi; t.rr_old = d.rr_old;
-  t.acc = (typename Acc<R>::T*)d.acc;
+  t.acc = (Acc::T*)d.acc;
   t.status = d.status; t.tm_phi = d.tm_phi; t.tm_ref = d.tm_ref; t.solid = d.solid;
   return t;
 }
@@ -298,7 +295,7 @@ template <typename S>
 int enqueue_batch_step(sym_batch* b, int k, cudaEvent_t* ev) {
   if (ev) cudaEventRecord(ev[0], b->st);
   if constexpr (kAccumulate<S>)
-    k_finalize_batch<S><<<(unsigned)b->nblocks, 256, 0, b->st>>>(b->d_desc[k], b->d_blk);
+    k_finalize_batch<<<(unsigned)b->nblocks, 256, 0, b->st>>>(b->d_desc[k], b->d_blk);
   else
     k_phase_batch<S><<<(unsigned)b->nblocks, 256, 0, b->st>>>(b->d_desc[k], b->d_blk);
   if (ev) cudaEventRecord(ev[1], b->st);

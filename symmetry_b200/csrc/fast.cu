@@ -61,10 +61,7 @@ float2* rr_new(sym_handle* h, int pc) { return h->fast.rref[pc]; }
 
 bool has_solids(const sym_handle* h) { return h->dp.par > 0 || h->dp.wall_x; }
 
-template <typename S>
-typename Acc<typename Codec<S>::R>::T* accbuf(sym_handle* h) {
-  return reinterpret_cast<typename Acc<typename Codec<S>::R>::T*>(h->fast.acc);
-}
+Acc::T* accbuf(sym_handle* h) { return reinterpret_cast<Acc::T*>(h->fast.acc); }
 
 // the particle and wall work of this handle's fused steps (sparse.cu); built
 // outside any stream capture
@@ -93,11 +90,9 @@ int enqueue_step(sym_handle* h, int cur, int pc, cudaEvent_t* ev) {
   if constexpr (kAccumulate<S>) {
     const unsigned fin_blocks = blocks_for(P.N, 256 * kFinalizeNPT);
     if (solid)
-      k_finalize<S, true><<<fin_blocks, 256, 0, h->st>>>(P, pd, accbuf<S>(h), phic, h->walls_all, rr_new(h, pc),
-                                                         h->fast.status);
+      k_finalize<true><<<fin_blocks, 256, 0, h->st>>>(P, pd, accbuf(h), phic, h->walls_all, h->fast.status);
     else
-      k_finalize<S, false><<<fin_blocks, 256, 0, h->st>>>(P, pd, accbuf<S>(h), phic, h->walls_all, rr_new(h, pc),
-                                                          h->fast.status);
+      k_finalize<false><<<fin_blocks, 256, 0, h->st>>>(P, pd, accbuf(h), phic, h->walls_all, h->fast.status);
   } else {
     if (solid)
       k_phase<S, true><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, pin_, phic, h->walls_all, rr_old(h, pc),
@@ -122,10 +117,10 @@ int enqueue_step(sym_handle* h, int cur, int pc, cudaEvent_t* ev) {
   if (ev) cudaEventRecord(ev[2], h->st);
   if (solid)
     k_collide<S, true><<<grid, kTPB, shm, h->st>>>(tile_params<R>(P), pd, pin_, pnext, h->walls, h->walls_all, h->pout, h->dpart,
-                                                   h->ffi, rr_old(h, pc), accbuf<S>(h), h->fast.status, tp, tr, xc);
+                                                   h->ffi, rr_old(h, pc), accbuf(h), h->fast.status, tp, tr, xc);
   else
     k_collide<S, false><<<grid, kTPB, shm, h->st>>>(tile_params<R>(P), pd, pin_, pnext, h->walls, h->walls_all, h->pout, h->dpart,
-                                                    h->ffi, rr_old(h, pc), accbuf<S>(h), h->fast.status, tp, tr, xc);
+                                                    h->ffi, rr_old(h, pc), accbuf(h), h->fast.status, tp, tr, xc);
   if (int e = sparse_enqueue_post(h->fast.sparse, cur, h->st)) return set_error(h, e, "interpolated bounce-back");
   if (ev) cudaEventRecord(ev[3], h->st);
   return check_cuda(h, cudaGetLastError(), "fast step");
@@ -274,18 +269,18 @@ int fast_import(sym_handle* h) {
   switch (F.storage) {
     case SYM_STORE_FP64:
       k_import_pops<double><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, h->ri, h->bi, popbuf<double>(h, 0), nullptr,
-                                                                accbuf<double>(h), F.status);
+                                                                accbuf(h), F.status);
       k_import_phi<double><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, h->rhoN, F.phi[1]);
       break;
     case SYM_STORE_FP32:
       k_import_pops<float><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, h->ri, h->bi, popbuf<float>(h, 0), nullptr,
-                                                               accbuf<float>(h), F.status);
+                                                               accbuf(h), F.status);
       k_import_phi<float><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, h->rhoN, F.phif[1]);
       break;
     default:
       // after import pc = 0: the next phase decodes with rref[1]
       k_import_pops<__half><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, h->ri, h->bi, popbuf<__half>(h, 0), F.rref[1],
-                                                                accbuf<__half>(h), F.status);
+                                                                accbuf(h), F.status);
       k_import_phi<float><<<blocks_for(P.N), 256, 0, h->st>>>(P, pd, h->rhoN, F.phif[1]);
   }
   if (int e = sparse_links_build(h, h->st)) return set_error(h, e, "momentum link lists");

@@ -184,26 +184,17 @@ __device__ __forceinline__ Ref ref_rest(const DevParams& P) { return make_float2
 // step's phase field (calmacros) reads 2 numbers per node instead of all 38
 // populations.  Integer addition is associative, so the totals do not depend
 // on the order in which the tiles' atomic adds land: the accumulated densities
-// are deterministic.  FP64 storage: 64-bit integers in units of 2^-52
-// (|rho| < 1024); FP32 arithmetic: 32-bit integers in units of 2^-26
-// (|rho| < 31).  A value outside that range or not finite sets the domain's
-// status word, and the next phase field is written as NaN (the NaN test of the
-// stop rule then retires the run).
-template <typename R>
-struct Acc;
-template <>
-struct Acc<double> {
+// are deterministic.  64-bit integers in units of 2^-52 (|rho| < 1024).  The
+// share that each of three planes sends to a node is rounded by itself, three
+// roundings of 1.1e-16 where one of the whole sum would do: the price of totals
+// that do not depend on the tiles' x extents.  A value outside the range or not
+// finite sets the domain's status word, and the next phase field is written as
+// NaN (the NaN test of the stop rule then retires the run).
+struct Acc {
   using T = unsigned long long;
   __device__ __forceinline__ static T fix(double v) { return (T)__double2ll_rn(v * 0x1p52); }
   __device__ __forceinline__ static double val(T a) { return (double)(long long)a * 0x1p-52; }
   __device__ __forceinline__ static bool ok(double v) { return fabs(v) < 1024.0; }
-};
-template <>
-struct Acc<float> {
-  using T = unsigned int;
-  __device__ __forceinline__ static T fix(float v) { return (T)__float2int_rn(v * 0x1p26f); }
-  __device__ __forceinline__ static float val(T a) { return (float)(int)a * 0x1p-26f; }
-  __device__ __forceinline__ static bool ok(float v) { return fabsf(v) < 31.0f; }
 };
 // Whether the collide kernel of storage S accumulates the next step's colour
 // densities (the phase field then reads 2 values per node) or the phase field
@@ -216,17 +207,11 @@ struct Acc<float> {
 template <typename S>
 constexpr bool kAccumulate = sizeof(S) == 8;
 
-// v in fixed point; an out-of-range value sets *status and counts as nothing
-template <typename R>
-__device__ __forceinline__ typename Acc<R>::T acc_fix(R v, int* status) {
-  if (Acc<R>::ok(v)) return Acc<R>::fix(v);
-  atomicOr(status, 1);
-  return 0;
-}
-// add v to accumulator p (a reduction: nothing is returned)
-template <typename R>
-__device__ __forceinline__ void acc_add(typename Acc<R>::T* p, R v, int* status) {
-  atomicAdd(p, acc_fix<R>(v, status));
+// add v to accumulator p (a reduction: nothing is returned); an out-of-range
+// value sets *status and counts as nothing
+__device__ __forceinline__ void acc_add(Acc::T* p, double v, int* status) {
+  if (Acc::ok(v)) atomicAdd(p, Acc::fix(v));
+  else atomicOr(status, 1);
 }
 
 template <typename F, int... Is>
@@ -298,24 +283,19 @@ __global__ void __launch_bounds__(256) k_phase(DevParams P, Pad pd, const S* __r
   phase_node<S, SOLID>(P, pd, pops, phi, walls_all, rr_old, rr_new, blockIdx.x * 256LL + threadIdx.x);
 }
 
-// From the accumulated colour densities (the steady-state phase field):
+// From the accumulated colour densities (FP64, the steady-state phase field):
 // phi = (rhoR - rhoB) / rho on fluid nodes, 0 on solid nodes, written with its
 // periodic ghost images; the accumulators are cleared for the collide kernel
-// of this step.  A storage with references (kRef) would also record the
-// node's (rho, red fraction) in rr_new, as phase_node does.
+// of this step.
 // Nodes L0, L0 + 256, ..., L0 + 256 (NPT-1) per thread: every load of all of
 // them is issued before the first store, so a thread keeps 2 NPT accumulator
 // reads in flight (nothing waits on a store).
-template <typename S, bool SOLID, int NPT>
-__device__ __forceinline__ void finalize_nodes(const DevParams& P, const Pad& pd,
-                                               typename Acc<typename Codec<S>::R>::T* __restrict__ acc,
-                                               typename Codec<S>::R* __restrict__ phi,
-                                               const int32_t* __restrict__ walls_all, Ref* __restrict__ rr_new,
+template <bool SOLID, int NPT>
+__device__ __forceinline__ void finalize_nodes(const DevParams& P, const Pad& pd, Acc::T* __restrict__ acc,
+                                               double* __restrict__ phi, const int32_t* __restrict__ walls_all,
                                                const int* __restrict__ status, long long L0) {
-  using R = typename Codec<S>::R;
-  using A = Acc<R>;
   const int bad = *status;
-  typename A::T ar[NPT], ab[NPT];
+  Acc::T ar[NPT], ab[NPT];
   bool solid[NPT];
 #pragma unroll
   for (int k = 0; k < NPT; k++) {
@@ -337,29 +317,22 @@ __device__ __forceinline__ void finalize_nodes(const DevParams& P, const Pad& pd
     // 32-bit index arithmetic (the fused path keeps 38*N < 2^32)
     const unsigned Lu = (unsigned)L, q = Lu / (unsigned)P.nz;
     const int z = (int)(Lu - q * (unsigned)P.nz), x = (int)(q / (unsigned)P.ny), y = (int)(q - (unsigned)x * P.ny);
-    const R sr = A::val(ar[k]), sb = A::val(ab[k]);
-    R v = R(0);
-    Ref nref = ref_rest(P);
-    if (!solid[k]) {
-      v = qdiv<R>(sr - sb, sr + sb);
-      nref = ref_pair(float(sr), float(sb));
-    }
-    if (bad) v = R(NAN);
-    phi_store<R>(P, pd, phi, x, y, z, v);
-    if constexpr (Codec<S>::kRef) phi_store<Ref>(P, pd, rr_new, x, y, z, nref);
+    const double sr = Acc::val(ar[k]), sb = Acc::val(ab[k]);
+    double v = solid[k] ? 0.0 : (sr - sb) / (sr + sb);
+    if (bad) v = NAN;
+    phi_store<double>(P, pd, phi, x, y, z, v);
   }
 }
 
 // nodes finalised per thread by the single-domain kernel
 constexpr int kFinalizeNPT = 4;
 
-template <typename S, bool SOLID>
-__global__ void __launch_bounds__(256) k_finalize(DevParams P, Pad pd, typename Acc<typename Codec<S>::R>::T* acc,
-                                                  typename Codec<S>::R* __restrict__ phi,
-                                                  const int32_t* __restrict__ walls_all, Ref* __restrict__ rr_new,
+template <bool SOLID>
+__global__ void __launch_bounds__(256) k_finalize(DevParams P, Pad pd, Acc::T* acc, double* __restrict__ phi,
+                                                  const int32_t* __restrict__ walls_all,
                                                   const int* __restrict__ status) {
-  finalize_nodes<S, SOLID, kFinalizeNPT>(P, pd, acc, phi, walls_all, rr_new, status,
-                                         blockIdx.x * (256LL * kFinalizeNPT) + threadIdx.x);
+  finalize_nodes<SOLID, kFinalizeNPT>(P, pd, acc, phi, walls_all, status,
+                                      blockIdx.x * (256LL * kFinalizeNPT) + threadIdx.x);
 }
 
 // ---- wetting rotation of a node normal (derivatives :535-587) ---------------------
@@ -488,11 +461,11 @@ __device__ __forceinline__ void collide_tile(const TileParams<double>& P, const 
                                              const int32_t* __restrict__ walls_all,
                                              const int32_t* __restrict__ pout,
                                              const sym_particles* __restrict__ Sp, double* __restrict__ ffi,
-                                             Acc<double>::T* acc, int* status, const CUtensorMap* tm_phi,
+                                             Acc::T* acc, int* status, const CUtensorMap* tm_phi,
                                              int z0, int y0, int xa, int xb, Smem& sm, unsigned& nload,
                                              bool solid_rt = true) {
   using R = double;
-  using A = Acc<double>;
+  using A = Acc;
   using AT = A::T;
   constexpr int BY = kBY<double>, kRow = BZ + 4;
   const bool SOLIDX = SOLID && solid_rt;
@@ -1057,7 +1030,7 @@ __device__ __forceinline__ void refill_import_node(const DevParams& P, const Pad
 // colour densities (the rest pair where both are 0: solid or empty nodes)
 template <typename S>
 __global__ void k_import_pops(DevParams P, Pad pd, const double* __restrict__ ri, const double* __restrict__ bi,
-                              S* pops, Ref* rr, typename Acc<typename Codec<S>::R>::T* acc, int* status) {
+                              S* pops, Ref* rr, Acc::T* acc, int* status) {
   using R = typename Codec<S>::R;
   const long long L = blockIdx.x * 256LL + threadIdx.x;
   if (L >= P.N) return;
@@ -1081,11 +1054,10 @@ __global__ void k_import_pops(DevParams P, Pad pd, const double* __restrict__ ri
   });
   // the accumulators the first phase field after the import reads (storages
   // that accumulate)
-  using A = Acc<R>;
-  if (acc) {
-    if (!A::ok(sr) || !A::ok(sb)) atomicOr(status, 1);
-    acc[L] = A::ok(sr) ? A::fix(sr) : 0;
-    acc[L + P.N] = A::ok(sb) ? A::fix(sb) : 0;
+  if constexpr (kAccumulate<S>) {
+    if (!Acc::ok(sr) || !Acc::ok(sb)) atomicOr(status, 1);
+    acc[L] = Acc::ok(sr) ? Acc::fix(sr) : 0;
+    acc[L + P.N] = Acc::ok(sb) ? Acc::fix(sb) : 0;
   }
 }
 template <typename S>

@@ -493,7 +493,7 @@ template <typename S, bool SOLID>
 __device__ __forceinline__ void collide_any(const TileParams<typename Codec<S>::R>& P, const Pad& pd, const S* pin_, S* pout_,
                                             const int32_t* walls, const int32_t* walls_all, const int32_t* pout,
                                             const sym_particles* Sp, double* ffi, const Ref* rr_old,
-                                            typename Acc<typename Codec<S>::R>::T* acc, int* status,
+                                            Acc::T* acc, int* status,
                                             const CUtensorMap* tm_phi, const CUtensorMap* tm_ref, int z0, int y0, int xa,
                                             int xb, TileSmem<S>& sm, unsigned& nload, bool solid_rt = true) {
   if constexpr (std::is_same<S, double>::value)
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(kTPB, collide_ctas<S>())
     k_collide(const __grid_constant__ TileParams<typename Codec<S>::R> P, Pad pd, const S* __restrict__ pin_, S* __restrict__ pout_,
               const int32_t* __restrict__ walls, const int32_t* __restrict__ walls_all,
               const int32_t* __restrict__ pout, const sym_particles* __restrict__ Sp, double* __restrict__ ffi,
-              const Ref* __restrict__ rr_old, typename Acc<typename Codec<S>::R>::T* acc, int* status,
+              const Ref* __restrict__ rr_old, Acc::T* acc, int* status,
               const __grid_constant__ CUtensorMap tm_phi, const __grid_constant__ CUtensorMap tm_ref, int xchunk) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   TileSmem<S>& sm = smem_view<S>(smem_raw);

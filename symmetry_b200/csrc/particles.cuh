@@ -101,16 +101,8 @@ __device__ __forceinline__ bool inside(const DevParams& P, const sym_particles* 
   const double d = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
   return d <= r2;
 }
-__device__ __forceinline__ void walls_mark_node(const DevParams& P, const sym_particles* S, int pp, double r2, int x,
-                                                int y, int z, int32_t* walls, int32_t* walls_all) {
-  if (inside(P, S, pp, r2, x, y, z)) {
-    const long long L = lin(P, x, y, z);
-    walls[L] = pp;
-    walls_all[L] = 10;
-  }
-}
-// the same where all particles are marked at once: a node inside several keeps
-// the last one's mark
+// all particles are marked at once: a node inside several keeps the last one's
+// mark
 __device__ __forceinline__ void walls_mark_last(const DevParams& P, const sym_particles* S, int pp, double r2, int x,
                                                 int y, int z, int32_t* walls, int32_t* walls_all) {
   if (!inside(P, S, pp, r2, x, y, z)) return;

@@ -378,10 +378,9 @@ __global__ void __launch_bounds__(kT) k_sp_curve2(const SpDom* __restrict__ doms
     dr += vr - (double)hr;
     db += vb - (double)hb;
   });
-  using AT = typename Acc<R>::T;
   if (kAccumulate<S> && (dr != 0.0 || db != 0.0)) {
-    acc_add<R>((AT*)D.acc + L, R(dr), D.status);
-    acc_add<R>((AT*)D.acc + P.N + L, R(db), D.status);
+    acc_add((Acc::T*)D.acc + L, dr, D.status);
+    acc_add((Acc::T*)D.acc + P.N + L, db, D.status);
   }
 }
 
