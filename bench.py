@@ -469,8 +469,8 @@ def main():
                     help="auxiliary measurements at N=1 (comma list; 'none' for the timed region only)")
     ap.add_argument("--domains", type=int, default=96, help="mix: the first D domains of the manifest "
                                                              "(smaller cases for profiler captures)")
-    ap.add_argument("--xchunk", type=int, default=0, help="mix: fixed tile x extent for every domain instead of "
-                                                           "the autotuner (profiler captures)")
+    ap.add_argument("--xchunk", type=int, default=0, help="mix: most x planes per tile for every domain instead "
+                                                           "of the autotuner's (profiler captures)")
     ap.add_argument("--serve-seconds", type=float, default=60.0)
     ap.add_argument("--serve-cap", type=int, default=6000)
     ap.add_argument("--serve-wall", type=float, default=120.0)

@@ -143,7 +143,8 @@ const char* sym_last_error(const sym_handle* h);
  * moment matrix m[r*19+c] = M(r,c) of the data statement (:105-123).  Any
  * pointer may be NULL. */
 int sym_lattice_tables(int32_t tables[7 * 19], double wi[19], double m[19 * 19]);
-/* Device bytes the handle holds (state + fast-path buffers). */
+/* Device bytes the handle holds from creation (state + fast-path buffers).  Not
+ * counted: what the first sym_step of a REFERENCE handle adds (see there). */
 int sym_footprint(const sym_params* p, size_t* bytes);
 
 /* ---- state transfer (Fortran layout on the host) ------------------------ */
@@ -228,11 +229,13 @@ int sym_movement(sym_handle* h);          /* movement         Source1.f90:1263-1
 int sym_refilling(sym_handle* h);         /* refilling        Source1.f90:1351-1418 */
 
 /* One loop body of main (Source1.f90:216-251, output gate excluded), nsteps
- * times.  REFERENCE mode runs the reference's order with passes over the
- * populations merged (halfway bounce-back; the first call allocates a second
- * streaming target of 152 bytes per node, and where there is no room for it the
- * subroutine kernels above run one by one); CONFIG mode runs the fused fast path
- * in the handle's storage mode. */
+ * times.  REFERENCE mode runs the reference's order; with the halfway
+ * bounce-back passes over the populations are merged, and their arithmetic is
+ * the fused path's, with fused multiply-adds: the results differ from the
+ * subroutines called one after another by rounding.  The first such call
+ * allocates 153 bytes per node more (a second streaming target of 152 and one
+ * mark); where there is no room for them the subroutine kernels above run one
+ * by one.  CONFIG mode runs the fused fast path in the handle's storage mode. */
 int sym_step(sym_handle* h, int nsteps);
 /* sym_step with CUDA events recorded on the handle's stream (CONFIG mode).
  * use_graph=0: eager launches, ms[0]=whole region, ms[1]=phase-field kernel,
@@ -244,10 +247,10 @@ int sym_step_timed(sym_handle* h, int nsteps, int use_graph, double ms[4]);
  * No counterpart in the reference (it runs one domain).  A batch references
  * existing handles (same device, CONFIG mode, same storage) and steps them in
  * lockstep: one CUDA graph per step containing one phase-field launch for all
- * domains, the particle and wall work of all domains (one launch per
- * subroutine over a (domain, particle, block) table), and one persistent
- * collide launch whose CTAs pull 32x8xX tiles of any domain from a work-tile
- * table (largest first).  Results per domain are identical to sym_step on that
+ * domains, the particle and wall work of all domains (six launches over
+ * (domain, particle, block) tables), and one persistent collide launch whose
+ * CTAs pull 32x8xX (FP64) or 32x16xX (FP32, 16-bit) tiles of any domain from a
+ * work-tile table (largest first).  Results per domain are identical to sym_step on that
  * domain alone, whatever the tiles' x extents.  Member handles stay usable on
  * their own; the batch rebuilds its graphs when a member was stepped or read
  * back outside it. */
@@ -258,14 +261,15 @@ const char* sym_batch_last_error(const sym_batch* b);
 int sym_batch_step(sym_batch* b, int nsteps);
 /* nsteps graph steps bracketed by CUDA events on the batch stream; *ms = elapsed. */
 int sym_batch_step_timed(sym_batch* b, int nsteps, double* ms);
-/* The most x planes per collide tile of one domain (default 32); shorter tiles
- * are taken when the batch has too few to fill the GPU.  Never changes a result. */
+/* The most x planes per collide tile of one domain (default 32; more than 64
+ * counts as 64); shorter tiles are taken when the batch has too few to fill the
+ * GPU.  Never changes a result. */
 int sym_batch_set_xchunk(sym_batch* b, int domain, int xchunk);
 int sym_batch_get_xchunk(sym_batch* b, int domain, int* xchunk);
 /* Resident collide CTAs per SM of the persistent launch (1 .. the most that
  * fit; default the most): grid = per_sm x SM count. */
 int sym_batch_set_ctas_per_sm(sym_batch* b, int per_sm);
-/* Picks the tile x extent per size class (nx <= 32, <= 48, larger) from
+/* Picks the largest tile x extent per size class (nx <= 32, <= 48, larger) from
  * {8,12,16,24,32,64}, then the resident CTAs per SM, by timing; the trial steps
  * advance every domain (*steps_taken). */
 int sym_batch_autotune(sym_batch* b, int trial_steps, int* steps_taken);
@@ -349,8 +353,9 @@ int sym_server_submit(sym_server* s, const sym_job_spec* spec, int64_t* id);
  * after the device work of the round; *running and *pending may be NULL. */
 int sym_server_tick(sym_server* s, int max_steps, int* running, int* pending);
 int sym_server_result(sym_server* s, int64_t id, sym_job_result* out);
-/* Tile x extent used for jobs of one size class (0: nx <= 32, 1: <= 48,
- * 2: larger) in the batches the server builds (default 32). */
+/* The most x planes per tile (as sym_batch_set_xchunk) for jobs of one size
+ * class (0: nx <= 32, 1: <= 48, 2: larger) in the batches the server builds
+ * (default 32). */
 int sym_server_set_xchunk(sym_server* s, int size_class, int xchunk);
 /* out[0] node updates, [1] device milliseconds of the batch steps, [2] jobs
  * done, [3] jobs failed, [4] running, [5] pending, [6] resident footprint

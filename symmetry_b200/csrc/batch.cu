@@ -6,15 +6,16 @@
 //                     counts): from the colour densities the previous collide
 //                     accumulated (FP64) or from the populations (16-bit, FP32);
 //   sparse work       particle coupling and pin fill of every domain with
-//                     solids, one launch per subroutine for all of them
-//                     (sparse.cu);
+//                     solids, six launches for all of them (sparse.cu);
 //   k_collide_batch   one persistent launch (one CTA per SM slot) whose CTAs
-//                     take 32x8xX tiles of any domain from a work-tile table
-//                     through an atomic counter, largest tiles first, so
-//                     domains of uneven size share the GPU without tails.
+//                     take 32x8xX (FP64) or 32x16xX (FP32, 16-bit) tiles of any
+//                     domain from a work-tile table through an atomic counter,
+//                     largest tiles first, so domains of uneven size share the
+//                     GPU without tails.
 // Each domain keeps its own buffers and parity; two graphs (one per parity
-// of the domain buffers) alternate.  The x extent X of the tiles is chosen per
-// size class by sym_batch_autotune.
+// of the domain buffers) alternate.  The x extent X of the tiles comes from an
+// estimate over the whole batch (best_extent), limited per domain by
+// sym_batch_set_xchunk or per size class by sym_batch_autotune.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
@@ -103,7 +104,11 @@ struct TileDesc {
 // read a tile's descriptor from global memory into shared memory.
 template <typename S>
 constexpr int kParamDomains = 32 * 1000 / (int)sizeof(TileDesc<S>) < 128 ? 32 * 1000 / (int)sizeof(TileDesc<S>) : 128;
-constexpr int kFewDomains = 16;   // a smaller table, copied with each launch
+// A smaller table for few domains: the parameters are copied with each launch
+// (with the large one alone, per step: 1 domain of 16x16x48 FP64 20.3 -> 20.6 us
+// and 16-bit 18.6 -> 19.8, 6 domains 38.9 -> 41.2 and 27.1 -> 27.6, 16 domains
+// 170 -> 174 and 81 -> 84).
+constexpr int kFewDomains = 16;
 template <typename S, int N>
 struct DescTable {
   TileDesc<S> d[N];
@@ -565,8 +570,8 @@ int sym_batch_step_timed(sym_batch* b, int nsteps, double* ms) {
   return rc;
 }
 
-// Choose the tile x extent per size class (domains grouped by nx: <=32, <=48,
-// larger) from {8, 12, 16, 24, 32, 64}, then the persistent collide grid
+// Choose the largest tile x extent per size class (domains grouped by nx: <=32,
+// <=48, larger) from {8, 12, 16, 24, 32, 64}, then the persistent collide grid
 // (resident CTAs per SM, from the most that fit down to 1), each by timing trial_steps
 // graph steps per candidate.  The trial steps advance every domain;
 // *steps_taken reports how many.

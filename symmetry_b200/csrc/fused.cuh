@@ -870,8 +870,9 @@ __device__ __forceinline__ void collide_tile(const TileParams<double>& P, const 
   if (!fine) atomicOr(status, 1);
 }
 
-// Plane times a tile spends before its first plane (five plane loads and the
-// normals of two planes).
+// Plane times a tile is charged for what comes before its first plane (five
+// plane loads and the normals of two planes).  A CTA by itself spends two of
+// any storage, of which others on the SM hide about half.
 constexpr double kTileLead = 1.0;
 // x extent of a tile whose column of x planes is nx long, at most `cap`: the
 // column in equal parts
@@ -884,11 +885,12 @@ inline int split_extent(int nx, int cap) {
 // footprints) of nx[i] planes each on `slots` resident CTAs: the one with the
 // least estimated time, in planes: the work of all slots evenly shared plus
 // half a tile of tail, or one whole tile when there are fewer tiles than
-// slots.  A CTA needs about 6 us for an FP64 plane (2.8 FP32, 4.9 16-bit)
-// whether the GPU is full or not, so a domain of few columns is bound by the
-// length of one march.  Measured per step, extent 32 against this rule's:
-// 32x32x96 FP64 209 -> 29 us (3 planes), 53x53x374 269 -> 210, 64x64x128
-// 219 -> 111, FP32 113 -> 51, 16-bit 172 -> 57; 256x256x256 keeps 32.
+// slots.  A CTA needs about 6.6 us for an FP64 plane of 8 rows (6.0 FP32, 5.3
+// 16-bit, 16 rows) whether the GPU is full or not, so a domain of few columns is
+// bound by the length of one march.  Measured per step, extent 32 against this
+// rule's: 32x32x96 FP64 243 -> 28.5 us (2 planes), FP32 205 -> 20.5 (1), 16-bit
+// 184 -> 20.5 (1); 64x64x128 FP64 281 -> 102 (4), FP32 222 -> 59 (3), 16-bit
+// 198 -> 51 (3); 53x53x374 FP64 263 -> 194 (6); 256x256x512 FP64 keeps 32.
 inline int best_extent(const std::vector<long long>& columns, const std::vector<int>& nx, int cap, long long slots) {
   int best = 1;
   double least = 1e300;
