@@ -699,6 +699,10 @@ __global__ void __launch_bounds__(TPB) k_step_macros(DevParams P, const sym_part
 // 366 us at 152^3).  PULL: the populations of nodes that k_step_macros did not
 // keep are streamed here from (rs, bs), without curve, which they were not part
 // of; a node that has become solid since gets them unchanged.
+// A node uncovered without being refilled (it is next to no particle any more: one
+// that moved by more than a node) collides what calmacros left of a solid node:
+// the totals fi of the step that covered it, rho0, no velocity, its old colour
+// densities.
 template <bool FULL, bool PULL>
 __global__ void __launch_bounds__(128, 4) k_collide_recolor(
     DevParams P, const __grid_constant__ TileParams<double> T, const int32_t* __restrict__ walls_all,
@@ -706,7 +710,8 @@ __global__ void __launch_bounds__(128, 4) k_collide_recolor(
     const double* __restrict__ nyv, const double* __restrict__ nzv, const double* __restrict__ gx,
     const double* __restrict__ gy, const double* __restrict__ gz, const double* __restrict__ rhoN, double* ux,
     double* uy, double* uz, double* fi, double* ffi, double* ri, double* bi, const double* __restrict__ rs,
-    const double* __restrict__ bs, const unsigned char* __restrict__ kept) {
+    const double* __restrict__ bs, const unsigned char* __restrict__ kept, const int32_t* __restrict__ walls_old,
+    const double* __restrict__ rhoR, const double* __restrict__ rhoB) {
   using namespace fused;
   const unsigned t = blockIdx.x * 128u + threadIdx.x;
   const unsigned rz = P.hi[2] - P.lo[2] + 1, ry = P.hi[1] - P.lo[1] + 1;
@@ -716,7 +721,8 @@ __global__ void __launch_bounds__(128, 4) k_collide_recolor(
   const long long L = lin(P, x, y, z), N = P.N;
   const bool solid = walls_all[L] > 0;
   const bool pull = PULL && !kept[L];
-  if (solid && !pull) return;
+  const bool covered = !FULL && solid && walls_old[L] <= 0;
+  if (solid && !pull && !covered) return;
   const int pp = pout[L];
   const bool fl = flag[L] != 0;
   double f[19], cr[19];
@@ -732,8 +738,11 @@ __global__ void __launch_bounds__(128, 4) k_collide_recolor(
   if (solid) {
 #pragma unroll
     for (int i = 0; i < 19; i++) {
-      ri[i * N + L] = cr[i];
-      bi[i * N + L] = f[i];
+      if (pull) {
+        ri[i * N + L] = cr[i];
+        bi[i * N + L] = f[i];
+      }
+      if (covered) fi[i * N + L] = cr[i] + f[i];
     }
     return;
   }
@@ -743,14 +752,26 @@ __global__ void __launch_bounds__(128, 4) k_collide_recolor(
   };
   // each colour's own sum: as a difference of densities the smaller one would
   // carry the rounding of the larger (at EVAP_LIM 1e-9 of itself)
-  const double sr = sum(cr), sb = sum(f);
+  double sr = sum(cr), sb = sum(f);
 #pragma unroll
   for (int i = 0; i < 19; i++) f[i] = cr[i] + f[i];
+  const double phi = rhoN[L];
+  const bool stale = phi == 0.0 && pp <= 0 && walls_old[L] >= 1;   // (phi of a solid node is 0)
+  if (stale) {
+    sr = rhoR[L];
+    sb = rhoB[L];
+#pragma unroll
+    for (int i = 0; i < 19; i++) f[i] = fi[i * N + L];
+  }
   Moments<double> m;
   to_moments<double, double>(f, m);
+  if (stale) {
+    m.rho = P.rho0;
+    m.jx = m.jy = m.jz = 0.0;
+  }
   const double rh = m.rho;
   double irho, su, sq;
-  node_rates_fused<double>(T, rhoN[L], rh, irho, su, sq);
+  node_rates_fused<double>(T, phi, rh, irho, su, sq);
   const double n0 = nxv[L], n1 = nyv[L], n2 = nzv[L];
   double fx = 0.0, fy = 0.0, fz = 0.0;
   if (fl && pp <= 0 && z >= 2 && x >= 2) {   // z>=3 .and. x>=3 (1-based), :624
@@ -1177,7 +1198,7 @@ int ref_collide_recolor(sym_handle* h, bool full, bool pulled) {
   auto go = [&](auto kern) {
     kern<<<g, 128, 0, h->st>>>(P, tile_params<double>(P), h->walls_all, h->pout, h->flag, h->nx, h->ny, h->nz, h->gx,
                                h->gy, h->gz, h->rhoN, h->ux, h->uy, h->uz, h->fi, h->ffi, h->ri, h->bi, h->ft, h->ft2,
-                               h->kept);
+                               h->kept, h->walls_old, h->rhoR, h->rhoB);
   };
   if (full) go(k_collide_recolor<true, false>);
   else if (pulled) go(k_collide_recolor<false, true>);

@@ -292,3 +292,44 @@ def test_reference_steps_between_streaming_calls(bounce):
             s.step(n)
         for f in ("ri", "bi", "rho", "rho_N"):
             assert rel_l2(L.get(f), o.arr(f)) <= 1e-10, (k, f)
+
+
+@pytest.mark.parametrize("moved,runs", [("by hand", (1, 1, 1)), ("by hand", (2, 2)), ("by hand", (1, 3)),
+                                        ("by velocity", (1, 1, 1, 1)), ("by velocity", (4,)), ("by velocity", (3, 1))])
+def test_reference_particles_that_jump(moved, runs):
+    """Particles that move by about a node at once uncover nodes next to no
+    particle, which nothing refills: the reference collides what their arrays
+    were left with when they were covered.  Placed by hand between calls, or
+    moving inside them; heavy particles.  The parity targets of this file."""
+    p = params.reference_params(36, 42, 36)
+    p.par, p.rad = 2, 4.0
+    p.mass, p.inertia = 1e6 * p.mass, 1e6 * p.inertia
+    at = np.array([(17.3, 13.0, 18.0), (18.0, 30.5, 16.2)])
+    hand = np.array([(-1.22, 0.13, -0.23), (-0.61, 0.34, 1.08)]) * (moved == "by hand")
+    up = np.array([(-0.27, 0.04, -0.99), (-0.83, -0.45, -0.13)]) * (moved == "by velocity")
+    o = Oracle(p)
+    params.particles_set(o.particles, "center", 2, at.tolist())
+    params.particles_set(o.particles, "center0", 2, at.tolist())
+    params.particles_set(o.particles, "up", 2, up.tolist())
+    o.call("set_walls")
+    o.call("initialization")
+    o.call("derivatives")
+    L = Lattice(p)
+    copy_oracle_to_lattice(o, L)
+    unfilled = 0
+    for k, n in enumerate(runs):
+        if k and moved == "by hand":
+            s = L.particles()
+            for q in (o.particles, s):
+                params.particles_set(q, "center", 2, (at + k * hand).tolist())
+            L.set_particles(s)
+        L.step(n)
+        for _ in range(n):
+            o.step(1)
+            unfilled += int(((o.arr("walls_old") > 0) & (o.arr("walls_all") == 0) & (o.arr("pout") == 0)).sum())
+    assert unfilled
+    compare_masks(o, L, ["walls", "walls_old", "walls_all", "pin", "pout"])
+    for f in [f for f in SCALARS if f not in ("n_x", "n_y", "n_z")] + POPS:
+        e = rel_l2(L.get(f), o.arr(f))
+        assert e <= 1e-10, (f, e)
+    compare_particles(o, L, 2, 1e-9)
