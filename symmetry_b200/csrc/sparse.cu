@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(kT) k_sp_masks(const SpDom* __restrict__ doms,
 // (v = 3) with the import of each refilled node into the fused state: a
 // refilled node's import reads only what its own refill wrote, no refill reads a
 // refilled node (it averages fluid neighbours only), and the particle it
-// belongs to -- the last one next to it -- is read off the masks, not off pout
+// belongs to -- the last one next to it -- is read off the masks, not off pout,
+// which is being marked
 template <typename S>
 __global__ void __launch_bounds__(kT, 4) k_sp_pins(const SpDom* __restrict__ doms, const Blk* __restrict__ map) {
   using R = typename Codec<S>::R;
@@ -268,6 +269,9 @@ __global__ void __launch_bounds__(kT, 4) k_sp_pins(const SpDom* __restrict__ dom
     if (!part::box_node(P, D.bref, D.S->center_old, e.pp, t, x, y, z) || !part::in_range(P, x, y, z)) return;
     const long long L = lin(P, x, y, z);
     if (D.walls_old[L] < 1 || D.walls_all[L] != 0) return;
+    // pout is marked around the particle where it is now; beyond, next to marks
+    // that a particle moved away by hand left behind, it belongs to nobody
+    if (!part::in_box(P, D.bpin, D.S->center, e.pp, x, y, z)) return;
     int owner = 0;
     for (int i = 1; i < 19; i++) {
       const int w =

@@ -13,6 +13,7 @@ import pytest
 from oracle.oracle import Oracle, setup_workload as orc_setup
 from symmetry_b200 import configs
 from symmetry_b200.lib import Lattice, setup_workload
+from symmetry_b200.params import particles_set
 from tests.common import compare_masks, compare_particles, copy_oracle_to_lattice, rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -328,3 +329,24 @@ def test_noisy_thread_between_wetting_walls_stays_finite(storage):
     L.step(20)
     assert all(np.isfinite(v).all() for v in L.macros().values())
     L.close()
+
+
+def test_fast_sphere_moved_by_hand_refills_its_own_nodes_only():
+    """A sphere put elsewhere between steps leaves marks outside its new
+    surroundings behind (until set_walls).  A node uncovered there is next to
+    those marks but not to the particle (pout 0): its densities stay as they
+    were, and no node gets any that is not next to the particle."""
+    w = configs.c2_wall_particle(nx=30, ny=24, nz=26, rad=3.1, centre=(11.7, 9.9, 6.9), z0=6.0, z1=18.0)
+    w.params.mass *= 1e4
+    w.params.inertia *= 1e4
+    w.particles[0]["up"] = [0.2, -0.18, 0.19]
+    L = setup_workload(w)
+    s = L.particles()
+    particles_set(s, "center", 1, [(19.5, 2.46, 14.0)])
+    L.set_particles(s)
+    before = {f: L.get(f).copy() for f in ("rho_R", "rho_B")}
+    L.step(1)
+    left = (L.get("walls_old") > 0) & (L.get("walls_all") == 0) & (L.get("pout") == 0)
+    assert left.any()
+    for f, v in before.items():
+        assert np.array_equal(L.get(f)[left], v[left]), f
