@@ -41,6 +41,7 @@ struct PairSmem {
 };
 
 __host__ __device__ __forceinline__ constexpr float WF(int i) { return float(W(i)); }
+constexpr float kFloatMax = 3.40282347e+38f;
 
 template <typename S, bool SOLID>
 __device__ __forceinline__ void collide_pair_tile(const TileParams<float>& P, const Pad& pd, const S* __restrict__ pin_,
@@ -105,6 +106,12 @@ __device__ __forceinline__ void collide_pair_tile(const TileParams<float>& P, co
       F2 rf(g2s[0] > evap * evap ? rsqrtf(g2s[0]) : 0.f, g2s[1] > evap * evap ? rsqrtf(g2s[1]) : 0.f);
       F2 fn = g2s * rf;
       F2 n0 = g0 * rf, n1 = g1 * rf, n2 = g2 * rf;
+      // a gradient that is not finite is none, as in the reference, whose test
+      // against EVAP_LIM a NaN fails (0 times it would hand it to the neighbours)
+      if (!(g2s[0] <= kFloatMax && g2s[1] <= kFloatMax)) {
+        if (!(g2s[0] <= kFloatMax)) n0.v.x = n1.v.x = n2.v.x = fn.v.x = 0.f;
+        if (!(g2s[1] <= kFloatMax)) n0.v.y = n1.v.y = n2.v.y = fn.v.y = 0.f;
+      }
       if (solid) {
         // both rows' masks are read at once (nodes beyond the halo, read by
         // nobody, take the last one's)

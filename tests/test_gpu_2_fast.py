@@ -350,3 +350,28 @@ def test_fast_sphere_moved_by_hand_refills_its_own_nodes_only():
     assert left.any()
     for f, v in before.items():
         assert np.array_equal(L.get(f)[left], v[left]), f
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("storage", ["fp64", "fp32", "fp16"])
+def test_not_a_number_spreads_as_in_the_reference(storage, bad):
+    """A population that is not finite reaches one node further a step, by
+    streaming: a gradient taken from it is none (the reference's comparison
+    with EVAP_LIM), so it does not reach the neighbours' curvature.  The nodes
+    without a number are the oracle's, rows of both halves of a tile among
+    them."""
+    w = configs.c1_thread(nx=24, ny=21, nz=40, radius=5.0)
+    p = w.params.copy()
+    p.storage = {"fp64": 0, "fp32": 1, "fp16": 2}[storage]
+    o = orc_setup(w)
+    for at in ((9, 3, 7), (14, 11, 33)):
+        o.arr("ri")[at + (0,)] = bad
+    L = Lattice(p)
+    copy_oracle_to_lattice(o, L)
+    for _ in range(3):
+        L.step(1)
+        o.step(1)
+        with np.errstate(all="ignore"):
+            want = ~np.isfinite(o.arr("ri").sum(-1) + o.arr("bi").sum(-1))
+        assert np.array_equal(~np.isfinite(L.macros()["rho"]), want)
+    assert want.any() and not want.all()
